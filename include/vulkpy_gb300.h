@@ -66,7 +66,8 @@ enum vkc_reduce_precision {
 
 /* matmul arithmetic */
 enum vkc_matmul_precision {
-  VKC_MM_FP32 = 0,   /* SIMT fp32 FMA (the drop-in default)                   */
+  VKC_MM_FP32 = 0,   /* fp32 (the drop-in default): FMAs, or exact three-part
+                      * bf16 operands on tcgen05 where there is enough work */
   VKC_MM_BF16 = 1,   /* tcgen05 bf16 x bf16 -> fp32 accumulate                */
   VKC_MM_BF16X3 = 2  /* tcgen05 split-bf16: hi*hi + hi*lo + lo*hi, fp32 acc   */
 };
@@ -360,9 +361,9 @@ typedef struct vkc_gemm_problem {
 } vkc_gemm_problem;
 /* All `count` problems in persistent launches (128 problems per launch):
  * the output tiles of every problem form one work list, longest K first.
- * fp32: bit-identical to vkc_gemm per problem.  bf16x3: bit-identical to
- * vkc_gemm when that call does not split K; bf16: accumulated per 64-wide K
- * block in fp32 (at least as accurate as vkc_gemm's bf16). */
+ * fp32 and bf16x3: bit-identical per problem to vkc_gemm when that call does
+ * not split K; bf16: accumulated per 64-wide K block in fp32 (at least as
+ * accurate as vkc_gemm's bf16). */
 int vkc_gemm_grouped(vkc_device_t dev, int precision, const vkc_gemm_problem* problems, int count);
 /* A parameter step fused into a grouped gradient GEMM: for every problem i
  * with updates[i].value not NULL, after C is stored (the gradient, kept),

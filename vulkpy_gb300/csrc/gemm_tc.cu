@@ -8,12 +8,27 @@
 // keeps ~16 significant bits per operand (relative representation error
 // <= 2^-17) at three tensor-core products instead of fp32 FMA.
 //
+// Plain fp32 products of enough work run here too (fp32_on_tensor_cores):
+// x = hi + mid + lo exactly, three bf16 parts of 8 bits each, and the six
+// products whose terms reach 2^-24 of hi*hi: mid*mid, hi*mid, mid*hi, hi*lo,
+// lo*hi, hi*hi (the dropped mid*lo and lo*lo are below 2^-27).  hi*hi has TMEM
+// accumulators of its own, restarted every 64 (or 32) of K, and the five
+// small products, 2^-8 of it, have theirs, restarted every kLoSpan blocks; so
+// the tensor pipe's truncation touches four (two) full-size additions, and
+// all accumulations are added in fp32 registers with round-to-nearest.
+// Measured against float64 (N(0,1) operands): 6.5e-8 to 1.7e-7 for K from 64
+// to 8192 where FMAs in order of k give 1.45e-7 to 1.1e-6.  Values the split cannot hold (inf, NaN, |x| >= 2^127 or
+// 0 < |x| < 2^-110) become NaN in hi, so every result they reach is not
+// finite; results that are not finite are recomputed from the fp32 operands
+// with ordered FMAs (k_gemm_repair, or inside the split-K reduction).
+//
 // k_gemm_tcp is persistent (one CTA per SM; each CTA loads every operand tile
 // it multiplies into its own shared memory) with two TMEM accumulators, so a
 // tile's epilogue overlaps the next tile's MMAs.  Every mbarrier wait is
 // bounded by a wall-clock limit; on expiry the CTA records bit1 in the device
 // error word, drains what it issued and returns.
 #include "gemm_tc.cuh"
+#include "gemm_repair.cuh"
 #include "tc_ptx.cuh"
 #include "tc_epilogue.cuh"
 
@@ -46,24 +61,31 @@ namespace {
 // quarter its warp rank allows) and columns 128*((w-2)/4).. of a buffer.
 //
 // bf16 mode: one accumulation per unit over the whole K range.
-// split mode (hi*hi + hi*lo + lo*hi): one accumulation per DRAIN K blocks;
-// the epilogue adds each into fp32 registers with round-to-nearest, so the
-// tensor pipe's truncating accumulation spans at most DRAIN*64 of K.
+// split modes: one accumulation per DRAIN K blocks; the epilogue adds each
+// into fp32 registers with round-to-nearest, so the tensor pipe's truncating
+// accumulation spans at most DRAIN*64 of K.
+//
+// PARTS: bf16 copies per operand (1: bf16, 2: split-bf16x3, 3: fp32).  With
+// three parts a K block is 96 KB of tiles and only two fit, so its tiles are
+// released one by one as their last product is issued (five barrier pairs per
+// stage: b_mid, a_mid, b_lo, a_lo, then both hi) and the next-but-one
+// block's copies start while this block is still multiplied.
 constexpr int kEpiWarps = 8;
 constexpr int kThreadsP = 32 * (2 + kEpiWarps);
 constexpr int kGroupM = 16;        // tile rows per raster group (L2 reuse)
 
 
 // BN: columns of C per CTA tile (256 or 128; the autotuner picks per shape).
-template <bool X3, int BN, int STAGES>
+template <int PARTS, int BN, int STAGES>
 struct PCfg {
   static constexpr uint32_t kABytes = kBM * kBK * 2;             // 16 KB
   static constexpr uint32_t kBBytes = BN * kBK * 2;
-  static constexpr uint32_t kStageBytes = (X3 ? 2u : 1u) * (kABytes + kBBytes);
+  static constexpr uint32_t kStageBytes = (uint32_t)PARTS * (kABytes + kBBytes);
   static constexpr uint32_t kBarOff = STAGES * kStageBytes;
-  // full[S], empty[S], accf[2], acce[2], drain, red[2], epi, then tmem slot
-  // + abort flag
-  static constexpr uint32_t kSlotOff = kBarOff + 8u * (2 * STAGES + 8);
+  static constexpr int kRing = STAGES * (PARTS == 3 ? 5 : 1);  // stage barrier pairs
+  // full[kRing], empty[kRing], accf[2], acce[2], drain, red[2], epi, loe[2],
+  // then tmem slot + abort flag
+  static constexpr uint32_t kSlotOff = kBarOff + 8u * (2 * kRing + 10);
   static constexpr uint32_t kEpiOff = (kSlotOff + 16 + 127) / 128 * 128;  // per-warp epilogue stages
   static constexpr uint32_t kSmem = kEpiOff + kEpiWarps * kEpiStageBytes + 1024 /*alignment slack*/;
 };
@@ -132,15 +154,21 @@ __device__ __forceinline__ void cluster_reduce_rows(const float* partial, int sp
 
 // cl_reduce: the grid is made of clusters of `splits` CTAs (one per K range
 // of a tile) that reduce their partial sums themselves (no separate launch).
-template <bool X3, int BN, int STAGES, int DRAIN>
+// map_a / map_b: the hi copies (PARTS == 3: the three copies one after the
+// other as 3 M and 3 N rows); map_alo / map_blo: the lo copies (PARTS == 2).
+// repair (PARTS == 3): count of 32 x 32 blocks of C left to k_gemm_repair,
+// then their numbers.
+template <int PARTS, int BN, int STAGES, int DRAIN>
 __global__ void __launch_bounds__(kThreadsP, 1)
 k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
            const __grid_constant__ CUtensorMap map_alo, const __grid_constant__ CUtensorMap map_blo, int M, int N,
            int K, float alpha, float beta, float* __restrict__ C, int64_t ldc, const float* __restrict__ bias, int act,
            uint32_t* err, float* __restrict__ partial, int splits, int kps, int m_blocks, int n_blocks,
-           int cl_reduce, const float* __restrict__ dmask, int dact) {
-  using Cfg = PCfg<X3, BN, STAGES>;
-  constexpr uint32_t kCols = 2 * BN;  // two accumulators
+           int cl_reduce, const float* __restrict__ dmask, int dact, uint32_t* __restrict__ repair) {
+  using Cfg = PCfg<PARTS, BN, STAGES>;
+  constexpr bool X3 = PARTS > 1;      // a split mode: accumulations drained into fp32 registers
+  constexpr int R = Cfg::kRing;
+  constexpr uint32_t kCols = (PARTS == 3 ? 4 : 2) * BN;  // two accumulators (PARTS == 3: hi*hi and small terms)
   constexpr int CW = BN / 2;          // columns per epilogue warp
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -148,15 +176,16 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   uint8_t* gbase = smem_raw + (base - raw);
   const uint32_t bars = base + Cfg::kBarOff;
   auto full_bar = [&](int s) { return bars + 8u * s; };
-  auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
-  auto accf_bar = [&](int b) { return bars + 8u * (2 * STAGES + b); };
-  auto acce_bar = [&](int b) { return bars + 8u * (2 * STAGES + 2 + b); };
-  const uint32_t drain_bar = bars + 8u * (2 * STAGES + 4);
+  auto empty_bar = [&](int s) { return bars + 8u * (R + s); };
+  auto accf_bar = [&](int b) { return bars + 8u * (2 * R + b); };
+  auto acce_bar = [&](int b) { return bars + 8u * (2 * R + 2 + b); };
+  const uint32_t drain_bar = bars + 8u * (2 * R + 4);
   // red[u & 1]: all partials of the cluster's u-th tile stored (two, used in
   // turn: a peer already on the next tile arrives on the other one, so it
   // cannot complete a phase early); epi: this CTA's epilogue warps stored
-  auto red_bar = [&](int u) { return bars + 8u * (2 * STAGES + 5 + (u & 1)); };
-  const uint32_t epi_bar = bars + 8u * (2 * STAGES + 7);
+  auto red_bar = [&](int u) { return bars + 8u * (2 * R + 5 + (u & 1)); };
+  const uint32_t epi_bar = bars + 8u * (2 * R + 7);
+  auto loe_bar = [&](int b) { return bars + 8u * (2 * R + 8 + b); };  // PARTS == 3: small-term accumulator read
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + Cfg::kSlotOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -166,13 +195,14 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   const int units = m_blocks * n_blocks * splits;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < R; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);  // the MMA issuer's commit
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(accf_bar(b), 1);
       mbar_init(acce_bar(b), kEpiWarps);
+      mbar_init(loe_bar(b), kEpiWarps);
     }
     mbar_init(drain_bar, 1);
     if (cl_reduce) {
@@ -203,27 +233,48 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   auto stage_b = [&](int s) { return stage_a(s) + Cfg::kABytes; };
   auto stage_alo = [&](int s) { return stage_b(s) + Cfg::kBBytes; };
   auto stage_blo = [&](int s) { return stage_alo(s) + Cfg::kABytes; };
+  // PARTS == 3: part p of either operand (0 hi, 1 mid, 2 lo)
+  auto part_a = [&](int s, int p) { return stage_a(s) + (uint32_t)p * (Cfg::kABytes + Cfg::kBBytes); };
+  auto part_b = [&](int s, int p) { return part_a(s, p) + Cfg::kABytes; };
 
   if (warp == 0 && lane == 0) {
     // ---------------- TMA producer
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_b)) : "memory");
-    if (X3) {
+    if (PARTS == 2) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_alo)) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_blo)) : "memory");
     }
     int it = 0;
     bool ok = true;
+    int part = 0;  // PARTS == 3: tile groups of the current block already issued
     for (int u = (int)blockIdx.x; u < units && ok; u += (int)gridDim.x) {
       const PUnit p = unit_of<BN>(u, splits, kps, nk, m_blocks, n_blocks);
       for (int kb = 0; kb < p.nkb; ++kb, ++it) {
         const int s = it % STAGES;
+        if constexpr (PARTS == 3) {
+          // in the order the issuer releases them: b_mid, a_mid, b_lo, a_lo, a_hi + b_hi
+          const uint32_t ph = ((it / STAGES) & 1) ^ 1;
+          const int kx = (p.kb0 + kb) * kBK;
+          for (part = 0; part < 5; ++part) {
+            const int r = s * 5 + part;
+            if (*abort_flag || !mbar_wait(empty_bar(r), ph)) { ok = false; break; }
+            const int q = part == 4 ? 0 : 1 + part / 2;  // 1 1 2 2 0
+            const bool b_side = (part & 1) == 0, a_side = part == 4 || !b_side;
+            mbar_expect_tx(full_bar(r), (a_side ? Cfg::kABytes : 0u) + (b_side ? Cfg::kBBytes : 0u));
+            if (a_side) tma_load_2d(part_a(s, q), &map_a, full_bar(r), kx, q * M + p.m0);
+            if (b_side) tma_load_2d(part_b(s, q), &map_b, full_bar(r), kx, q * N + p.n0);
+          }
+          if (!ok) break;
+          part = 0;
+          continue;
+        }
         if (*abort_flag || !mbar_wait(empty_bar(s), ((it / STAGES) & 1) ^ 1)) { ok = false; break; }
         mbar_expect_tx(full_bar(s), Cfg::kStageBytes);
         const int kx = (p.kb0 + kb) * kBK;
         tma_load_2d(stage_a(s), &map_a, full_bar(s), kx, p.m0);
         tma_load_2d(stage_b(s), &map_b, full_bar(s), kx, p.n0);
-        if (X3) {
+        if (PARTS == 2) {
           tma_load_2d(stage_alo(s), &map_alo, full_bar(s), kx, p.m0);
           tma_load_2d(stage_blo(s), &map_blo, full_bar(s), kx, p.n0);
         }
@@ -235,23 +286,74 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     }
     // Tail: wait until the MMAs have released every stage, so no copy or
     // commit is still in flight at exit.
-    for (int t = 0; t < STAGES && it - STAGES + t >= 0; ++t) {
-      const int j = it - STAGES + t;
-      if (!mbar_wait(empty_bar(j % STAGES), (j / STAGES) & 1)) {
+    constexpr int G = R / STAGES;
+    for (int t = 0; t < STAGES * G; ++t) {
+      const int j = it - STAGES + t / G;
+      if (j < 0) continue;
+      if (!mbar_wait(empty_bar((j % STAGES) * G + t % G), (j / STAGES) & 1)) {
         atomicOr(err, 2u);
         break;
       }
     }
+    // a block given up half way: its copies must land before the CTA leaves
+    for (int t = 0; !ok && t < part; ++t) mbar_wait(full_bar((it % STAGES) * G + t), (it / STAGES) & 1);
   } else if (warp == 1 && lane == 0) {
     // ---------------- MMA issuer
     constexpr uint32_t idesc = (1u << 4)            // D: fp32
                                | (1u << 7)          // A: bf16
                                | (1u << 10)         // B: bf16
                                | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-    int it = 0, acc_it = 0;
+    int it = 0, acc_it = 0, lo_it = 0;
     bool ok = true;
     for (int u = (int)blockIdx.x; u < units && ok; u += (int)gridDim.x) {
       const PUnit p = unit_of<BN>(u, splits, kps, nk, m_blocks, n_blocks);
+      if constexpr (PARTS == 3) {
+        // small product i: op(A) part pa times op(B) part pb; a tile is
+        // released after its last product.  hi*hi follows, in DRAIN
+        // accumulations per K block (buffers 0 and 1); the small products
+        // have buffers 2 and 3.
+        constexpr int pa[5] = {1, 0, 1, 0, 2}, pb[5] = {1, 1, 0, 2, 0}, rel[5] = {-1, 0, 1, 2, 3};
+        for (int kb = 0; kb < p.nkb && ok; ++kb, ++it) {
+          const int s = it % STAGES;
+          const uint32_t ph = (it / STAGES) & 1;
+          const bool lo_first = kb % kLoSpan == 0, lo_last = kb % kLoSpan == kLoSpan - 1 || kb == p.nkb - 1;
+          const int lb = lo_it & 1;
+          if (*abort_flag || (lo_first && !mbar_wait(loe_bar(lb), ((lo_it >> 1) & 1) ^ 1))) { ok = false; break; }
+          const uint32_t d_lo = tmem + (uint32_t)((2 + lb) * BN);
+#pragma unroll
+          for (int i = 0; i < 5; ++i) {
+            // the tiles this product is the first to read
+            if (i == 0) ok = mbar_wait(full_bar(s * 5), ph) && mbar_wait(full_bar(s * 5 + 1), ph);
+            if (i == 1) ok = mbar_wait(full_bar(s * 5 + 4), ph);
+            if (i == 3) ok = mbar_wait(full_bar(s * 5 + 2), ph);
+            if (i == 4) ok = mbar_wait(full_bar(s * 5 + 3), ph);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k)
+              mma_bf16(d_lo, sw128_desc(part_a(s, pa[i]) + 32u * k), sw128_desc(part_b(s, pb[i]) + 32u * k), idesc,
+                       (i == 0 && k == 0 && lo_first) ? 0u : 1u);
+            if (rel[i] >= 0) mma_commit(empty_bar(s * 5 + rel[i]));
+          }
+          constexpr int STEPS = kBK / 16 / DRAIN;
+#pragma unroll
+          for (int sub = 0; sub < DRAIN && ok; ++sub, ++acc_it) {
+            const int b = acc_it & 1;
+            ok = mbar_wait(acce_bar(b), ((acc_it >> 1) & 1) ^ 1);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int k = sub * STEPS; k < (sub + 1) * STEPS; ++k)
+              mma_bf16(tmem + (uint32_t)(b * BN), sw128_desc(part_a(s, 0) + 32u * k),
+                       sw128_desc(part_b(s, 0) + 32u * k), idesc, k == sub * STEPS ? 0u : 1u);
+            mma_commit(accf_bar(b));  // the small products issued so far are complete with it
+          }
+          if (!ok) break;
+          mma_commit(empty_bar(s * 5 + 4));
+          if (lo_last) ++lo_it;
+        }
+        continue;
+      }
       const int span = X3 ? DRAIN : p.nkb;  // K blocks per accumulation
       for (int g0 = 0; g0 < p.nkb && ok; g0 += span, ++acc_it) {
         const int b = acc_it & 1;
@@ -268,7 +370,7 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             const uint64_t a = sw128_desc(stage_a(s) + 32u * k);
             const uint64_t bb = sw128_desc(stage_b(s) + 32u * k);
             const uint32_t first = (kb == g0 && k == 0) ? 0u : 1u;
-            if (X3) {
+            if (PARTS == 2) {
               // small cross terms first, the dominant hi*hi term last
               mma_bf16(d, a, sw128_desc(stage_blo(s) + 32u * k), idesc, first);
               mma_bf16(d, sw128_desc(stage_alo(s) + 32u * k), bb, idesc, 1);
@@ -296,12 +398,12 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     const int q = warp & 3;          // TMEM lane quarter
     const int h = (warp - 2) >> 2;   // column half of the tile
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
-    int acc_it = 0, red_it = 0;
+    int acc_it = 0, red_it = 0, lo_it = 0;
     bool ok = true;
     for (int u = (int)blockIdx.x; u < units && ok; u += (int)gridDim.x) {
       const PUnit p = unit_of<BN>(u, splits, kps, nk, m_blocks, n_blocks);
       const int span = X3 ? DRAIN : p.nkb;
-      const int ngroups = (p.nkb + span - 1) / span;
+      const int ngroups = PARTS == 3 ? p.nkb * DRAIN : (p.nkb + span - 1) / span;
       float acc[X3 ? CW : 1];
       if (X3) {
 #pragma unroll
@@ -312,7 +414,37 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         b = acc_it & 1;
         if (*abort_flag || !mbar_wait(accf_bar(b), (acc_it >> 1) & 1)) { ok = false; break; }
         tc_fence_after();
-        if (X3 && ngroups > 1) {
+        if constexpr (PARTS == 3) {
+          // hi*hi, and every kLoSpan blocks the small terms, into the fp32 sums; at the end of the unit the sums go back into
+          // the buffer for the store loop below
+          const bool last = gi == ngroups - 1;
+          const bool with_lo = last || (gi + 1) % (kLoSpan * DRAIN) == 0;
+          const int lb = lo_it & 1;
+#pragma unroll
+          for (int c = 0; c < CW / 32; ++c) {
+            const uint32_t ta = tmem + lane_addr + (uint32_t)(b * BN + h * CW + c * 32);
+            uint32_t r0[32];
+            if (with_lo) {
+              tmem_ld32(ta + (uint32_t)((2 + lb - b) * BN), r0);
+#pragma unroll
+              for (int j = 0; j < 32; ++j) acc[c * 32 + j] += __uint_as_float(r0[j]);
+            }
+            tmem_ld32(ta, r0);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              acc[c * 32 + j] += __uint_as_float(r0[j]);
+              r0[j] = __float_as_uint(acc[c * 32 + j]);
+            }
+            if (last) tmem_st32_nw(ta, r0);
+          }
+          if (last) tmem_wait_st();
+          if (with_lo) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(loe_bar(lb));
+            ++lo_it;
+          }
+        } else if (X3 && ngroups > 1) {
           // add this accumulation to the fp32 sums; after the last one, put
           // the sums back into the buffer for the store loop below (with a
           // single accumulation the store loop reads it as it is)
@@ -355,10 +487,20 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         uint32_t r0[32];
         tmem_ld32(tmem + lane_addr + (uint32_t)(b * BN + h * CW + c * 32), r0);
         const int col0 = p.n0 + h * CW + c * 32;
+        if (PARTS == 3 && !raw_out && p.m0 + q * 32 < M && col0 < N) {
+          // a block with a result that is not finite is left to k_gemm_repair,
+          // whole (C may be read with beta != 0, so it is not touched here)
+          if (!block_finite(r0, p.m0 + q * 32 + lane < M, N - col0)) {
+            if (lane == 0)
+              repair[1 + atomicAdd(repair, 1u)] =
+                  (uint32_t)((p.m0 / 32 + q) * ((N + 31) / 32) + col0 / 32);
+            continue;
+          }
+        }
         if (p.m0 + q * 32 < M && col0 < N)
           // (the split kernel with 256-column tiles holds 128 running sums per
           // thread and has no registers to spare for the fixed forms)
-          epilogue_tile32<!(X3 && BN == 256)>(r0, stage, cbase, raw_out ? nullptr : dmask, bias, ld, p.m0 + q * 32, M,
+          epilogue_tile32<!(PARTS == 2 && BN == 256)>(r0, stage, cbase, raw_out ? nullptr : dmask, bias, ld, p.m0 + q * 32, M,
                                               col0, N, alpha, beta, act, raw_out, nullptr, 0.f, dact);
       }
       tc_fence_before();
@@ -420,12 +562,33 @@ __device__ __forceinline__ void split_bf16(float x, __nv_bfloat16& h, __nv_bfloa
   l = __float2bfloat16_rn(x - __bfloat162float(h));
 }
 
+// 8 values of one row as 16-byte stores: hi, with lo (or NULL), or as three
+// parts `part` elements apart (part != 0).
+template <int PARTS>
+__device__ __forceinline__ void put8(const float (&x)[8], __nv_bfloat16* hi, __nv_bfloat16* lo, int64_t part) {
+  __align__(16) __nv_bfloat16 h[8], l[8];
+  if (PARTS == 3) {
+    __align__(16) __nv_bfloat16 m[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) split_bf16_3(x[t], h[t], m[t], l[t]);
+    *reinterpret_cast<uint4*>(hi) = *reinterpret_cast<const uint4*>(h);
+    *reinterpret_cast<uint4*>(hi + part) = *reinterpret_cast<const uint4*>(m);
+    *reinterpret_cast<uint4*>(hi + 2 * part) = *reinterpret_cast<const uint4*>(l);
+  } else {
+#pragma unroll
+    for (int t = 0; t < 8; ++t) split_bf16(x[t], h[t], l[t]);
+    *reinterpret_cast<uint4*>(hi) = *reinterpret_cast<const uint4*>(h);
+    if (lo) *reinterpret_cast<uint4*>(lo) = *reinterpret_cast<const uint4*>(l);
+  }
+}
+
 // K contiguous in the source: dst[r*Kp + k] from src[r*ld + k], zero padding
 // k >= K.  8 elements per thread: 2 x float4 in (`vec`: ld % 4 == 0 and a
 // 16-byte aligned source; otherwise element loads), one 16-byte store per
 // output (Kp % 8 == 0); the chunk that straddles K is read element by
 // element, chunks past K are zero.  Blocks `blk` of `nblk` stride over the
 // chunks.
+template <int PARTS>
 __device__ __forceinline__ void split_kmajor8_body(const float* __restrict__ src, int64_t R, int64_t K, int64_t ld,
                                                    __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
                                                    int64_t Kp, int64_t blk, int64_t nblk, bool vec = true) {
@@ -442,11 +605,7 @@ __device__ __forceinline__ void split_kmajor8_body(const float* __restrict__ src
 #pragma unroll
       for (int t = 0; t < 8; ++t) x[t] = k + t < K ? src[r * ld + k + t] : 0.f;
     }
-    __align__(16) __nv_bfloat16 h[8], l[8];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) split_bf16(x[t], h[t], l[t]);
-    *reinterpret_cast<uint4*>(hi + r * Kp + k) = *reinterpret_cast<const uint4*>(h);
-    if (lo) *reinterpret_cast<uint4*>(lo + r * Kp + k) = *reinterpret_cast<const uint4*>(l);
+    put8<PARTS>(x, hi + r * Kp + k, lo ? lo + r * Kp + k : nullptr, R * Kp);
   }
 }
 
@@ -458,6 +617,7 @@ __device__ __forceinline__ void split_kmajor8_body(const float* __restrict__ src
 // multiple of 4 (the tail of a row is read element by element).  256
 // threads; tile (bx, by) covers rows r in [64 bx, 64 bx + 64), k in
 // [64 by, 64 by + 64).
+template <int PARTS>
 __device__ __forceinline__ void split_transpose_body(const float* __restrict__ src, int64_t R, int64_t K, int64_t ld,
                                                      __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
                                                      int64_t Kp, int64_t bx, int64_t by, float (*tile)[65],
@@ -494,11 +654,10 @@ __device__ __forceinline__ void split_transpose_body(const float* __restrict__ s
   for (int j = rr; j < 64; j += 32) {
     const int64_t r = r0 + j, k = k0 + k8;
     if (r < R && k < Kp) {  // Kp % 8 == 0, so all 8 are inside the row
-      __align__(16) __nv_bfloat16 h[8], l[8];
+      float x[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) split_bf16(tile[k8 + q][j], h[q], l[q]);
-      *reinterpret_cast<uint4*>(hi + r * Kp + k) = *reinterpret_cast<const uint4*>(h);
-      if (lo) *reinterpret_cast<uint4*>(lo + r * Kp + k) = *reinterpret_cast<const uint4*>(l);
+      for (int q = 0; q < 8; ++q) x[q] = tile[k8 + q][j];
+      put8<PARTS>(x, hi + r * Kp + k, lo ? lo + r * Kp + k : nullptr, R * Kp);
     }
   }
 }
@@ -516,27 +675,32 @@ struct SplitJob {
   int vec;          // 16-byte loads allowed (ld % 4 == 0, aligned source)
 };
 
+// PARTS == 3: hi, mid and lo one after the other at `hi`; `repair` (may be
+// NULL) is the count of blocks k_gemm_repair will have to do, zeroed here.
+template <int PARTS>
 __global__ void __launch_bounds__(256) k_split_pair(const __grid_constant__ SplitJob a,
-                                                    const __grid_constant__ SplitJob b) {
+                                                    const __grid_constant__ SplitJob b, uint32_t* repair) {
   __shared__ float tile[64][65];
   pdl_wait();
   pdl_trigger();
+  if (PARTS == 3 && blockIdx.x == 0 && threadIdx.x == 0) *repair = 0u;
   const bool first = blockIdx.x < a.blocks;
   const SplitJob& j = first ? a : b;
   const int64_t blk = first ? (int64_t)blockIdx.x : (int64_t)blockIdx.x - a.blocks;
   if (j.tiles_x == 0)
-    split_kmajor8_body(j.src, j.R, j.K, j.ld, j.hi, j.lo, j.Kp, blk, j.blocks, j.vec != 0);
+    split_kmajor8_body<PARTS>(j.src, j.R, j.K, j.ld, j.hi, j.lo, j.Kp, blk, j.blocks, j.vec != 0);
   else
-    split_transpose_body(j.src, j.R, j.K, j.ld, j.hi, j.lo, j.Kp, blk % j.tiles_x, blk / j.tiles_x, tile, j.vec != 0);
+    split_transpose_body<PARTS>(j.src, j.R, j.K, j.ld, j.hi, j.lo, j.Kp, blk % j.tiles_x, blk / j.tiles_x, tile, j.vec != 0);
 }
 
 // Both operands in one k_split_pair launch (16-byte loads where a source
 // allows them, element loads where it does not).
+template <int PARTS>
 int split_operands(vkc_device_t dev, const float* A, int64_t M, int64_t lda, bool a_kcontig, __nv_bfloat16* a_hi,
                    __nv_bfloat16* a_lo, const float* B, int64_t N, int64_t ldb, bool b_kcontig,
-                   __nv_bfloat16* b_hi, __nv_bfloat16* b_lo, int64_t K, int64_t Kp) {
+                   __nv_bfloat16* b_hi, __nv_bfloat16* b_lo, int64_t K, int64_t Kp, uint32_t* repair = nullptr) {
   auto aligned = [](const float* p, int64_t ld) { return ld % 4 == 0 && ((uintptr_t)p & 15u) == 0; };
-  const int64_t cap = (int64_t)dev->sm_count * resident_blocks((const void*)k_split_pair, 256);
+  const int64_t cap = (int64_t)dev->sm_count * resident_blocks((const void*)k_split_pair<PARTS>, 256);
   auto job = [&](const float* src, int64_t R, int64_t ld, bool kcontig, __nv_bfloat16* hi, __nv_bfloat16* lo) {
     SplitJob j{src, R, K, ld, Kp, hi, lo, 0, 0, aligned(src, ld) ? 1 : 0};
     if (kcontig) {
@@ -550,7 +714,8 @@ int split_operands(vkc_device_t dev, const float* A, int64_t M, int64_t lda, boo
   const SplitJob ja = job(A, M, lda, a_kcontig, a_hi, a_lo), jb = job(B, N, ldb, b_kcontig, b_hi, b_lo);
   const int64_t grid = ja.blocks + jb.blocks;
   if (grid > 0x7fffffff) return set_error(VKC_ERR_INVALID, "matmul: operands too large for the pre-pass grid");
-  const cudaError_t e = launch_pdl(k_split_pair, dim3((unsigned)grid), dim3(256), 0, dev->stream, ja, jb);
+  const cudaError_t e = launch_pdl(k_split_pair<PARTS>, dim3((unsigned)grid), dim3(256), 0, dev->stream, ja, jb,
+                                   repair);
   if (e != cudaSuccess) return set_error(VKC_ERR_CUDA, "split_operands launch: %s", cudaGetErrorString(e));
   return check_launch("split_operands");
 }
@@ -673,10 +838,12 @@ __device__ __forceinline__ void split_out1(const SplitOut& so, int64_t r, int64_
 
 // Four columns per thread (N % 4 == 0, ldc % 4 == 0, 16-byte aligned C);
 // the split loads are issued four at a time ahead of their (ordered) adds.
+// REPAIR: sums that are not finite are recomputed from the operands `ro`.
+template <bool REPAIR>
 __global__ void __launch_bounds__(256)
 k_splitk_reduce4(const float* __restrict__ partial, int splits, int64_t M, int64_t N, float alpha, float beta,
                  float* __restrict__ C, int64_t ldc, const float* __restrict__ bias, int act,
-                 const float* __restrict__ dmask, int dact, SplitOut so) {
+                 const float* __restrict__ dmask, int dact, SplitOut so, RepairOperands ro) {
   pdl_wait();
   pdl_trigger();
   const int64_t total = M * N, quads = total / 4;
@@ -696,6 +863,12 @@ k_splitk_reduce4(const float* __restrict__ partial, int splits, int64_t M, int64
     }
     for (; z < splits; ++z) add4(s, __ldcs(p + (int64_t)z * quads));
     const int64_t r = i / N, col = i - r * N;
+    if (REPAIR && !all_finite(s.x, s.y, s.z, s.w)) {
+      if (!isfinite(s.x)) s.x = repair_dot(ro, r, col);
+      if (!isfinite(s.y)) s.y = repair_dot(ro, r, col + 1);
+      if (!isfinite(s.z)) s.z = repair_dot(ro, r, col + 2);
+      if (!isfinite(s.w)) s.w = repair_dot(ro, r, col + 3);
+    }
     float4* cp = reinterpret_cast<float4*>(C + r * ldc + col);
     const float4 c0 = beta != 0.f ? *cp : make_float4(0.f, 0.f, 0.f, 0.f);
     float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -718,10 +891,11 @@ k_splitk_reduce4(const float* __restrict__ partial, int splits, int64_t M, int64
   }
 }
 
+template <bool REPAIR>
 __global__ void __launch_bounds__(256)
 k_splitk_reduce(const float* __restrict__ partial, int splits, int64_t M, int64_t N, float alpha, float beta,
                 float* __restrict__ C, int64_t ldc, const float* __restrict__ bias, int act,
-                const float* __restrict__ dmask, int dact, SplitOut so) {
+                const float* __restrict__ dmask, int dact, SplitOut so, RepairOperands ro) {
   pdl_wait();
   pdl_trigger();
   const int64_t total = M * N;
@@ -730,6 +904,7 @@ k_splitk_reduce(const float* __restrict__ partial, int splits, int64_t M, int64_
     float s = partial[i];
     for (int z = 1; z < splits; ++z) s += partial[(int64_t)z * total + i];
     const int64_t r = i / N, col = i - r * N;
+    if (REPAIR && !isfinite(s)) s = repair_dot(ro, r, col);
     float* c = C + r * ldc + col;
     float v = splitk_epilogue(s, alpha, beta, beta != 0.f ? *c : 0.f, bias != nullptr, bias ? bias[col] : 0.f, act);
     if (dmask) v = act_deriv(v, dmask[r * ldc + col], dact);
@@ -739,19 +914,23 @@ k_splitk_reduce(const float* __restrict__ partial, int splits, int64_t M, int64_
 }
 
 int splitk_reduce(vkc_device_t dev, const float* partial, int splits, int64_t M, int64_t N, float alpha, float beta,
-                  float* C, int64_t ldc, const GemmEpilogue& epi, const SplitOut* out = nullptr) {
+                  float* C, int64_t ldc, const GemmEpilogue& epi, const SplitOut* out = nullptr,
+                  const RepairOperands& ro = RepairOperands{}) {
   const SplitOut so = out ? *out : SplitOut{nullptr, nullptr, 0};
-  if (N % 4 == 0 && ldc % 4 == 0 && ((uintptr_t)C & 15u) == 0 && ((uintptr_t)epi.dmask & 15u) == 0) {
-    unsigned g = wave_grid(dev, k_splitk_reduce4, (size_t)(M * N / 4), 256);
-    const cudaError_t e = launch_pdl(k_splitk_reduce4, dim3(g), dim3(256), 0, dev->stream, partial, splits, M, N,
-                                     alpha, beta, C, ldc, epi.bias, epi.act, epi.dmask, epi.dact, so);
-    if (e != cudaSuccess) return set_error(VKC_ERR_CUDA, "splitk_reduce launch: %s", cudaGetErrorString(e));
+  const bool vec = N % 4 == 0 && ldc % 4 == 0 && ((uintptr_t)C & 15u) == 0 && ((uintptr_t)epi.dmask & 15u) == 0;
+  auto launch = [&](auto kern, unsigned grid) {
+    return launch_pdl(kern, dim3(grid), dim3(256), 0, dev->stream, partial, splits, M, N, alpha, beta, C, ldc,
+                      epi.bias, epi.act, epi.dmask, epi.dact, so, ro);
+  };
+  cudaError_t e;
+  if (vec) {
+    const unsigned g = wave_grid(dev, k_splitk_reduce4<false>, (size_t)(M * N / 4), 256);
+    e = ro.a ? launch(k_splitk_reduce4<true>, g) : launch(k_splitk_reduce4<false>, g);
   } else {
-    unsigned g = stream_grid(dev, (size_t)(M * N), 256);
-    const cudaError_t e = launch_pdl(k_splitk_reduce, dim3(g), dim3(256), 0, dev->stream, partial, splits, M, N,
-                                     alpha, beta, C, ldc, epi.bias, epi.act, epi.dmask, epi.dact, so);
-    if (e != cudaSuccess) return set_error(VKC_ERR_CUDA, "splitk_reduce launch: %s", cudaGetErrorString(e));
+    const unsigned g = stream_grid(dev, (size_t)(M * N), 256);
+    e = ro.a ? launch(k_splitk_reduce<true>, g) : launch(k_splitk_reduce<false>, g);
   }
+  if (e != cudaSuccess) return set_error(VKC_ERR_CUDA, "splitk_reduce launch: %s", cudaGetErrorString(e));
   return check_launch("splitk_reduce");
 }
 
@@ -797,12 +976,13 @@ int max_clusters(Kern kern, uint32_t smem, int size) {
   return n;
 }
 
-template <bool X3, int BN, int STAGES, int DRAIN>
+template <int PARTS, int BN, int STAGES, int DRAIN>
 int launch_tcp(vkc_device_t dev, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& malo,
                const CUtensorMap& mblo, int64_t M, int64_t N, int64_t K, float alpha, float beta, float* C,
-               int64_t ldc, const GemmEpilogue& epi, int splits, const SplitOut* out) {
-  using Cfg = PCfg<X3, BN, STAGES>;
-  auto kern = k_gemm_tcp<X3, BN, STAGES, DRAIN>;
+               int64_t ldc, const GemmEpilogue& epi, int splits, const SplitOut* out,
+               const RepairOperands& ro = RepairOperands{}, uint32_t* repair = nullptr) {
+  using Cfg = PCfg<PARTS, BN, STAGES>;
+  auto kern = k_gemm_tcp<PARTS, BN, STAGES, DRAIN>;
   static bool attr_set = false;
   if (!attr_set) {
     VKC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem));
@@ -839,7 +1019,7 @@ int launch_tcp(vkc_device_t dev, const CUtensorMap& ma, const CUtensorMap& mb, c
     cudaGetLastError();
     cap = cudaStreamCaptureStatusActive;
   }
-  const int clusters = splits > 1 && cap == cudaStreamCaptureStatusNone && !out &&
+  const int clusters = PARTS < 3 && splits > 1 && cap == cudaStreamCaptureStatusNone && !out &&
                                g_cluster_splitk.load(std::memory_order_relaxed)
                            ? max_clusters(kern, Cfg::kSmem, splits)
                            : 0;
@@ -848,19 +1028,21 @@ int launch_tcp(vkc_device_t dev, const CUtensorMap& ma, const CUtensorMap& mb, c
     const int ctas = (int)std::min<int64_t>(tiles, clusters) * splits;
     e = launch_pdl_cluster(kern, dim3((unsigned)ctas), dim3(kThreadsP), Cfg::kSmem, dev->stream, (unsigned)splits, ma,
                            mb, malo, mblo, (int)M, (int)N, (int)K, alpha, beta, C, ldc, epi.bias, epi.act,
-                           dev->err_word, partial, splits, kps, (int)m_blocks, n_blocks, 1, epi.dmask, epi.dact);
+                           dev->err_word, partial, splits, kps, (int)m_blocks, n_blocks, 1, epi.dmask, epi.dact, nullptr);
   } else {
     const int ctas = (int)std::min<int64_t>(units, max_ctas(dev, kern, Cfg::kSmem));
     e = launch_pdl(kern, dim3((unsigned)ctas), dim3(kThreadsP), Cfg::kSmem, dev->stream, ma, mb, malo, mblo, (int)M,
                    (int)N, (int)K, alpha, beta, C, ldc, epi.bias, epi.act, dev->err_word, partial, splits, kps,
-                   (int)m_blocks, n_blocks, 0, epi.dmask, epi.dact);
+                   (int)m_blocks, n_blocks, 0, epi.dmask, epi.dact, repair);
   }
   int r = e == cudaSuccess ? check_launch("gemm_tc")
                            : set_error(VKC_ERR_CUDA, "gemm_tc launch: %s", cudaGetErrorString(e));
   if (r == VKC_OK && splits > 1 && clusters == 0)
-    r = splitk_reduce(dev, partial, splits, M, N, alpha, beta, C, ldc, epi, out);
+    r = splitk_reduce(dev, partial, splits, M, N, alpha, beta, C, ldc, epi, out, ro);
+  else if (r == VKC_OK && PARTS == 3)
+    r = gemm_repair(dev, ro, M, N, alpha, beta, C, ldc, epi, repair);
   else if (r == VKC_OK && out)  // no reduction launch to write it: the pre-pass kernel on C
-    r = split_operands(dev, C, M, ldc, true, out->hi, out->lo, nullptr, 0, 0, true, nullptr, nullptr, N, out->ldk);
+    r = split_operands<2>(dev, C, M, ldc, true, out->hi, out->lo, nullptr, 0, 0, true, nullptr, nullptr, N, out->ldk);
   scratch_free(dev, partial);
   return r;
 }
@@ -937,7 +1119,7 @@ namespace vkc {
 int tc_split_operands(vkc_device_t dev, const float* A, int64_t M, int64_t lda, bool a_kcontig,
                       __nv_bfloat16* a_hi, __nv_bfloat16* a_lo, const float* B, int64_t N, int64_t ldb,
                       bool b_kcontig, __nv_bfloat16* b_hi, __nv_bfloat16* b_lo, int64_t K, int64_t Kp) {
-  return split_operands(dev, A, M, lda, a_kcontig, a_hi, a_lo, B, N, ldb, b_kcontig, b_hi, b_lo, K, Kp);
+  return split_operands<2>(dev, A, M, lda, a_kcontig, a_hi, a_lo, B, N, ldb, b_kcontig, b_hi, b_lo, K, Kp);
 }
 
 // The GEMM on operands already in K-major bf16 form ([M][Kp] and [N][Kp],
@@ -960,14 +1142,14 @@ int gemm_tc_presplit(vkc_device_t dev, int precision, int64_t M, int64_t N, int6
   if (r != VKC_OK) return r;
   // stages fill ~192 KB of shared memory
   if (x3 && plan.bn == 256)
-    return launch_tcp<true, 256, 2, kDrainX3>(dev, ma, mb, malo, mblo, M, N, K, alpha, beta, C, ldc, epi, plan.splits,
+    return launch_tcp<2, 256, 2, kDrainX3>(dev, ma, mb, malo, mblo, M, N, K, alpha, beta, C, ldc, epi, plan.splits,
                                               out);
   if (x3)
-    return launch_tcp<true, 128, 3, kDrainX3>(dev, ma, mb, malo, mblo, M, N, K, alpha, beta, C, ldc, epi, plan.splits,
+    return launch_tcp<2, 128, 3, kDrainX3>(dev, ma, mb, malo, mblo, M, N, K, alpha, beta, C, ldc, epi, plan.splits,
                                               out);
   if (plan.bn == 256)
-    return launch_tcp<false, 256, 4, 1>(dev, ma, mb, malo, mblo, M, N, K, alpha, beta, C, ldc, epi, plan.splits, out);
-  return launch_tcp<false, 128, 6, 1>(dev, ma, mb, malo, mblo, M, N, K, alpha, beta, C, ldc, epi, plan.splits, out);
+    return launch_tcp<1, 256, 4, 1>(dev, ma, mb, malo, mblo, M, N, K, alpha, beta, C, ldc, epi, plan.splits, out);
+  return launch_tcp<1, 128, 6, 1>(dev, ma, mb, malo, mblo, M, N, K, alpha, beta, C, ldc, epi, plan.splits, out);
 }
 
 int gemm_tc(vkc_device_t dev, int precision, bool ta, bool tb, int64_t M, int64_t N, int64_t K, float alpha,
@@ -993,9 +1175,50 @@ int gemm_tc(vkc_device_t dev, int precision, bool ta, bool tb, int64_t M, int64_
   __nv_bfloat16* b_lo = x3 ? a_lo + a_elems : nullptr;
   // op(A)(m,k): ta ? A[k*lda + m] : A[m*lda + k]  -> K contiguous iff !ta
   // op(B)(k,n): tb ? B[n*ldb + k] : B[k*ldb + n]  -> (n,k) K contiguous iff tb
-  r = split_operands(dev, A, M, lda, !ta, a_hi, a_lo, B, N, ldb, tb, b_hi, b_lo, K, Kp);
+  r = split_operands<2>(dev, A, M, lda, !ta, a_hi, a_lo, B, N, ldb, tb, b_hi, b_lo, K, Kp);
   if (r == VKC_OK) r = gemm_tc_presplit(dev, precision, M, N, K, alpha, a_hi, a_lo, b_hi, b_lo, beta, C, ldc, epi,
                                         nullptr);
+  scratch_free(dev, scratch);
+  return r;
+}
+
+int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t K, float alpha, const float* A,
+              int64_t lda, const float* B, int64_t ldb, float beta, float* C, int64_t ldc, GemmEpilogue epi) {
+  GemmEpilogue plain = epi;
+  plain.dmask = nullptr;
+  plain.dact = VKC_ACT_NONE;
+  auto simt = [&]() {
+    int r = gemm_simt(dev, ta, tb, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, plain);
+    return r == VKC_OK ? act_deriv_after(dev, epi, C, M, N, ldc) : r;
+  };
+  const int ranges = simt_splits(dev, M, N, K);
+  if (!fp32_on_tensor_cores(M, N, K, ranges)) return simt();
+  const int64_t Kp = (K + kBK - 1) / kBK * kBK;
+  const int64_t blocks = ((M + 31) / 32) * ((N + 31) / 32);
+  const size_t elems = 3 * (size_t)(M + N) * Kp;
+  const size_t list = (elems * sizeof(__nv_bfloat16) + 15) / 16 * 16;
+  void* scratch = nullptr;
+  if (scratch_alloc(dev, list + (size_t)(1 + blocks) * 4, &scratch) != VKC_OK) {
+    // no room for the operands' copies: the SIMT GEMM reads them in place
+    clear_error();
+    return simt();
+  }
+  auto* a = static_cast<__nv_bfloat16*>(scratch);
+  auto* b = a + 3 * (size_t)M * Kp;
+  auto* repair = reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + list);
+  int r = split_operands<3>(dev, A, M, lda, !ta, a, nullptr, B, N, ldb, tb, b, nullptr, K, Kp, repair);
+  CUtensorMap ma, mb;
+  if (r == VKC_OK) r = make_map(&ma, a, 3 * M, Kp, kBM);
+  if (r == VKC_OK) r = make_map(&mb, b, 3 * N, Kp, 128);
+  const int splits = std::min<int>(ranges, (int)(Kp / kBK));
+  if (r == VKC_OK)
+    // K in short ranges: two hi*hi accumulations per K block (256^3 in 4
+    // ranges, U[0,1) data: error 8.0e-8 -> 5.5e-8, where FMAs in 16 ranges of
+    // 16 gave 6.1e-8); else one, which drains half as often (2048^3 in 2
+    // ranges: 128 -> 114 us) and which the grouped kernel reproduces
+    r = (splits > 1 && Kp / splits <= 256 ? launch_tcp<3, 128, 2, 2> : launch_tcp<3, 128, 2, 1>)(
+        dev, ma, mb, ma, mb, M, N, K, alpha, beta, C, ldc, epi, splits, nullptr,
+        RepairOperands{A, B, lda, ldb, K, ta ? 1 : 0, tb ? 1 : 0}, repair);
   scratch_free(dev, scratch);
   return r;
 }

@@ -23,6 +23,32 @@ int gemm_tc(vkc_device_t dev, int precision, bool ta, bool tb, int64_t M, int64_
             const float* A, int64_t lda, const float* B, int64_t ldb, float beta, float* C, int64_t ldc,
             GemmEpilogue epi);
 
+// Whether a plain fp32 product runs as six bf16 tensor-core products (three
+// exact parts per operand) instead of fp32 FMAs in `splits` K ranges.
+// The FMA GEMM's time is its chain of K steps (0.115 us per step, 2.5 us of
+// launch, 3.5 us more for the reduction of several ranges) until the output
+// fills the GPU several times over; the tensor path's three launches cost 8 us
+// with one K block.  Measured (us, FMA -> tensor, graph replay): 256 x 256 x
+// 64 10.9 -> 9.4, 128^3 17.5 -> 10.4, 300^3 (19 ranges of 16) 12.6 -> 11.2,
+// 256^3 (16 ranges of 16) 9.3 -> 10.9, 1024 x 1024 x 48 9.2 -> 9.6, 4096 x
+// 4096 x 16 30.6 -> 27.9.  Run call by call the third launch costs another 1.5
+// us of host time, hence 96 steps rather than 64.
+inline bool fp32_on_tensor_cores(int64_t M, int64_t N, int64_t K, int splits) {
+  if (M < 2 || N < 2 || K < 16) return false;                            // vectors are bound by reading the matrix
+  if (M > (1 << 22) || N > (1 << 22) || K >= (1ll << 31)) return false;  // 32-bit tile and row coordinates
+  const int64_t chain = (K + splits - 1) / splits;
+  return chain + (splits > 1 ? 32 : 0) >= 96 || M * N >= (1 << 24);
+}
+
+// C = act(alpha * op(A) op(B) + beta * C + bias) (* act'(dmask)) in fp32: on
+// the tensor cores or with FMAs, by fp32_on_tensor_cores.
+int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t K, float alpha, const float* A,
+              int64_t lda, const float* B, int64_t ldb, float beta, float* C, int64_t ldc, GemmEpilogue epi);
+
+// C *= act'(epi.dmask) as a launch of its own, after a GEMM that could not
+// apply it (nn.cu).
+int act_deriv_after(vkc_device_t dev, const GemmEpilogue& epi, float* C, int64_t M, int64_t N, int64_t ldc);
+
 // gemm_tc on operands already split ([M][Kp] and [N][Kp] K-major bf16, Kp =
 // K rounded up to 64, zero past K); `out` (may be NULL) also receives C in
 // that form (pitch out->ldk, zero from N on).  M, N, K > 0.

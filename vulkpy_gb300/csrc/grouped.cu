@@ -8,8 +8,10 @@
 // Here the output tiles of all problems form one work list, ordered by K
 // (longest first), and a persistent grid walks it round-robin.
 //
-// fp32: each tile is computed by the same code as the single-problem SIMT
-// kernel (simt_tile), so results are bit-identical to vkc_gemm.
+// fp32: problems that vkc_gemm computes with FMAs use the same code per tile
+// (simt_tile); those it computes as three-part tensor-core products run in
+// the tensor-core kernel here too, with the same sums; either way results
+// are bit-identical to vkc_gemm when that call does not split K.
 // bf16 / split-bf16x3: a pre-pass converts every operand into 128 x 64 bf16
 // tiles already laid out as the 128-byte-swizzled shared-memory image the
 // MMA descriptors expect (tile (r, k): row r's 16-byte chunk c at byte
@@ -20,7 +22,9 @@
 // order), so split-bf16x3 results are bit-identical to vkc_gemm when that call
 // does not split K.
 #include "colsum.cuh"
+#include "gemm_repair.cuh"
 #include "gemm_simt.cuh"
+#include "gemm_tc.cuh"
 #include "tc_ptx.cuh"
 #include "tc_epilogue.cuh"
 
@@ -45,7 +49,7 @@ struct SimtProb {
   int64_t lda, ldb, ldc;
   int64_t m, n, k;
   float alpha, beta;
-  int act, trans;  // trans: bit0 op(A) = A^T, bit1 op(B) = B^T
+  int act, trans;  // trans: bit0 op(A) = A^T, bit1 op(B) = B^T; bit2: tiles of C^T (repair only)
   int tiles_n, tile0;
 };
 
@@ -105,6 +109,7 @@ struct TileOp {
   const float* src;
   __nv_bfloat16* hi;
   __nv_bfloat16* lo;  // NULL: plain bf16
+  __nv_bfloat16* mid; // three parts (fp32 products); NULL: two or one
   int64_t ld;
   int64_t rows, k;    // logical operand: rows x k, element (r, k)
   int k_contig;       // element (r, k) at src[r*ld + k]; else src[k*ld + r]
@@ -119,11 +124,14 @@ struct TileTable {
 
 // One 128 x 64 tile per block iteration: load (coalesced along whichever
 // index is contiguous) into shared memory, then write 16-byte chunks of hi
-// (and lo = bf16(x - hi)) at their swizzled positions.  Rows >= rows and
-// k >= K are written as zeros.
-__global__ void __launch_bounds__(256, 3) k_tile_operands(const __grid_constant__ TileTable tab) {
+// (and lo = bf16(x - hi), or mid and lo) at their swizzled positions.  Rows
+// >= rows and k >= K are written as zeros.  THREE: three parts; `repair` is
+// then the count of blocks left to k_gemm_repair_grouped, zeroed here.
+template <bool THREE>
+__global__ void __launch_bounds__(256, 3) k_tile_operands(const __grid_constant__ TileTable tab, uint32_t* repair) {
   __shared__ float s[kTileRows][kTileK + 1];
   const int tid = threadIdx.x;
+  if (THREE && blockIdx.x == 0 && tid == 0) *repair = 0u;
   for (int t = blockIdx.x; t < tab.total; t += gridDim.x) {
     const TileOp& op = tab.op[find_problem(tab.op, tab.count, t)];
     const int local = t - op.tile0;
@@ -165,11 +173,29 @@ __global__ void __launch_bounds__(256, 3) k_tile_operands(const __grid_constant_
     const size_t tile_elems = (size_t)local * (kTileRows * kTileK);
     uint8_t* hi = reinterpret_cast<uint8_t*>(op.hi + tile_elems);
     uint8_t* lo = op.lo ? reinterpret_cast<uint8_t*>(op.lo + tile_elems) : nullptr;
+    uint8_t* mid = THREE ? reinterpret_cast<uint8_t*>(op.mid + tile_elems) : nullptr;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int cidx = i * 256 + tid;  // 128 rows x 8 chunks of 8 elements
       const int r = cidx >> 3, c = cidx & 7;
       uint32_t h[4], l[4];
+      const size_t off = (size_t)r * 128 + (size_t)(((c ^ (r & 7)) << 4));
+      if (THREE) {
+        uint32_t m[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          __nv_bfloat16 h0, m0, l0, h1, m1, l1;
+          split_bf16_3(s[r][c * 8 + 2 * j], h0, m0, l0);
+          split_bf16_3(s[r][c * 8 + 2 * j + 1], h1, m1, l1);
+          h[j] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
+          m[j] = (uint32_t)__bfloat16_as_ushort(m0) | ((uint32_t)__bfloat16_as_ushort(m1) << 16);
+          l[j] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
+        }
+        *reinterpret_cast<uint4*>(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
+        *reinterpret_cast<uint4*>(mid + off) = make_uint4(m[0], m[1], m[2], m[3]);
+        *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
+        continue;
+      }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float x0 = s[r][c * 8 + 2 * j], x1 = s[r][c * 8 + 2 * j + 1];
@@ -179,7 +205,6 @@ __global__ void __launch_bounds__(256, 3) k_tile_operands(const __grid_constant_
         h[j] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
         l[j] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
       }
-      const size_t off = (size_t)r * 128 + (size_t)(((c ^ (r & 7)) << 4));
       *reinterpret_cast<uint4*>(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
       if (lo) *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
     }
@@ -200,6 +225,8 @@ struct TcProb {
   const uint8_t* a_lo;
   const uint8_t* b_hi;  // tiles of the kernel's B side: [nk/128][K/64] x 16 KB
   const uint8_t* b_lo;
+  const uint8_t* a_mid;
+  const uint8_t* b_mid;
   float* c;
   const float* bias;
   const float* mask;
@@ -234,30 +261,37 @@ struct TcTable {
   TcProb p[kMaxGroup];
 };
 
-constexpr int kGroupedStages = 3;
+constexpr int grouped_stages(int parts) { return parts == 3 ? 2 : 3; }
 // warps: 0 producer, 1 TMEM owner + MMA issuer, 2..9 epilogue (two per TMEM
 // lane quarter, 64 columns each: the per-tile epilogue is the critical path
 // of the short-K tiles, so it gets eight warps)
 constexpr int kGroupedEpiWarps = 8;
 constexpr int kThreadsGrouped = 32 * (2 + kGroupedEpiWarps);
 
-template <bool X3>
+template <int PARTS>
 struct GroupedCfg {
-  static constexpr uint32_t kStageBytes = (X3 ? 4u : 2u) * kTileBytes;
-  static constexpr uint32_t kBarBytes = 8u * (2 * kGroupedStages + 2 * kAccBufs + 1) + 16;
-  static constexpr uint32_t kEpiOff = kGroupedStages * kStageBytes + (kBarBytes + 127) / 128 * 128;
+  static constexpr int kStages = grouped_stages(PARTS);
+  static constexpr uint32_t kStageBytes = 2u * PARTS * kTileBytes;
+  static constexpr uint32_t kBarBytes = 8u * (2 * kStages + 2 * kAccBufs + 1) + 16;
+  static constexpr uint32_t kEpiOff = kStages * kStageBytes + (kBarBytes + 127) / 128 * 128;
   static constexpr uint32_t kSmem = kEpiOff + kGroupedEpiWarps * kEpiStageBytes + 1024;
 };
 
 // One CTA per SM walks the tile list.  The stage ring and the TMEM buffer
 // ring continue across tiles (a running K-block counter gives every slot and
 // parity), so the next tile's copies and MMAs overlap this tile's epilogue.
-template <bool X3>
+// PARTS == 3 (fp32): hi*hi products use TMEM buffers 0 and 1, one
+// accumulation per K block; the five small ones buffers 2 and 3, one per
+// kLoSpan blocks (their "full" barriers are not needed: a block's hi*hi commit
+// covers them).  repair: as k_gemm_tcp, entries are 16 * tile + 4 * lane
+// quarter + 32-column chunk.
+template <int PARTS>
 __global__ void __launch_bounds__(kThreadsGrouped, 1)
-k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err) {
+k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err, uint32_t* __restrict__ repair) {
   constexpr int BN = 128;
-  constexpr int S = kGroupedStages;
-  using Cfg = GroupedCfg<X3>;
+  constexpr bool X3 = PARTS > 1;
+  using Cfg = GroupedCfg<PARTS>;
+  constexpr int S = Cfg::kStages;
   constexpr uint32_t kCols = BN * kAccBufs;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -315,13 +349,17 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err) {
       for (int kb = 0; kb < P.kt; ++kb, ++g) {
         const int s = g % S;
         if (*abort_flag || !mbar_wait(empty_bar(s), ((g / S) & 1) ^ 1)) { ok = false; break; }
-        mbar_expect_tx(full_bar(s), (X3 ? 2u : 1u) * (kTileBytes + b_bytes));
+        mbar_expect_tx(full_bar(s), (uint32_t)PARTS * (kTileBytes + b_bytes));
         const size_t kofs = (size_t)kb * kTileBytes;
         bulk_load(stage(s, 0), P.a_hi + a_off + kofs, kTileBytes, full_bar(s));
         bulk_load(stage(s, 1), P.b_hi + b_off + kofs, b_bytes, full_bar(s));
         if (X3) {
           bulk_load(stage(s, 2), P.a_lo + a_off + kofs, kTileBytes, full_bar(s));
           bulk_load(stage(s, 3), P.b_lo + b_off + kofs, b_bytes, full_bar(s));
+        }
+        if (PARTS == 3) {
+          bulk_load(stage(s, 4), P.a_mid + a_off + kofs, kTileBytes, full_bar(s));
+          bulk_load(stage(s, 5), P.b_mid + b_off + kofs, b_bytes, full_bar(s));
         }
       }
     }
@@ -335,12 +373,45 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err) {
   } else if (warp == 1 && lane == 0) {
     // ---------------- MMA issuer
     uint32_t g = 0, acc = 0;  // g: K blocks (stage ring), acc: accumulations (TMEM ring)
+    uint32_t lo_it = 0;       // PARTS == 3: accumulations of small products
     bool ok = true;
     for (int t = blockIdx.x; t < tab.total && ok; t += gridDim.x) {
       const TcProb& P = tab.p[find_problem(tab.p, tab.count, t)];
       const int bn = tile_bn(P, ((t - P.tile0) % P.tiles_n) * BN);
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) |
                              ((uint32_t)(kTileRows >> 4) << 24);
+      if constexpr (PARTS == 3) {
+        // stage tiles: 0 a_hi, 1 b_hi, 2 a_lo, 3 b_lo, 4 a_mid, 5 b_mid; the
+        // products in k_gemm_tcp's order (hi*mid before mid*hi in terms of
+        // op(A), op(B), which change sides in a swapped problem)
+        for (int kb = 0; kb < P.kt && ok; ++kb, ++g, ++acc) {
+          const int s = g % S, b = acc & 1, lb = 2 + (lo_it & 1);
+          const bool lo_first = kb % kLoSpan == 0, lo_last = kb % kLoSpan == kLoSpan - 1 || kb == P.kt - 1;
+          if (*abort_flag || (lo_first && !mbar_wait(acce_bar(lb), ((lo_it >> 1) & 1) ^ 1)) ||
+              !mbar_wait(acce_bar(b), ((acc >> 1) & 1) ^ 1) || !mbar_wait(full_bar(s), (g / S) & 1)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const int ksteps = kb == P.kt - 1 ? P.klast : kTileK / 16;
+          const uint32_t d_lo = tmem + (uint32_t)(lb * BN), d_hi = tmem + (uint32_t)(b * BN);
+          constexpr int ta[5] = {4, 0, 4, 0, 2}, tb[5] = {5, 5, 1, 3, 1};          // mm hm mh hl lh
+          constexpr int sa[5] = {4, 4, 0, 2, 0}, sb[5] = {5, 1, 5, 1, 3};          // swapped sides
+#pragma unroll
+          for (int i = 0; i < 5; ++i) {
+            const uint32_t wa = (uint32_t)(P.swap ? sa[i] : ta[i]), wb = (uint32_t)(P.swap ? sb[i] : tb[i]);
+            for (int k = 0; k < ksteps; ++k)
+              mma_bf16(d_lo, sw128_desc(stage(s, wa) + 32u * k), sw128_desc(stage(s, wb) + 32u * k), idesc,
+                       (i == 0 && k == 0 && lo_first) ? 0u : 1u);
+          }
+          for (int k = 0; k < ksteps; ++k)
+            mma_bf16(d_hi, sw128_desc(stage(s, 0) + 32u * k), sw128_desc(stage(s, 1) + 32u * k), idesc, k ? 1u : 0u);
+          mma_commit(empty_bar(s));
+          mma_commit(accf_bar(b));
+          if (lo_last) ++lo_it;
+        }
+        continue;
+      }
       const int span = X3 ? kDrainX3 : P.kt;  // K blocks per TMEM accumulation
       for (int g0 = 0; g0 < P.kt && ok; g0 += span, ++acc) {
         const int b = acc % kAccBufs;
@@ -396,7 +467,7 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err) {
     const int q = warp & 3;           // TMEM lane quarter
     const int hc = (warp - 2) >> 2;   // column half
     const uint32_t lane_addr = ((uint32_t)(q * 32) << 16) + (uint32_t)(hc * CW);
-    uint32_t g = 0;
+    uint32_t g = 0, lo_it = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < tab.total && ok; t += gridDim.x) {
       const TcProb& P = tab.p[find_problem(tab.p, tab.count, t)];
@@ -415,7 +486,7 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err) {
           for (int r = n0 + lane; r < min(n0 + CW, P.m); r += 32) prefetch_seg_l2(aux, P.ldc, r, c0, c1);
         }
       }
-      const int span = X3 ? kDrainX3 : P.kt;
+      const int span = PARTS == 3 ? 1 : X3 ? kDrainX3 : P.kt;
       const int ngroups = (P.kt + span - 1) / span;
       float sum[X3 ? CW : 1];
       if (X3) {
@@ -424,10 +495,38 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err) {
       }
       int b = 0;
       for (int gi = 0; gi < ngroups; ++gi, ++g) {
-        b = g % kAccBufs;
-        if (*abort_flag || !mbar_wait(accf_bar(b), (g / kAccBufs) & 1)) { ok = false; break; }
+        constexpr int RING = PARTS == 3 ? 2 : kAccBufs;
+        b = g % RING;
+        if (*abort_flag || !mbar_wait(accf_bar(b), (g / RING) & 1)) { ok = false; break; }
         tc_fence_after();
-        if (X3 && ngroups > 1) {  // one accumulation: the store loop reads it from TMEM as it is
+        if constexpr (PARTS == 3) {  // as k_gemm_tcp
+          const bool last = gi == ngroups - 1, with_lo = last || (gi + 1) % kLoSpan == 0;
+          const int lb = 2 + (lo_it & 1);
+#pragma unroll
+          for (int c = 0; c < CW / 32; ++c) {
+            const uint32_t ta = tmem + lane_addr + (uint32_t)(b * BN + c * 32);
+            uint32_t r0[32];
+            if (with_lo) {
+              tmem_ld32(ta + (uint32_t)((lb - b) * BN), r0);
+#pragma unroll
+              for (int j = 0; j < 32; ++j) sum[c * 32 + j] += __uint_as_float(r0[j]);
+            }
+            tmem_ld32(ta, r0);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              sum[c * 32 + j] += __uint_as_float(r0[j]);
+              r0[j] = __float_as_uint(sum[c * 32 + j]);
+            }
+            if (last) tmem_st32_nw(ta, r0);
+          }
+          if (last) tmem_wait_st();
+          if (with_lo) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acce_bar(lb));
+            ++lo_it;
+          }
+        } else if (X3 && ngroups > 1) {  // one accumulation: the store loop reads it from TMEM as it is
           const bool last = gi == ngroups - 1;
 #pragma unroll
           for (int c = 0; c < CW / 32; c += 2) {
@@ -464,6 +563,13 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err) {
         if (col0 >= P.nk) break;
         uint32_t r[32];
         tmem_ld32(tmem + lane_addr + (uint32_t)(b * BN + c * 32), r);
+        if (PARTS == 3 && m0 + q * 32 < (P.swap ? P.n : P.m)) {
+          // results that are not finite are left to k_gemm_repair_grouped
+          if (!block_finite(r, m0 + q * 32 + lane < (P.swap ? P.n : P.m), P.nk - col0)) {
+            if (lane == 0) repair[1 + atomicAdd(repair, 1u)] = (uint32_t)t * 16u + (uint32_t)(q * 4 + hc * 2 + c);
+            continue;
+          }
+        }
         if (P.swap) {
           // lanes are columns of C (kernel rows), TMEM columns rows of C
           if (m0 + q * 32 < P.n)
@@ -496,6 +602,26 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err) {
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
+  }
+}
+
+// The blocks that k_gemm_tc_grouped<3> left, from the fp32 operands.
+__global__ void __launch_bounds__(256)
+k_gemm_repair_grouped(const __grid_constant__ SimtTable tab, const uint32_t* list) {
+  __shared__ RepairSmem sm;
+  const uint32_t count = list[0];
+  for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+    const int t = (int)(list[1 + i] >> 4), q = (int)(list[1 + i] >> 2) & 3, c = (int)list[1 + i] & 3;
+    const SimtProb& P = tab.p[find_problem(tab.p, tab.count, t)];
+    const int local = t - P.tile0;
+    // kernel coordinates; a swapped problem's are those of C^T
+    const int64_t r0 = (int64_t)(local / P.tiles_n) * kTileRows + q * 32;
+    const int64_t c0 = (int64_t)(local % P.tiles_n) * 128 + c * 32;
+    const int64_t m0 = P.trans & 4 ? c0 : r0, n0 = P.trans & 4 ? r0 : c0;
+    const RepairOperands o{P.a, P.b, P.lda, P.ldb, P.k, P.trans & 1, (P.trans >> 1) & 1};
+    float acc[4];
+    repair_block(o, P.m, P.n, m0, n0, sm, acc);
+    repair_store(acc, P.m, P.n, m0, n0, P.alpha, P.beta, P.c, P.ldc, P.bias, P.act, P.mask, VKC_ACT_RELU);
   }
 }
 
@@ -854,27 +980,39 @@ int grouped_simt(vkc_device_t dev, const vkc_gemm_problem* probs, const std::vec
   return VKC_OK;
 }
 
-int grouped_tc(vkc_device_t dev, bool x3, const vkc_gemm_problem* probs, const vkc_gemm_update* upd,
+template <int PARTS>
+int grouped_tc(vkc_device_t dev, const vkc_gemm_problem* probs, const vkc_gemm_update* upd,
                const std::vector<int>& order) {
   for (size_t s = 0; s < order.size(); s += kMaxGroup) {
     const size_t e = std::min(order.size(), s + kMaxGroup);
     // operand tile buffers: one allocation for the chunk
     std::vector<size_t> a_off, b_off;
-    size_t bytes = 0;
+    size_t bytes = 0, ctiles = 0;
     for (size_t j = s; j < e; ++j) {
       const vkc_gemm_problem& q = probs[order[j]];
       const size_t kt = (size_t)((q.k + kTileK - 1) / kTileK);
       const size_t at = (size_t)((q.m + kTileRows - 1) / kTileRows) * kt;
       const size_t bt = (size_t)((q.n + kTileRows - 1) / kTileRows) * kt;
       a_off.push_back(bytes);
-      bytes += at * kTileBytes * (x3 ? 2 : 1);
+      bytes += at * kTileBytes * PARTS;
       b_off.push_back(bytes);
-      bytes += bt * kTileBytes * (x3 ? 2 : 1);
+      bytes += bt * kTileBytes * PARTS;
+      ctiles += (size_t)((q.m + kTileRows - 1) / kTileRows) * (size_t)((q.n + 127) / 128);
     }
+    const size_t list = bytes;  // bytes is a multiple of 16 KB
+    if (PARTS == 3) bytes += 4 * (1 + 16 * ctiles);
     void* scratch = nullptr;
     int r = scratch_alloc(dev, bytes, &scratch);
+    if (r != VKC_OK && PARTS == 3) {
+      // no room for the operands' copies: the SIMT kernel reads them in place
+      clear_error();
+      r = grouped_simt(dev, probs, std::vector<int>(order.begin() + (long)s, order.begin() + (long)e));
+      if (r == VKC_OK) continue;
+    }
     if (r != VKC_OK) return r;
     uint8_t* sbase = static_cast<uint8_t*>(scratch);
+    uint32_t* repair = PARTS == 3 ? reinterpret_cast<uint32_t*>(sbase + list) : nullptr;
+    SimtTable rt{};  // PARTS == 3: the problems as the repair kernel needs them
 
     TileTable tt{};
     TcTable tab{};
@@ -884,14 +1022,18 @@ int grouped_tc(vkc_device_t dev, bool x3, const vkc_gemm_problem* probs, const v
       const int kt = (int)((q.k + kTileK - 1) / kTileK);
       const int mt = (int)((q.m + kTileRows - 1) / kTileRows), nt = (int)((q.n + kTileRows - 1) / kTileRows);
       uint8_t* a_hi = sbase + a_off[j - s];
-      uint8_t* a_lo = x3 ? a_hi + (size_t)mt * kt * kTileBytes : nullptr;
+      const size_t a_part = (size_t)mt * kt * kTileBytes, b_part = (size_t)nt * kt * kTileBytes;
+      uint8_t* a_lo = PARTS > 1 ? a_hi + a_part : nullptr;
+      uint8_t* a_mid = PARTS == 3 ? a_hi + 2 * a_part : nullptr;
       uint8_t* b_hi = sbase + b_off[j - s];
-      uint8_t* b_lo = x3 ? b_hi + (size_t)nt * kt * kTileBytes : nullptr;
+      uint8_t* b_lo = PARTS > 1 ? b_hi + b_part : nullptr;
+      uint8_t* b_mid = PARTS == 3 ? b_hi + 2 * b_part : nullptr;
       // op(A)(m, k): ta ? A[k*lda + m] : A[m*lda + k]  -> K contiguous iff !ta
       TileOp& oa = tt.op[tt.count++];
       oa.src = q.a;
       oa.hi = reinterpret_cast<__nv_bfloat16*>(a_hi);
       oa.lo = reinterpret_cast<__nv_bfloat16*>(a_lo);
+      oa.mid = reinterpret_cast<__nv_bfloat16*>(a_mid);
       oa.ld = q.lda;
       oa.rows = q.m;
       oa.k = q.k;
@@ -904,6 +1046,7 @@ int grouped_tc(vkc_device_t dev, bool x3, const vkc_gemm_problem* probs, const v
       ob.src = q.b;
       ob.hi = reinterpret_cast<__nv_bfloat16*>(b_hi);
       ob.lo = reinterpret_cast<__nv_bfloat16*>(b_lo);
+      ob.mid = reinterpret_cast<__nv_bfloat16*>(b_mid);
       ob.ld = q.ldb;
       ob.rows = q.n;
       ob.k = q.k;
@@ -919,6 +1062,8 @@ int grouped_tc(vkc_device_t dev, bool x3, const vkc_gemm_problem* probs, const v
       P.a_lo = swap ? b_lo : a_lo;
       P.b_hi = swap ? a_hi : b_hi;
       P.b_lo = swap ? a_lo : b_lo;
+      P.a_mid = swap ? b_mid : a_mid;
+      P.b_mid = swap ? a_mid : b_mid;
       P.nk = (int)(swap ? q.m : q.n);
       P.klast = (int)(((q.k - (int64_t)(kt - 1) * kTileK) + 15) / 16);
       P.c = q.c;
@@ -935,33 +1080,48 @@ int grouped_tc(vkc_device_t dev, bool x3, const vkc_gemm_problem* probs, const v
       P.tile0 = total;
       P.upd = upd ? upd[order[j]].value : nullptr;
       P.upd_scale = upd ? upd[order[j]].scale : 0.f;
+      if (PARTS == 3) {
+        SimtProb& S = rt.p[rt.count++];
+        S.a = q.a;
+        S.b = q.b;
+        S.c = q.c;
+        S.bias = q.bias;
+        S.mask = q.relu_mask;
+        S.lda = q.lda;
+        S.ldb = q.ldb;
+        S.ldc = q.ldc;
+        S.m = q.m;
+        S.n = q.n;
+        S.k = q.k;
+        S.alpha = q.alpha;
+        S.beta = q.beta;
+        S.act = q.act;
+        S.trans = (q.ta ? 1 : 0) | (q.tb ? 2 : 0) | (swap ? 4 : 0);
+        S.tiles_n = P.tiles_n;
+        S.tile0 = P.tile0;
+      }
       total += mt * nt;
     }
     tt.total = ttotal;
     tab.total = total;
-    const unsigned tgrid = wave_grid(dev, k_tile_operands, (size_t)ttotal * 256, 256);
-    k_tile_operands<<<tgrid, 256, 0, dev->stream>>>(tt);
+    const unsigned tgrid = wave_grid(dev, k_tile_operands<PARTS == 3>, (size_t)ttotal * 256, 256);
+    k_tile_operands<PARTS == 3><<<tgrid, 256, 0, dev->stream>>>(tt, repair);
     r = check_launch("gemm_grouped tiling");
     if (r == VKC_OK) {
       const unsigned grid = (unsigned)std::min<int>(total, dev->sm_count);
-      if (x3) {
-        static bool attr = false;
-        if (!attr) {
-          cudaFuncSetAttribute(k_gemm_tc_grouped<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               GroupedCfg<true>::kSmem);
-          attr = true;
-        }
-        k_gemm_tc_grouped<true><<<grid, kThreadsGrouped, GroupedCfg<true>::kSmem, dev->stream>>>(tab, dev->err_word);
-      } else {
-        static bool attr = false;
-        if (!attr) {
-          cudaFuncSetAttribute(k_gemm_tc_grouped<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               GroupedCfg<false>::kSmem);
-          attr = true;
-        }
-        k_gemm_tc_grouped<false><<<grid, kThreadsGrouped, GroupedCfg<false>::kSmem, dev->stream>>>(tab, dev->err_word);
+      using Cfg = GroupedCfg<PARTS>;
+      static bool attr = false;
+      if (!attr) {
+        cudaFuncSetAttribute(k_gemm_tc_grouped<PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
+        attr = true;
       }
+      k_gemm_tc_grouped<PARTS><<<grid, kThreadsGrouped, Cfg::kSmem, dev->stream>>>(tab, dev->err_word, repair);
       r = check_launch("gemm_grouped (tensor cores)");
+      if (r == VKC_OK && PARTS == 3) {
+        rt.total = total;
+        k_gemm_repair_grouped<<<(unsigned)dev->sm_count, 256, 0, dev->stream>>>(rt, repair);
+        r = check_launch("gemm_grouped repair");
+      }
     }
     scratch_free(dev, scratch);
     if (r != VKC_OK) return r;
@@ -997,17 +1157,27 @@ int gemm_grouped(vkc_device_t dev, int precision, const vkc_gemm_problem* proble
   std::vector<int> order = work_order(problems, count);
   std::vector<int> tc, simt;
   // K = 0 has no tensor-core work: C = act(beta*C + bias) through the SIMT path
-  for (int i : order) (precision != VKC_MM_FP32 && problems[i].k > 0 ? tc : simt).push_back(i);
+  // fp32: as vkc_gemm without a split of K decides
+  for (int i : order) {
+    const vkc_gemm_problem& q = problems[i];
+    const bool on_tc = precision == VKC_MM_FP32 ? fp32_on_tensor_cores(q.m, q.n, q.k, 1) : q.k > 0;
+    (on_tc ? tc : simt).push_back(i);
+  }
   // Another problem may read an updated value as its operand (dx = dy W
   // beside dW's step): the tensor-core path reads operands only in its
   // tiling pass before the GEMM, so the step can run in the epilogue when all
   // its problems go in one launch; the SIMT path reads them in the GEMM, so
   // its steps (and those of a tensor-core call of several launches) run as
   // one separate update after every product.
-  const bool fuse = updates && tc.size() <= (size_t)kMaxGroup;
+  // fp32 results may be recomputed from the operands after the GEMM, so its
+  // steps are separate too.
+  const bool fuse = updates && precision != VKC_MM_FP32 && tc.size() <= (size_t)kMaxGroup;
   int r = grouped_simt(dev, problems, simt);
   if (r != VKC_OK) return r;
-  r = grouped_tc(dev, precision == VKC_MM_BF16X3, problems, fuse ? updates : nullptr, tc);
+  const vkc_gemm_update* in_gemm = fuse ? updates : nullptr;
+  r = precision == VKC_MM_FP32     ? grouped_tc<3>(dev, problems, in_gemm, tc)
+      : precision == VKC_MM_BF16X3 ? grouped_tc<2>(dev, problems, in_gemm, tc)
+                                   : grouped_tc<1>(dev, problems, in_gemm, tc);
   if (r != VKC_OK || !updates) return r;
   std::vector<float*> val;
   std::vector<const float*> grad;

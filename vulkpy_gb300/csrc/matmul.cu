@@ -21,7 +21,7 @@ VKC_EXPORT int vkc_gemm(vkc_device_t dev, int precision, int trans_a, int trans_
   }
   switch (precision) {
     case VKC_MM_FP32:
-      return vkc::gemm_simt(dev, trans_a != 0, trans_b != 0, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc,
+      return vkc::gemm_fp32(dev, trans_a != 0, trans_b != 0, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc,
                             vkc::GemmEpilogue{});
     case VKC_MM_BF16:
     case VKC_MM_BF16X3:

@@ -27,23 +27,32 @@ __device__ __forceinline__ float act_bwd(float yi, float dyi);
 template <int ACT>
 __global__ void __launch_bounds__(kThreads) k_act_backward(const float* y, const float* dy, float* dx, size_t n);
 
+}  // namespace
+
+namespace vkc {
+
 // C *= act'(epi.dmask) elementwise after a GEMM that could not apply it in
 // its epilogue (C contiguous: ldc == N); in place, the separate
 // activation-backward kernel's arithmetic.
-int act_deriv_after(vkc_device_t dev, const vkc::GemmEpilogue& epi, float* C, int64_t M, int64_t N, int64_t ldc) {
+int act_deriv_after(vkc_device_t dev, const GemmEpilogue& epi, float* C, int64_t M, int64_t N, int64_t ldc) {
   if (epi.dact == VKC_ACT_NONE || M == 0 || N == 0) return VKC_OK;
   VKC_REQUIRE(ldc == N, "activation derivative after a GEMM needs a contiguous C");
   const size_t n = (size_t)(M * N);
-  const unsigned grid = vkc::stream_grid(dev, n, kThreads);
+  const unsigned grid = stream_grid(dev, n, kThreads);
   if (epi.dact == VKC_ACT_RELU)
     k_act_backward<VKC_ACT_RELU><<<grid, kThreads, 0, dev->stream>>>(epi.dmask, C, C, n);
   else
     k_act_backward<VKC_ACT_SIGMOID><<<grid, kThreads, 0, dev->stream>>>(epi.dmask, C, C, n);
-  return vkc::check_launch("gemm activation derivative");
+  return check_launch("gemm activation derivative");
 }
 
+}  // namespace vkc
+
+namespace {
+
 // The tensor-core GEMM applies epi.dmask/dact in its epilogue (or split-K
-// reduction); the GEMV and SIMT paths run the derivative as one more launch.
+// reduction), for fp32 too where it runs there; the GEMV and SIMT paths run
+// the derivative as one more launch.
 int gemm_any(vkc_device_t dev, int precision, bool ta, bool tb, int64_t M, int64_t N, int64_t K, float alpha,
              const float* A, int64_t lda, const float* B, int64_t ldb, float beta, float* C, int64_t ldc,
              vkc::GemmEpilogue epi) {
@@ -52,11 +61,13 @@ int gemm_any(vkc_device_t dev, int precision, bool ta, bool tb, int64_t M, int64
   plain.dact = VKC_ACT_NONE;
   if (precision == VKC_MM_FP32 || precision == VKC_MM_BF16 || precision == VKC_MM_BF16X3) {
     const int r = vkc::gemm_as_gemv(dev, ta, tb, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, plain);
-    if (r >= 0) return r == VKC_OK ? act_deriv_after(dev, epi, C, M, N, ldc) : r;
+    if (r >= 0) return r == VKC_OK ? vkc::act_deriv_after(dev, epi, C, M, N, ldc) : r;
   }
-  if (precision == VKC_MM_FP32 || ((precision == VKC_MM_BF16 || precision == VKC_MM_BF16X3) && K == 0)) {
+  if (precision == VKC_MM_FP32)
+    return vkc::gemm_fp32(dev, ta, tb, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, epi);
+  if ((precision == VKC_MM_BF16 || precision == VKC_MM_BF16X3) && K == 0) {
     const int r = vkc::gemm_simt(dev, ta, tb, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, plain);
-    return r == VKC_OK ? act_deriv_after(dev, epi, C, M, N, ldc) : r;
+    return r == VKC_OK ? vkc::act_deriv_after(dev, epi, C, M, N, ldc) : r;
   }
   if (precision == VKC_MM_BF16 || precision == VKC_MM_BF16X3)
     return vkc::gemm_tc(dev, precision, ta, tb, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, epi);

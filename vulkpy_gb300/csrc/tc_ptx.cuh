@@ -142,6 +142,10 @@ constexpr int kAccBufs = 4;
 // so fewer drains are faster (8192^3: 398 / 432 / 439 / 457 / 499 TFLOP/s).
 constexpr int kDrainX3 = 8;
 
+// Three-part fp32 products: K blocks per accumulation of the five small
+// products (hi*hi gets one or two accumulations per block).
+constexpr int kLoSpan = 8;
+
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }

@@ -1035,9 +1035,11 @@ class Array(_GPUArray):
 
 
 def matmul(a: Array, b: Array, precision: Optional[str] = None) -> Array:
-    """``a @ b`` with an explicit arithmetic: "fp32" (SIMT FMA, the drop-in
-    default), "bf16" (tensor cores, fp32 accumulate) or "bf16x3" (split
-    bf16 on tensor cores: ~fp32 accuracy, relative error ~1e-6..1e-5)."""
+    """``a @ b`` with an explicit arithmetic: "fp32" (the drop-in default:
+    FMAs, or for larger products exact three-part bf16 operands on the tensor
+    cores, at least as accurate), "bf16" (tensor cores, fp32 accumulate) or
+    "bf16x3" (split bf16 on tensor cores: ~fp32 accuracy, relative error
+    ~1e-6..1e-5)."""
     if precision is None:
         return a @ b
     old = a._gpu.matmul_precision
