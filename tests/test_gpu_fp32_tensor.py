@@ -6,10 +6,10 @@ at most 2^-23 of the running sum; the blocks are added with round-to-nearest
 (2^-24 each).  For random data the relative Frobenius error stays below one
 accumulation's worst case, 4 * 2^-23 < 5e-7, at every K.
 
-Values outside the split (inf, NaN, |x| >= 2^127, 0 < |x| < 2^-110) reach
-only results that the kernels recompute from the fp32 operands in order of k,
-so those behave like float32 FMAs: inf and NaN where float32 arithmetic has
-them, tiny and huge values to float32 accuracy."""
+Results that values outside the split (inf, NaN, |x| >= 2^103) reach, or that
+overflow on the way (2^79 and more), are recomputed from the fp32 operands in
+order of k, so they behave like float32 FMAs: inf and NaN where float32
+arithmetic has them.  Small values, subnormals included, are split exactly."""
 import ctypes as C
 
 import numpy as np
@@ -84,7 +84,11 @@ def _poison(A, B, kind):
     elif kind == "huge":          # overflows in the sum, and hi alone would round to inf
         A[1, 3], A[40, :] = np.float32(3.4e38), np.float32(2e37)
         B[5, 2] = np.float32(-3.3e38)
-    elif kind == "tiny":          # whole rows below what three bf16 parts hold
+    elif kind == "large":         # finite results that overflow the scaled accumulators
+        A[1, :] *= np.float32(2.0 ** 60)
+        A[40, 9] = np.float32(2.0 ** 104)
+        B[:, 2] *= np.float32(2.0 ** 20)
+    elif kind == "tiny":          # rows and columns down to subnormals
         A[1, :] *= np.float32(2.0 ** -115)
         A[40, ::2] = np.float32(1e-40)
         B[:, 2] *= np.float32(2.0 ** -112)
@@ -111,7 +115,7 @@ def _same(got, A, B):
     np.testing.assert_array_equal(got[inputs_inf], e[inputs_inf])
 
 
-@pytest.mark.parametrize("kind", ["inf", "nan", "huge", "tiny"])
+@pytest.mark.parametrize("kind", ["inf", "nan", "huge", "large", "tiny"])
 @pytest.mark.parametrize("splits", [1, 2])
 def test_values_outside_the_split(gpu, vk, plans, kind, splits):
     rng = np.random.default_rng(11)
@@ -134,7 +138,7 @@ def test_values_outside_the_split(gpu, vk, plans, kind, splits):
     assert gpu.check_errors() == 0
 
 
-@pytest.mark.parametrize("kind", ["inf", "nan", "huge", "tiny"])
+@pytest.mark.parametrize("kind", ["inf", "nan", "huge", "large", "tiny"])
 def test_grouped_equals_single_with_unusual_values(gpu, vk, plans, kind):
     """Grouped products (swapped ones among them: m <= 64 < n) give
     vkc_gemm's bits, recomputed results included."""

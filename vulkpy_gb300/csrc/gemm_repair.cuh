@@ -20,117 +20,86 @@ struct RepairOperands {
 
 namespace {
 
-// x = h + m + l exactly (8 significant bits each), or h NaN for a value the
-// three parts cannot hold: inf, NaN, |x| >= 2^127 (h could round to inf) and
-// 0 < |x| < 2^-110 (l would fall below bf16's smallest subnormal, 2^-133).
+// Operands are scaled by 2^24 for the split, so every float32 below 2^103,
+// subnormals included, is the exact sum of three bf16 normals (or zeros) of 8
+// significant bits each, and products by 2^48, which the epilogue takes back
+// (a result of 2^79 or more overflows on the way and is recomputed).
+constexpr float kSplitScale = 0x1p24f, kSplitUnscale = 0x1p-48f;
+
+// 2^24 x = h + m + l exactly, or h NaN for a value the three parts cannot
+// hold (inf, NaN, |x| >= 2^103).
 __device__ __forceinline__ void split_bf16_3(float x, __nv_bfloat16& h, __nv_bfloat16& m, __nv_bfloat16& l) {
-  h = __float2bfloat16_rn(x);
-  const float r = x - __bfloat162float(h);
+  const float v = x * kSplitScale;
+  h = __float2bfloat16_rn(v);
+  const float r = v - __bfloat162float(h);
   m = __float2bfloat16_rn(r);
   l = __float2bfloat16_rn(r - __bfloat162float(m));
-  const float a = fabsf(x);
-  if (!(a < 0x1p127f) || (a < 0x1p-110f && a != 0.f)) h = __ushort_as_bfloat16(0x7fffu);
+  if (!(fabsf(x) < 0x1p103f)) h = __ushort_as_bfloat16(0x7fffu);
 }
 
 __device__ __forceinline__ bool all_finite(float a, float b, float c, float d) {
   return (a * 0.f + b * 0.f) + (c * 0.f + d * 0.f) == 0.f;
 }
 
-// Whether this warp's 32 x 32 block of accumulators is finite: the lane's
-// row counts if row_in, its first `cols` values.  Warp-uniform result.
-__device__ __forceinline__ bool block_finite(const uint32_t (&r)[32], bool row_in, int cols) {
+// Whether the first `cols` of a lane's N accumulators are finite.
+template <int N>
+__device__ __forceinline__ bool lane_finite(const float (&r)[N], int cols) {
   float t = 0.f;
 #pragma unroll
-  for (int j = 0; j < 32; ++j) t = fmaf(j < cols ? __uint_as_float(r[j]) : 0.f, 0.f, t);
-  return !__any_sync(0xffffffffu, row_in && !(t == 0.f));
+  for (int j = 0; j < N; ++j) t = fmaf(j < cols ? r[j] : 0.f, 0.f, t);
+  return t == 0.f;
 }
 
-// One result by itself.
-__device__ __noinline__ float repair_dot(const RepairOperands& o, int64_t m, int64_t n) {
+// W neighbouring results (m, n..n+W-1) by one thread, eight k's loads ahead of
+// their (ordered) FMAs.
+template <int W>
+__device__ __noinline__ void repair_dots(const RepairOperands& o, int64_t m, int64_t n, float (&acc)[W]) {
   const float* a = o.a + (o.ta ? m : m * o.lda);
   const float* b = o.b + (o.tb ? n * o.ldb : n);
-  const int64_t sa = o.ta ? o.lda : 1, sb = o.tb ? 1 : o.ldb;
-  float acc = 0.f;
-  for (int64_t k = 0; k < o.k; ++k) acc = fmaf(a[k * sa], b[k * sb], acc);
-  return acc;
-}
-
-// The 32 x 32 block at (m0, n0): 256 threads, four rows of one column each;
-// K in steps of 32 through shared memory.  acc[i]: row m0 + 4 (tid / 32) + i,
-// column n0 + tid % 32.  The caller synchronises before the next block.
-struct RepairSmem {
-  float a[32][33], b[32][33];  // [k][row], [k][column]
-};
-__device__ __forceinline__ void repair_block(const RepairOperands& o, int64_t M, int64_t N, int64_t m0, int64_t n0,
-                                             RepairSmem& sm, float (&acc)[4]) {
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t sa = o.ta ? o.lda : 1, sb = o.tb ? 1 : o.ldb, sw = o.tb ? o.ldb : 1;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) acc[i] = 0.f;
-  for (int64_t k0 = 0; k0 < o.k; k0 += 32) {
+  for (int w = 0; w < W; ++w) acc[w] = 0.f;
+  for (int64_t k0 = 0; k0 < o.k; k0 += 8) {
+    float av[8], bv[8][W];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int slow = ty * 4 + i;  // tx runs along the operand's contiguous index
-      const int64_t am = m0 + (o.ta ? tx : slow), ak = k0 + (o.ta ? slow : tx);
-      const float va = am < M && ak < o.k ? o.a[o.ta ? ak * o.lda + am : am * o.lda + ak] : 0.f;
-      if (o.ta) sm.a[slow][tx] = va;
-      else sm.a[tx][slow] = va;
-      const int64_t bn = n0 + (o.tb ? slow : tx), bk = k0 + (o.tb ? tx : slow);
-      const float vb = bn < N && bk < o.k ? o.b[o.tb ? bn * o.ldb + bk : bk * o.ldb + bn] : 0.f;
-      if (o.tb) sm.b[tx][slow] = vb;
-      else sm.b[slow][tx] = vb;
+    for (int t = 0; t < 8; ++t) {
+      const bool in = k0 + t < o.k;
+      av[t] = in ? a[(k0 + t) * sa] : 0.f;
+#pragma unroll
+      for (int w = 0; w < W; ++w) bv[t][w] = in ? b[(k0 + t) * sb + w * sw] : 0.f;
     }
-    __syncthreads();
-    const int kk = (int)(o.k - k0 < 32 ? o.k - k0 : 32);
-    for (int k = 0; k < kk; ++k) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[i] = fmaf(sm.a[k][ty * 4 + i], sm.b[k][tx], acc[i]);
-    }
-    __syncthreads();
+    for (int t = 0; t < 8; ++t)
+#pragma unroll
+      for (int w = 0; w < W; ++w) acc[w] = fmaf(av[t], bv[t][w], acc[w]);
   }
 }
 
-// C = act(alpha * acc + beta * C + bias) (* act'(dmask)) for repair_block's values.
-__device__ __forceinline__ void repair_store(const float (&acc)[4], int64_t M, int64_t N, int64_t m0, int64_t n0,
-                                             float alpha, float beta, float* C, int64_t ldc, const float* bias,
-                                             int act, const float* dmask, int dact) {
-  const int64_t n = n0 + (threadIdx.x & 31);
-  if (n >= N) return;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t m = m0 + (threadIdx.x >> 5) * 4 + i;
-    if (m >= M) continue;
-    float v = alpha * acc[i];
-    if (beta != 0.f) v += beta * C[m * ldc + n];
-    if (bias) v += bias[n];
-    if (act == VKC_ACT_RELU) v = fmaxf(v, 0.f);
-    else if (act == VKC_ACT_SIGMOID) v = 1.0f / (1.0f + expf(0.0f - v));
-    if (dmask) v = act_deriv(v, dmask[m * ldc + n], dact);
-    C[m * ldc + n] = v;
-  }
-}
-
-// The blocks that a GEMM launch left (list[0] of them, numbered along rows of
-// 32 x 32 blocks).  Usually none: the launch then reads one word and ends.
-__global__ void __launch_bounds__(256)
+// The 128 x 128 tiles that a GEMM launch left (list[0] of them, numbered along
+// rows of tiles), by the SIMT GEMM's tile code.  Usually none: the launch then
+// reads one word and ends.
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(kGemmThreads, 2)
 k_gemm_repair(RepairOperands o, int64_t M, int64_t N, float alpha, float beta, float* C, int64_t ldc,
-              const float* bias, int act, const float* dmask, int dact, const uint32_t* list) {
-  __shared__ RepairSmem sm;
+              GemmEpilogue epi, const uint32_t* list) {
+  __shared__ __align__(16) SimtSmem sm;
   pdl_wait();
   pdl_trigger();
-  const uint32_t count = list[0], per_row = (uint32_t)((N + 31) / 32);
+  const uint32_t count = list[0], per_row = (uint32_t)((N + kGemmBN - 1) / kGemmBN);
   for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
-    const uint32_t blk = list[1 + i];
-    const int64_t m0 = (int64_t)(blk / per_row) * 32, n0 = (int64_t)(blk % per_row) * 32;
-    float acc[4];
-    repair_block(o, M, N, m0, n0, sm, acc);
-    repair_store(acc, M, N, m0, n0, alpha, beta, C, ldc, bias, act, dmask, dact);
+    const uint32_t t = list[1 + i];
+    __syncthreads();  // the previous tile's reads of `sm` are done
+    simt_tile<TA, TB>(M, N, o.k, alpha, o.a, o.lda, o.b, o.ldb, beta, C, ldc, epi, epi.dmask,
+                      (int64_t)(t / per_row) * kGemmBM, (int64_t)(t % per_row) * kGemmBN, sm, epi.dact);
   }
 }
 
 inline int gemm_repair(vkc_device_t dev, const RepairOperands& o, int64_t M, int64_t N, float alpha, float beta,
                        float* C, int64_t ldc, const GemmEpilogue& epi, const uint32_t* list) {
-  const cudaError_t e = launch_pdl(k_gemm_repair, dim3((unsigned)dev->sm_count), dim3(256), 0, dev->stream, o, M, N,
-                                   alpha, beta, C, ldc, epi.bias, epi.act, epi.dmask, epi.dact, list);
+  auto kern = o.ta ? (o.tb ? k_gemm_repair<true, true> : k_gemm_repair<true, false>)
+                   : (o.tb ? k_gemm_repair<false, true> : k_gemm_repair<false, false>);
+  const cudaError_t e = launch_pdl(kern, dim3((unsigned)(2 * dev->sm_count)), dim3(kGemmThreads), 0, dev->stream, o, M, N,
+                                   alpha, beta, C, ldc, epi, list);
   if (e != cudaSuccess) return set_error(VKC_ERR_CUDA, "gemm repair launch: %s", cudaGetErrorString(e));
   return check_launch("gemm repair");
 }

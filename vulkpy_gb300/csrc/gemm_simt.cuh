@@ -46,13 +46,14 @@ __device__ __forceinline__ float act_deriv(float v, float y, int act) {
 }
 
 // One 128 x 128 output tile at (m0, n0).  `mask` (may be NULL, same layout
-// as C) multiplies the result by the ReLU derivative of mask[m, n].  The
-// caller synchronises the block before reusing `sm` for another tile.
+// as C) multiplies the result by the derivative of activation `mact` at
+// mask[m, n].  The caller synchronises the block before reusing `sm` for
+// another tile.
 template <bool TA, bool TB>
 __device__ __forceinline__ void simt_tile(int64_t M, int64_t N, int64_t K, float alpha, const float* __restrict__ A,
                                           int64_t lda, const float* __restrict__ B, int64_t ldb, float beta, float* C,
                                           int64_t ldc, GemmEpilogue epi, const float* __restrict__ mask, int64_t m0,
-                                          int64_t n0, SimtSmem& sm) {
+                                          int64_t n0, SimtSmem& sm, int mact = VKC_ACT_RELU) {
   auto& As = sm.As;
   auto& Bs = sm.Bs;
   const int tid = threadIdx.x;
@@ -172,7 +173,7 @@ __device__ __forceinline__ void simt_tile(int64_t M, int64_t N, int64_t K, float
       if (epi.bias) v += epi.bias[gn];
       if (epi.act == VKC_ACT_RELU) v = fmaxf(v, 0.f);
       else if (epi.act == VKC_ACT_SIGMOID) v = 1.0f / (1.0f + expf(0.0f - v));
-      if (mask) v = relu_mask(v, mask[gm * ldc + gn]);
+      if (mask) v = act_deriv(v, mask[gm * ldc + gn], mact);
       C[gm * ldc + gn] = v;
     }
   }

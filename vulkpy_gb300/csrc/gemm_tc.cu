@@ -17,10 +17,11 @@
 // the tensor pipe's truncation touches four (two) full-size additions, and
 // all accumulations are added in fp32 registers with round-to-nearest.
 // Measured against float64 (N(0,1) operands): 6.5e-8 to 1.7e-7 for K from 64
-// to 8192 where FMAs in order of k give 1.45e-7 to 1.1e-6.  Values the split cannot hold (inf, NaN, |x| >= 2^127 or
-// 0 < |x| < 2^-110) become NaN in hi, so every result they reach is not
-// finite; results that are not finite are recomputed from the fp32 operands
-// with ordered FMAs (k_gemm_repair, or inside the split-K reduction).
+// to 8192 where FMAs in order of k give 1.45e-7 to 1.1e-6.  Values the split
+// cannot hold (inf, NaN, |x| >= 2^103) become NaN in hi, so every result they
+// reach is not finite; tiles with results that are not finite are recomputed
+// from the fp32 operands with ordered FMAs (k_gemm_repair; with split K the
+// reduction recomputes single results).
 //
 // k_gemm_tcp is persistent (one CTA per SM; each CTA loads every operand tile
 // it multiplies into its own shared memory) with two TMEM accumulators, so a
@@ -84,7 +85,7 @@ struct PCfg {
   static constexpr uint32_t kBarOff = STAGES * kStageBytes;
   static constexpr int kRing = STAGES * (PARTS == 3 ? 5 : 1);  // stage barrier pairs
   // full[kRing], empty[kRing], accf[2], acce[2], drain, red[2], epi, loe[2],
-  // then tmem slot + abort flag
+  // then tmem slot, abort flag and two tile flags
   static constexpr uint32_t kSlotOff = kBarOff + 8u * (2 * kRing + 10);
   static constexpr uint32_t kEpiOff = (kSlotOff + 16 + 127) / 128 * 128;  // per-warp epilogue stages
   static constexpr uint32_t kSmem = kEpiOff + kEpiWarps * kEpiStageBytes + 1024 /*alignment slack*/;
@@ -156,8 +157,8 @@ __device__ __forceinline__ void cluster_reduce_rows(const float* partial, int sp
 // of a tile) that reduce their partial sums themselves (no separate launch).
 // map_a / map_b: the hi copies (PARTS == 3: the three copies one after the
 // other as 3 M and 3 N rows); map_alo / map_blo: the lo copies (PARTS == 2).
-// repair (PARTS == 3): count of 32 x 32 blocks of C left to k_gemm_repair,
-// then their numbers.
+// repair (PARTS == 3): count of tiles of C left to k_gemm_repair, then their
+// numbers.
 template <int PARTS, int BN, int STAGES, int DRAIN>
 __global__ void __launch_bounds__(kThreadsP, 1)
 k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -208,9 +209,9 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     if (cl_reduce) {
       mbar_init(red_bar(0), (uint32_t)splits);  // one arrival from each CTA of the cluster
       mbar_init(red_bar(1), (uint32_t)splits);
-      mbar_init(epi_bar, kEpiWarps);
     }
-    *abort_flag = 0;
+    mbar_init(epi_bar, kEpiWarps);
+    abort_flag[0] = abort_flag[1] = abort_flag[2] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -433,7 +434,7 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
               acc[c * 32 + j] += __uint_as_float(r0[j]);
-              r0[j] = __float_as_uint(acc[c * 32 + j]);
+              r0[j] = __float_as_uint(acc[c * 32 + j] * kSplitUnscale);
             }
             if (last) tmem_st32_nw(ta, r0);
           }
@@ -479,24 +480,31 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       if (!ok) break;
       if (ngroups == 0) continue;
       const bool raw_out = partial != nullptr;
+      bool skip = false;
+      if (PARTS == 3 && !raw_out) {
+        // A tile with a result that is not finite is left to k_gemm_repair
+        // whole: the eight warps agree (bounded wait) before any of them
+        // stores, since C may be read (beta != 0).  Two flags in turn, marked
+        // with the tile's number: one is written again only after every warp
+        // has read it (it has then arrived for the tile between).
+        volatile int* bad = abort_flag + 1 + (red_it & 1);
+        if (p.m0 + q * 32 + lane < M && !lane_finite(acc, N - (p.n0 + h * CW))) *bad = red_it + 1;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(epi_bar);
+        if (!mbar_wait(epi_bar, red_it & 1)) { ok = false; break; }
+        skip = *bad == red_it + 1;
+        ++red_it;
+        if (skip && warp == 2 && lane == 0)
+          repair[1 + atomicAdd(repair, 1u)] = (uint32_t)((p.m0 / kBM) * n_blocks + p.n0 / BN);
+      }
       float* cbase = raw_out ? partial + (int64_t)p.z * M * N : C;
       const int64_t ld = raw_out ? (int64_t)N : ldc;
       float* stage = reinterpret_cast<float*>(gbase + Cfg::kEpiOff) + (warp - 2) * (kEpiStageBytes / 4);
 #pragma unroll 1
-      for (int c = 0; c < CW / 32; ++c) {  // one copy of the epilogue code
+      for (int c = 0; c < CW / 32 && !skip; ++c) {  // one copy of the epilogue code
         uint32_t r0[32];
         tmem_ld32(tmem + lane_addr + (uint32_t)(b * BN + h * CW + c * 32), r0);
         const int col0 = p.n0 + h * CW + c * 32;
-        if (PARTS == 3 && !raw_out && p.m0 + q * 32 < M && col0 < N) {
-          // a block with a result that is not finite is left to k_gemm_repair,
-          // whole (C may be read with beta != 0, so it is not touched here)
-          if (!block_finite(r0, p.m0 + q * 32 + lane < M, N - col0)) {
-            if (lane == 0)
-              repair[1 + atomicAdd(repair, 1u)] =
-                  (uint32_t)((p.m0 / 32 + q) * ((N + 31) / 32) + col0 / 32);
-            continue;
-          }
-        }
         if (p.m0 + q * 32 < M && col0 < N)
           // (the split kernel with 256-column tiles holds 128 running sums per
           // thread and has no registers to spare for the fixed forms)
@@ -676,7 +684,7 @@ struct SplitJob {
 };
 
 // PARTS == 3: hi, mid and lo one after the other at `hi`; `repair` (may be
-// NULL) is the count of blocks k_gemm_repair will have to do, zeroed here.
+// NULL) is the count of tiles k_gemm_repair will have to do, zeroed here.
 template <int PARTS>
 __global__ void __launch_bounds__(256) k_split_pair(const __grid_constant__ SplitJob a,
                                                     const __grid_constant__ SplitJob b, uint32_t* repair) {
@@ -838,7 +846,8 @@ __device__ __forceinline__ void split_out1(const SplitOut& so, int64_t r, int64_
 
 // Four columns per thread (N % 4 == 0, ldc % 4 == 0, 16-byte aligned C);
 // the split loads are issued four at a time ahead of their (ordered) adds.
-// REPAIR: sums that are not finite are recomputed from the operands `ro`.
+// REPAIR: a quad with a sum that is not finite is recomputed from the
+// operands `ro`.
 template <bool REPAIR>
 __global__ void __launch_bounds__(256)
 k_splitk_reduce4(const float* __restrict__ partial, int splits, int64_t M, int64_t N, float alpha, float beta,
@@ -864,10 +873,9 @@ k_splitk_reduce4(const float* __restrict__ partial, int splits, int64_t M, int64
     for (; z < splits; ++z) add4(s, __ldcs(p + (int64_t)z * quads));
     const int64_t r = i / N, col = i - r * N;
     if (REPAIR && !all_finite(s.x, s.y, s.z, s.w)) {
-      if (!isfinite(s.x)) s.x = repair_dot(ro, r, col);
-      if (!isfinite(s.y)) s.y = repair_dot(ro, r, col + 1);
-      if (!isfinite(s.z)) s.z = repair_dot(ro, r, col + 2);
-      if (!isfinite(s.w)) s.w = repair_dot(ro, r, col + 3);
+      float v[4];
+      repair_dots<4>(ro, r, col, v);
+      s = make_float4(v[0], v[1], v[2], v[3]);
     }
     float4* cp = reinterpret_cast<float4*>(C + r * ldc + col);
     const float4 c0 = beta != 0.f ? *cp : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -904,7 +912,11 @@ k_splitk_reduce(const float* __restrict__ partial, int splits, int64_t M, int64_
     float s = partial[i];
     for (int z = 1; z < splits; ++z) s += partial[(int64_t)z * total + i];
     const int64_t r = i / N, col = i - r * N;
-    if (REPAIR && !isfinite(s)) s = repair_dot(ro, r, col);
+    if (REPAIR && !isfinite(s)) {
+      float v[1];
+      repair_dots<1>(ro, r, col, v);
+      s = v[0];
+    }
     float* c = C + r * ldc + col;
     float v = splitk_epilogue(s, alpha, beta, beta != 0.f ? *c : 0.f, bias != nullptr, bias ? bias[col] : 0.f, act);
     if (dmask) v = act_deriv(v, dmask[r * ldc + col], dact);
@@ -1194,11 +1206,11 @@ int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t 
   const int ranges = simt_splits(dev, M, N, K);
   if (!fp32_on_tensor_cores(M, N, K, ranges)) return simt();
   const int64_t Kp = (K + kBK - 1) / kBK * kBK;
-  const int64_t blocks = ((M + 31) / 32) * ((N + 31) / 32);
+  const int64_t tiles = cta_tiles(M, N, 128);
   const size_t elems = 3 * (size_t)(M + N) * Kp;
   const size_t list = (elems * sizeof(__nv_bfloat16) + 15) / 16 * 16;
   void* scratch = nullptr;
-  if (scratch_alloc(dev, list + (size_t)(1 + blocks) * 4, &scratch) != VKC_OK) {
+  if (scratch_alloc(dev, list + (size_t)(1 + tiles) * 4, &scratch) != VKC_OK) {
     // no room for the operands' copies: the SIMT GEMM reads them in place
     clear_error();
     return simt();

@@ -69,35 +69,52 @@ __device__ __forceinline__ int find_problem(const T* p, int count, int t) {
   return lo;
 }
 
+__device__ __forceinline__ void simt_grouped_tile(const SimtProb& P, int64_t m0, int64_t n0, SimtSmem& sm) {
+  GemmEpilogue epi;
+  epi.bias = P.bias;
+  epi.act = P.act;
+  __syncthreads();  // the previous tile's reads of `sm` are done
+  switch (P.trans & 3) {
+    case 0:
+      simt_tile<false, false>(P.m, P.n, P.k, P.alpha, P.a, P.lda, P.b, P.ldb, P.beta, P.c, P.ldc, epi, P.mask, m0, n0,
+                              sm);
+      break;
+    case 1:
+      simt_tile<true, false>(P.m, P.n, P.k, P.alpha, P.a, P.lda, P.b, P.ldb, P.beta, P.c, P.ldc, epi, P.mask, m0, n0,
+                             sm);
+      break;
+    case 2:
+      simt_tile<false, true>(P.m, P.n, P.k, P.alpha, P.a, P.lda, P.b, P.ldb, P.beta, P.c, P.ldc, epi, P.mask, m0, n0,
+                             sm);
+      break;
+    default:
+      simt_tile<true, true>(P.m, P.n, P.k, P.alpha, P.a, P.lda, P.b, P.ldb, P.beta, P.c, P.ldc, epi, P.mask, m0, n0,
+                            sm);
+      break;
+  }
+}
+
 __global__ void __launch_bounds__(kGemmThreads, 2) k_gemm_simt_grouped(const __grid_constant__ SimtTable tab) {
   __shared__ __align__(16) SimtSmem sm;
   for (int t = blockIdx.x; t < tab.total; t += gridDim.x) {
     const SimtProb& P = tab.p[find_problem(tab.p, tab.count, t)];
     const int local = t - P.tile0;
-    const int64_t m0 = (int64_t)(local / P.tiles_n) * kGemmBM;
-    const int64_t n0 = (int64_t)(local % P.tiles_n) * kGemmBN;
-    GemmEpilogue epi;
-    epi.bias = P.bias;
-    epi.act = P.act;
-    __syncthreads();  // the previous tile's reads of `sm` are done
-    switch (P.trans) {
-      case 0:
-        simt_tile<false, false>(P.m, P.n, P.k, P.alpha, P.a, P.lda, P.b, P.ldb, P.beta, P.c, P.ldc, epi, P.mask, m0,
-                                n0, sm);
-        break;
-      case 1:
-        simt_tile<true, false>(P.m, P.n, P.k, P.alpha, P.a, P.lda, P.b, P.ldb, P.beta, P.c, P.ldc, epi, P.mask, m0,
-                               n0, sm);
-        break;
-      case 2:
-        simt_tile<false, true>(P.m, P.n, P.k, P.alpha, P.a, P.lda, P.b, P.ldb, P.beta, P.c, P.ldc, epi, P.mask, m0,
-                               n0, sm);
-        break;
-      default:
-        simt_tile<true, true>(P.m, P.n, P.k, P.alpha, P.a, P.lda, P.b, P.ldb, P.beta, P.c, P.ldc, epi, P.mask, m0,
-                              n0, sm);
-        break;
-    }
+    simt_grouped_tile(P, (int64_t)(local / P.tiles_n) * kGemmBM, (int64_t)(local % P.tiles_n) * kGemmBN, sm);
+  }
+}
+
+// The tiles that k_gemm_tc_grouped<3> left (list[0] of them), from the fp32
+// operands; a swapped problem's tiles are those of C^T.
+__global__ void __launch_bounds__(kGemmThreads, 2)
+k_gemm_repair_grouped(const __grid_constant__ SimtTable tab, const uint32_t* list) {
+  __shared__ __align__(16) SimtSmem sm;
+  const uint32_t count = list[0];
+  for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+    const int t = (int)list[1 + i];
+    const SimtProb& P = tab.p[find_problem(tab.p, tab.count, t)];
+    const int local = t - P.tile0;
+    const int64_t r0 = (int64_t)(local / P.tiles_n) * 128, c0 = (int64_t)(local % P.tiles_n) * 128;
+    simt_grouped_tile(P, P.trans & 4 ? c0 : r0, P.trans & 4 ? r0 : c0, sm);
   }
 }
 
@@ -126,7 +143,7 @@ struct TileTable {
 // index is contiguous) into shared memory, then write 16-byte chunks of hi
 // (and lo = bf16(x - hi), or mid and lo) at their swizzled positions.  Rows
 // >= rows and k >= K are written as zeros.  THREE: three parts; `repair` is
-// then the count of blocks left to k_gemm_repair_grouped, zeroed here.
+// then the count of tiles left to k_gemm_repair_grouped, zeroed here.
 template <bool THREE>
 __global__ void __launch_bounds__(256, 3) k_tile_operands(const __grid_constant__ TileTable tab, uint32_t* repair) {
   __shared__ float s[kTileRows][kTileK + 1];
@@ -272,7 +289,7 @@ template <int PARTS>
 struct GroupedCfg {
   static constexpr int kStages = grouped_stages(PARTS);
   static constexpr uint32_t kStageBytes = 2u * PARTS * kTileBytes;
-  static constexpr uint32_t kBarBytes = 8u * (2 * kStages + 2 * kAccBufs + 1) + 16;
+  static constexpr uint32_t kBarBytes = 8u * (2 * kStages + 2 * kAccBufs + 2) + 16;
   static constexpr uint32_t kEpiOff = kStages * kStageBytes + (kBarBytes + 127) / 128 * 128;
   static constexpr uint32_t kSmem = kEpiOff + kGroupedEpiWarps * kEpiStageBytes + 1024;
 };
@@ -283,8 +300,7 @@ struct GroupedCfg {
 // PARTS == 3 (fp32): hi*hi products use TMEM buffers 0 and 1, one
 // accumulation per K block; the five small ones buffers 2 and 3, one per
 // kLoSpan blocks (their "full" barriers are not needed: a block's hi*hi commit
-// covers them).  repair: as k_gemm_tcp, entries are 16 * tile + 4 * lane
-// quarter + 32-column chunk.
+// covers them).  repair: as k_gemm_tcp, entries are numbers of the tile list.
 template <int PARTS>
 __global__ void __launch_bounds__(kThreadsGrouped, 1)
 k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err, uint32_t* __restrict__ repair) {
@@ -303,7 +319,8 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err, uint32_t* 
   auto accf_bar = [&](int b) { return bars + 8u * (2 * S + b); };
   auto acce_bar = [&](int b) { return bars + 8u * (2 * S + kAccBufs + b); };
   const uint32_t drain_bar = bars + 8u * (2 * S + 2 * kAccBufs);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + S * Cfg::kStageBytes + 8 * (2 * S + 2 * kAccBufs + 1));
+  const uint32_t epi_bar = drain_bar + 8u;  // PARTS == 3: the epilogue warps agree on a tile
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + S * Cfg::kStageBytes + 8 * (2 * S + 2 * kAccBufs + 2));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -318,7 +335,8 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err, uint32_t* 
       mbar_init(acce_bar(b), kGroupedEpiWarps);
     }
     mbar_init(drain_bar, 1);
-    *abort_flag = 0;
+    mbar_init(epi_bar, kGroupedEpiWarps);
+    abort_flag[0] = abort_flag[1] = abort_flag[2] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -468,6 +486,7 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err, uint32_t* 
     const int hc = (warp - 2) >> 2;   // column half
     const uint32_t lane_addr = ((uint32_t)(q * 32) << 16) + (uint32_t)(hc * CW);
     uint32_t g = 0, lo_it = 0;
+    int tiles_done = 0;  // PARTS == 3
     bool ok = true;
     for (int t = blockIdx.x; t < tab.total && ok; t += gridDim.x) {
       const TcProb& P = tab.p[find_problem(tab.p, tab.count, t)];
@@ -515,7 +534,7 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err, uint32_t* 
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
               sum[c * 32 + j] += __uint_as_float(r0[j]);
-              r0[j] = __float_as_uint(sum[c * 32 + j]);
+              r0[j] = __float_as_uint(sum[c * 32 + j] * kSplitUnscale);
             }
             if (last) tmem_st32_nw(ta, r0);
           }
@@ -556,20 +575,24 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err, uint32_t* 
         }
       }
       if (!ok) break;
+      bool skip = false;
+      if (PARTS == 3) {  // as k_gemm_tcp: tiles with results that are not finite are left whole
+        volatile int* bad = abort_flag + 1 + (tiles_done & 1);
+        if (m0 + q * 32 + lane < (P.swap ? P.n : P.m) && !lane_finite(sum, P.nk - n0)) *bad = tiles_done + 1;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(epi_bar);
+        if (!mbar_wait(epi_bar, tiles_done & 1)) { ok = false; break; }
+        skip = *bad == tiles_done + 1;
+        ++tiles_done;
+        if (skip && warp == 2 && lane == 0) repair[1 + atomicAdd(repair, 1u)] = (uint32_t)t;
+      }
       float* stage = reinterpret_cast<float*>(gbase + Cfg::kEpiOff) + (warp - 2) * (kEpiStageBytes / 4);
 #pragma unroll 1
-      for (int c = 0; c < CW / 32; ++c) {  // one copy of the epilogue code
+      for (int c = 0; c < CW / 32 && !skip; ++c) {  // one copy of the epilogue code
         const int col0 = n0 + c * 32;
         if (col0 >= P.nk) break;
         uint32_t r[32];
         tmem_ld32(tmem + lane_addr + (uint32_t)(b * BN + c * 32), r);
-        if (PARTS == 3 && m0 + q * 32 < (P.swap ? P.n : P.m)) {
-          // results that are not finite are left to k_gemm_repair_grouped
-          if (!block_finite(r, m0 + q * 32 + lane < (P.swap ? P.n : P.m), P.nk - col0)) {
-            if (lane == 0) repair[1 + atomicAdd(repair, 1u)] = (uint32_t)t * 16u + (uint32_t)(q * 4 + hc * 2 + c);
-            continue;
-          }
-        }
         if (P.swap) {
           // lanes are columns of C (kernel rows), TMEM columns rows of C
           if (m0 + q * 32 < P.n)
@@ -602,26 +625,6 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err, uint32_t* 
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
-  }
-}
-
-// The blocks that k_gemm_tc_grouped<3> left, from the fp32 operands.
-__global__ void __launch_bounds__(256)
-k_gemm_repair_grouped(const __grid_constant__ SimtTable tab, const uint32_t* list) {
-  __shared__ RepairSmem sm;
-  const uint32_t count = list[0];
-  for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
-    const int t = (int)(list[1 + i] >> 4), q = (int)(list[1 + i] >> 2) & 3, c = (int)list[1 + i] & 3;
-    const SimtProb& P = tab.p[find_problem(tab.p, tab.count, t)];
-    const int local = t - P.tile0;
-    // kernel coordinates; a swapped problem's are those of C^T
-    const int64_t r0 = (int64_t)(local / P.tiles_n) * kTileRows + q * 32;
-    const int64_t c0 = (int64_t)(local % P.tiles_n) * 128 + c * 32;
-    const int64_t m0 = P.trans & 4 ? c0 : r0, n0 = P.trans & 4 ? r0 : c0;
-    const RepairOperands o{P.a, P.b, P.lda, P.ldb, P.k, P.trans & 1, (P.trans >> 1) & 1};
-    float acc[4];
-    repair_block(o, P.m, P.n, m0, n0, sm, acc);
-    repair_store(acc, P.m, P.n, m0, n0, P.alpha, P.beta, P.c, P.ldc, P.bias, P.act, P.mask, VKC_ACT_RELU);
   }
 }
 
@@ -1000,7 +1003,7 @@ int grouped_tc(vkc_device_t dev, const vkc_gemm_problem* probs, const vkc_gemm_u
       ctiles += (size_t)((q.m + kTileRows - 1) / kTileRows) * (size_t)((q.n + 127) / 128);
     }
     const size_t list = bytes;  // bytes is a multiple of 16 KB
-    if (PARTS == 3) bytes += 4 * (1 + 16 * ctiles);
+    if (PARTS == 3) bytes += 4 * (1 + ctiles);
     void* scratch = nullptr;
     int r = scratch_alloc(dev, bytes, &scratch);
     if (r != VKC_OK && PARTS == 3) {
@@ -1119,7 +1122,7 @@ int grouped_tc(vkc_device_t dev, const vkc_gemm_problem* probs, const vkc_gemm_u
       r = check_launch("gemm_grouped (tensor cores)");
       if (r == VKC_OK && PARTS == 3) {
         rt.total = total;
-        k_gemm_repair_grouped<<<(unsigned)dev->sm_count, 256, 0, dev->stream>>>(rt, repair);
+        k_gemm_repair_grouped<<<(unsigned)(2 * dev->sm_count), kGemmThreads, 0, dev->stream>>>(rt, repair);
         r = check_launch("gemm_grouped repair");
       }
     }
