@@ -7,6 +7,12 @@
 // the high word and the complement of the index in the low word, so the
 // maximum key is the extreme value at the smallest index and every combine is
 // a plain integer max -- associative, so any tree order gives the same answer.
+//
+// A thread does not build a key per element (about ten instructions: with one
+// load each that bound rows of 32768 to 2.3 TB/s): it takes the NaN-passing
+// maximum of 16 elements (one instruction each), keeps the best group so far
+// and looks up the element in that group once at the end.  8192 x 32768: rows
+// 469 -> 151 us, whole 276 -> 152 us (7.0 TB/s).
 #include <algorithm>
 
 #include "common.cuh"
@@ -49,36 +55,110 @@ __device__ __forceinline__ uint64_t block_max(uint64_t k, uint64_t* sh) {
 
 constexpr int kThreads = 256;
 
-// Pass 1: each block reduces a grid-stride share of a[0..n) to one key.
+// max / min that returns NaN when an operand is NaN.
+template <bool MIN>
+__device__ __forceinline__ float extreme(float a, float b) {
+  float r;
+  if (MIN) asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  else asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+// Whether a later group's extreme m replaces the best so far: strictly
+// better, or the first NaN.
+template <bool MIN>
+__device__ __forceinline__ bool replaces(float m, float best) {
+  return (MIN ? m < best : m > best) || (m != m && best == best);
+}
+
+__device__ __forceinline__ bool is_best(float v, float best) { return v == best || (v != v && best != best); }
+
+template <bool MIN>
+constexpr float kWorst = MIN ? INFINITY : -INFINITY;
+
+constexpr int kGroup = 4;  // vectors per group
+
+// A thread's best group: element (at + u nt) W + w for u < U, w < W, or with
+// W == 0 the element `at` itself.
+struct Scan {
+  float best;
+  size_t at;
+  int w;
+  bool any;
+};
+
+// Elements t, t + nt, ... of a[0..n) (nt threads) for T = float4 (16-byte
+// aligned a; n counts whole float4) or float.
+template <bool MIN, class T>
+__device__ __forceinline__ Scan scan_groups(const float* __restrict__ a, size_t n, size_t t, size_t nt) {
+  constexpr int W = sizeof(T) / 4, U = W == 4 ? kGroup : 4 * kGroup;
+  const T* av = reinterpret_cast<const T*>(a);
+  Scan s{kWorst<MIN>, t, W, t < n};  // a group of nothing but kWorst is the first one's
+  const size_t last = (U - 1) * nt;
+  for (size_t i = t; i < n; i += U * nt) {
+    T v[U];
+    if (i + last < n) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = __ldcs(av + i + u * nt);
+    } else {
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = i + u * nt < n ? __ldcs(av + i + u * nt) : v[0];
+    }
+    float m = kWorst<MIN>;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int w = 0; w < W; ++w) m = extreme<MIN>(m, reinterpret_cast<const float*>(&v[u])[w]);
+    if (replaces<MIN>(m, s.best)) {
+      s.best = m;
+      s.at = i;
+    }
+  }
+  return s;
+}
+
+// Thread t of nt over a[0..n): whole float4 when a is aligned, the (at most
+// 3) elements after them one by one (nt >= 32).
+template <bool MIN>
+__device__ __forceinline__ Scan scan(const float* __restrict__ a, size_t n, size_t t, size_t nt) {
+  if ((((uintptr_t)a) & 15u) != 0) return scan_groups<MIN, float>(a, n, t, nt);
+  const size_t n4 = n / 4;
+  Scan s = scan_groups<MIN, float4>(a, n4, t, nt);
+  const size_t k = 4 * n4 + t;
+  if (k < n && (!s.any || replaces<MIN>(a[k], s.best))) s = Scan{a[k], k, 0, true};
+  return s;
+}
+
+// The key of the first element of the scan's group with its best value.
+template <bool MIN>
+__device__ __forceinline__ uint64_t scan_key(const Scan& s, const float* __restrict__ a, size_t n, size_t nt) {
+  if (s.w == 0) return make_key<MIN>(s.best, (uint32_t)s.at);
+  const size_t end = s.w == 4 ? n / 4 * 4 : n;
+  for (int e = 0; e < 4 * kGroup; ++e) {
+    const size_t k = s.w * (s.at + (size_t)(e / s.w) * nt) + e % s.w;
+    if (k < end && is_best(a[k], s.best)) return make_key<MIN>(s.best, (uint32_t)k);
+  }
+  return 0;  // not reached: the group holds its extreme
+}
+
+// The best key of a[0..n) over the block: the threads agree on the value
+// first, and only those that hold it look for their element.
+template <bool MIN>
+__device__ __forceinline__ uint64_t block_best(const float* __restrict__ a, size_t n, size_t t, size_t nt,
+                                               uint64_t* sh) {
+  const Scan s = scan<MIN>(a, n, t, nt);
+  const uint32_t word = s.any ? order_word<MIN>(s.best) : 0u;
+  const uint32_t top = (uint32_t)(block_max((uint64_t)word << 32, sh) >> 32);
+  return block_max(s.any && word == top ? scan_key<MIN>(s, a, n, nt) : 0, sh);
+}
+
+// Pass 1: each block reduces its share of a[0..n) to one key.
 template <bool MIN>
 __global__ void __launch_bounds__(kThreads) k_arg_partials(const float* __restrict__ a, size_t n,
                                                            uint64_t* __restrict__ part) {
   __shared__ uint64_t sh[32];
-  uint64_t best = 0;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if ((((uintptr_t)a) & 15u) == 0) {
-    const size_t n4 = n / 4;
-    const float4* a4 = reinterpret_cast<const float4*>(a);
-    for (size_t i = t; i < n4; i += 2 * stride) {
-      const float4 x = __ldg(a4 + i);
-      float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
-      const bool two = i + stride < n4;
-      if (two) y = __ldg(a4 + i + stride);
-      const uint32_t b0 = (uint32_t)(4 * i);
-      best = kmax(best, kmax(kmax(make_key<MIN>(x.x, b0), make_key<MIN>(x.y, b0 + 1)),
-                             kmax(make_key<MIN>(x.z, b0 + 2), make_key<MIN>(x.w, b0 + 3))));
-      if (two) {
-        const uint32_t b1 = (uint32_t)(4 * (i + stride));
-        best = kmax(best, kmax(kmax(make_key<MIN>(y.x, b1), make_key<MIN>(y.y, b1 + 1)),
-                               kmax(make_key<MIN>(y.z, b1 + 2), make_key<MIN>(y.w, b1 + 3))));
-      }
-    }
-    for (size_t i = 4 * n4 + t; i < n; i += stride) best = kmax(best, make_key<MIN>(a[i], (uint32_t)i));
-  } else {
-    for (size_t i = t; i < n; i += stride) best = kmax(best, make_key<MIN>(__ldg(a + i), (uint32_t)i));
-  }
-  best = block_max(best, sh);
+  const uint64_t best = block_best<MIN>(a, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x,
+                                        (size_t)gridDim.x * blockDim.x, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = best;
 }
 
@@ -87,12 +167,15 @@ __global__ void __launch_bounds__(1024) k_arg_final(const uint64_t* __restrict__
                                                    uint32_t* __restrict__ out) {
   __shared__ uint64_t sh[32];
   uint64_t best = 0;
+  pdl_wait();
   for (int i = threadIdx.x; i < m; i += blockDim.x) best = kmax(best, part[i]);
   best = block_max(best, sh);
   if (threadIdx.x == 0) out[0] = ~(uint32_t)best;
 }
 
-// Along a contiguous axis (post == 1): one warp per row.
+// Along a contiguous axis (post == 1) shorter than 2048: one warp per row,
+// the index kept beside the best value (a lane has too few elements for
+// groups to pay).
 template <bool MIN>
 __global__ void __launch_bounds__(kThreads) k_arg_rows_warp(const float* __restrict__ a, size_t rows,
                                                             size_t len, uint32_t* __restrict__ out) {
@@ -100,10 +183,21 @@ __global__ void __launch_bounds__(kThreads) k_arg_rows_warp(const float* __restr
   const int lane = threadIdx.x & 31;
   for (size_t r = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += warps) {
     const float* row = a + r * len;
-    uint64_t best = 0;
-    for (size_t k = lane; k < len; k += 32) best = kmax(best, make_key<MIN>(__ldg(row + k), (uint32_t)k));
-    best = warp_max(best);
-    if (lane == 0) out[r] = ~(uint32_t)best;
+    float best = kWorst<MIN>;
+    uint32_t at = lane;
+#pragma unroll 4
+    for (uint32_t k = lane; k < (uint32_t)len; k += 32) {
+      const float v = __ldg(row + k);
+      if (replaces<MIN>(v, best)) {
+        best = v;
+        at = k;
+      }
+    }
+    const bool any = lane < len;
+    const uint32_t word = any ? order_word<MIN>(best) : 0u;
+    const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, word);
+    at = __reduce_min_sync(0xFFFFFFFFu, any && word == top ? at : 0xFFFFFFFFu);
+    if (lane == 0) out[r] = at;
   }
 }
 
@@ -113,11 +207,7 @@ __global__ void __launch_bounds__(kThreads) k_arg_rows_block(const float* __rest
                                                              size_t len, uint32_t* __restrict__ out) {
   __shared__ uint64_t sh[32];
   for (size_t r = blockIdx.x; r < rows; r += gridDim.x) {
-    const float* row = a + r * len;
-    uint64_t best = 0;
-    for (size_t k = threadIdx.x; k < len; k += blockDim.x)
-      best = kmax(best, make_key<MIN>(__ldg(row + k), (uint32_t)k));
-    best = block_max(best, sh);
+    const uint64_t best = block_best<MIN>(a + r * len, len, threadIdx.x, kThreads, sh);
     if (threadIdx.x == 0) out[r] = ~(uint32_t)best;
   }
 }
@@ -155,15 +245,17 @@ __global__ void __launch_bounds__(kColsX* kColsY) k_arg_cols(const float* __rest
 
 template <bool MIN>
 int arg_all(vkc_device_t dev, const float* a, size_t n, uint32_t* out) {
-  const unsigned g = stream_grid(dev, (n + 7) / 8, kThreads, 4);
+  const unsigned g = stream_grid(dev, (n + 15) / 16, kThreads, 8);
   void* part = nullptr;
   int r = scratch_alloc(dev, (size_t)g * sizeof(uint64_t), &part);
   if (r != VKC_OK) return r;
   k_arg_partials<MIN><<<g, kThreads, 0, dev->stream>>>(a, n, static_cast<uint64_t*>(part));
   r = check_launch("argreduce partials");
   if (r == VKC_OK) {
-    k_arg_final<<<1, 1024, 0, dev->stream>>>(static_cast<const uint64_t*>(part), (int)g, out);
-    r = check_launch("argreduce final");
+    const cudaError_t e = launch_second(k_arg_final, dim3(1), dim3(1024), dev->stream, n,
+                                        static_cast<const uint64_t*>(part), (int)g, out);
+    r = e == cudaSuccess ? check_launch("argreduce final")
+                         : set_error(VKC_ERR_CUDA, "argreduce final launch: %s", cudaGetErrorString(e));
   }
   scratch_free(dev, part);
   return r;

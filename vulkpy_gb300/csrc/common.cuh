@@ -138,6 +138,19 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
+// The second kernel of a two-kernel op over n elements: with PDL from 2^21 on,
+// where the GPU is the bound and its launch then overlaps the first kernel's
+// tail (7 reductions over 60 x 8192 x 9: 272 -> 253 us); below, the calls are
+// bound by the host, and the plain launch costs it less (133 -> 130 us for 13
+// calls on 100 x 100).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_second(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t stream, size_t n,
+                                 Args&&... args) {
+  if (n >= (size_t(1) << 21)) return launch_pdl(kern, grid, block, 0, stream, std::forward<Args>(args)...);
+  kern<<<grid, block, 0, stream>>>(std::forward<Args>(args)...);
+  return cudaSuccess;  // check_launch reads the launch's error
+}
+
 // launch_pdl with the blocks grouped into 1-D thread-block clusters of
 // `cluster` CTAs (grid.x a multiple of it).
 template <typename... KArgs, typename... Args>

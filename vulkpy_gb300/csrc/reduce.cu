@@ -112,6 +112,7 @@ k_reduce_all(const float* a, size_t n, double* partials, float* out, float scale
 template <int OP, bool COMP, bool FP64>
 __global__ void __launch_bounds__(1024)
 k_reduce_partials(const double* partials, int np, float* out, float scale) {
+  vkc::pdl_wait();
   if constexpr (FP64) {
     __shared__ double sh[32];
     double v = (OP == VKC_SUM) ? 0.0 : (OP == VKC_PROD ? 1.0 : (double)identity<OP>());
@@ -146,6 +147,16 @@ k_reduce_partials(const double* partials, int np, float* out, float scale) {
   }
 }
 
+template <int OP, bool COMP>
+int reduce_partials(vkc_device_t dev, const double* partials, size_t np, size_t n, float* out, float scale) {
+  const bool fp64 = (OP == VKC_SUM || OP == VKC_PROD) && n >= (size_t(1) << 24);
+  const cudaError_t e =
+      vkc::launch_second(fp64 ? k_reduce_partials<OP, COMP, true> : k_reduce_partials<OP, COMP, false>, dim3(1),
+                         dim3(1024), dev->stream, n, partials, (int)np, out, scale);
+  if (e != cudaSuccess) return vkc::set_error(VKC_ERR_CUDA, "reduce_partials launch: %s", cudaGetErrorString(e));
+  return vkc::check_launch("reduce_partials");
+}
+
 template <int OP, bool COMP, int NACC>
 int reduce_all_impl(vkc_device_t dev, const float* a, size_t n, float* out, float scale) {
   const bool aligned = ((uintptr_t)a & 15u) == 0;
@@ -163,10 +174,7 @@ int reduce_all_impl(vkc_device_t dev, const float* a, size_t n, float* out, floa
   k_reduce_all<OP, COMP, NACC><<<grid, kThreads, 0, dev->stream>>>(a, n, partials, out, scale);
   r = vkc::check_launch("reduce_all");
   if (r == VKC_OK) {
-    const bool fp64 = (OP == VKC_SUM || OP == VKC_PROD) && n >= (size_t(1) << 24);
-    if (fp64) k_reduce_partials<OP, COMP, true><<<1, 1024, 0, dev->stream>>>(partials, (int)grid, out, scale);
-    else k_reduce_partials<OP, COMP, false><<<1, 1024, 0, dev->stream>>>(partials, (int)grid, out, scale);
-    r = vkc::check_launch("reduce_partials");
+    r = reduce_partials<OP, COMP>(dev, partials, grid, n, out, scale);
   }
   vkc::scratch_free(dev, partials);
   return r;
@@ -216,7 +224,7 @@ k_rows_warp(const float* a, size_t prev, size_t axis, float* out, int rebroadcas
 // post == 1: `splits` blocks per row (splits == 1 -> writes the result).
 template <int OP, bool COMP>
 __global__ void __launch_bounds__(kThreads)
-k_rows_block(const float* a, size_t prev, size_t axis, int splits, float* out, double* partials,
+k_rows_block(const float* a, size_t prev, size_t axis, int splits, float* out, float2* partials,
              int rebroadcast, float scale) {
   const size_t r = blockIdx.x / splits;
   const int sp = blockIdx.x % splits;
@@ -247,8 +255,7 @@ k_rows_block(const float* a, size_t prev, size_t axis, int splits, float* out, d
       result = v;
       if (!rebroadcast) out[r] = v;
     } else {
-      partials[2 * blockIdx.x] = acc.s;
-      partials[2 * blockIdx.x + 1] = acc.c;
+      partials[blockIdx.x] = make_float2(acc.s, acc.c);
     }
   }
   if (splits == 1 && rebroadcast) {
@@ -259,11 +266,14 @@ k_rows_block(const float* a, size_t prev, size_t axis, int splits, float* out, d
 }
 
 // Combine `splits` partials per output; writes out[i*post + j] (or the
-// rebroadcast row/column).  Layout of partials: [prev][splits][post] pairs.
+// rebroadcast row/column).  Layout of partials: [prev][splits][post] pairs
+// (value, error term) as the threads hold them, float32: the pass moves half
+// of what pairs of doubles did (38 slices of 32768 columns: 17 -> 8 us).
 template <int OP, bool COMP>
-__global__ void k_combine_splits(const double* partials, size_t prev, size_t axis, size_t post, int splits,
+__global__ void k_combine_splits(const float2* partials, size_t prev, size_t axis, size_t post, int splits,
                                  float* out, int rebroadcast, float scale) {
   size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  vkc::pdl_wait();
   if (idx >= prev * post) return;
   size_t i = idx / post, j = idx % post;
   Acc<OP, COMP> acc;
@@ -271,16 +281,13 @@ __global__ void k_combine_splits(const double* partials, size_t prev, size_t axi
   // eight splits' partials loaded ahead of their (ordered) merges: one
   // memory wait per eight instead of one per split
   for (int s0 = 0; s0 < splits; s0 += 8) {
-    double pv[8], pc[8];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      const size_t p = (i * splits + s0 + t) * post + j;
-      pv[t] = s0 + t < splits ? partials[2 * p] : 0.0;
-      pc[t] = s0 + t < splits ? partials[2 * p + 1] : 0.0;
-    }
+    float2 p[8];
 #pragma unroll
     for (int t = 0; t < 8; ++t)
-      if (s0 + t < splits) acc.merge((float)pv[t], (float)pc[t]);
+      p[t] = s0 + t < splits ? partials[(i * splits + s0 + t) * post + j] : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+      if (s0 + t < splits) acc.merge(p[t].x, p[t].y);
   }
   float v = acc.value();
   if (OP == VKC_SUM || OP == VKC_PROD) v *= scale;
@@ -295,7 +302,7 @@ __global__ void k_combine_splits(const double* partials, size_t prev, size_t axi
 // one (prev, slice) and walks its slice of the axis.
 template <int OP, bool COMP, int VW>
 __global__ void __launch_bounds__(kThreads)
-k_cols(const float* a, size_t prev, size_t axis, size_t post, int splits, float* out, double* partials,
+k_cols(const float* a, size_t prev, size_t axis, size_t post, int splits, float* out, float2* partials,
        int rebroadcast, float scale) {
   const size_t ncolv = post / VW;
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -323,21 +330,26 @@ k_cols(const float* a, size_t prev, size_t axis, size_t post, int splits, float*
       }
     }
   }
-  for (; k < k1; ++k) {
-    if constexpr (VW == 4) {
+  if constexpr (VW == 4) {
+    for (; k < k1; ++k) {
       float4 v = *reinterpret_cast<const float4*>(base + k * post);
       acc[0].push(v.x); acc[1].push(v.y); acc[2].push(v.z); acc[3].push(v.w);
-    } else {
-      acc[0].push(base[k * post]);
     }
+  } else {
+    // one column (post not a multiple of 4): 16 rows' loads ahead of their adds
+    for (; k + 15 < k1; k += 16) {
+      float v[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) v[u] = __ldcs(base + (k + u) * post);
+#pragma unroll
+      for (int u = 0; u < 16; ++u) acc[0].push(v[u]);
+    }
+#pragma unroll 4
+    for (; k < k1; ++k) acc[0].push(base[k * post]);
   }
   if (splits > 1) {
 #pragma unroll
-    for (int w = 0; w < VW; ++w) {
-      size_t p = (i * splits + sp) * post + j + w;
-      partials[2 * p] = acc[w].s;
-      partials[2 * p + 1] = acc[w].c;
-    }
+    for (int w = 0; w < VW; ++w) partials[(i * splits + sp) * post + j + w] = make_float2(acc[w].s, acc[w].c);
     return;
   }
 #pragma unroll
@@ -353,25 +365,26 @@ k_cols(const float* a, size_t prev, size_t axis, size_t post, int splits, float*
 }
 
 // post > 1, small inputs: one kernel instead of k_cols with axis slices
-// plus k_combine_splits (and their scratch).  A block of 32 warps owns
-// 32 x VW columns of one `prev` index; warp w walks axis slice w (the slices
-// k_cols would use with 32 splits), and the slices are merged in order
-// through shared memory, so the result equals that two-kernel path.
+// plus k_combine_splits (and their scratch).  A block of up to 32 warps owns
+// 32 x VW columns of one `prev` index; warp w walks axis slice w, and the
+// slices are merged in order through shared memory.  Fewer warps where the
+// axis is short or the columns alone nearly fill the GPU (37 x 33153, 4
+// warps: 15 -> 6 us against one thread per column).
 constexpr int kColsBlockWarps = 32;
 // inputs up to 16 MiB take k_cols_block; larger ones stream through k_cols
 constexpr size_t kColsBlockMaxElems = size_t(1) << 22;
 
-template <int OP, bool COMP, int VW>
-__global__ void __launch_bounds__(kColsBlockWarps * 32)
+template <int OP, bool COMP, int VW, int NW>
+__global__ void __launch_bounds__(NW * 32)
 k_cols_block(const float* a, size_t prev, size_t axis, size_t post, float* out, int rebroadcast, float scale) {
-  __shared__ float sh_s[kColsBlockWarps][32 * VW], sh_c[kColsBlockWarps][32 * VW];
+  __shared__ float sh_s[NW][32 * VW], sh_c[NW][32 * VW];
   __shared__ float res[32 * VW];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const size_t ngroups = (post + 32 * VW - 1) / (32 * VW);
   const size_t i = blockIdx.x / ngroups;
   const size_t j = (blockIdx.x % ngroups) * 32 * VW + (size_t)lane * VW;
   const bool cin = j < post;  // VW == 4 only when post % 4 == 0
-  const size_t span = (axis + kColsBlockWarps - 1) / kColsBlockWarps;
+  const size_t span = (axis + NW - 1) / NW;
   const size_t k0 = std::min(axis, (size_t)w * span), k1 = std::min(axis, k0 + span);
   Acc<OP, COMP> acc[VW];
 #pragma unroll
@@ -401,7 +414,12 @@ k_cols_block(const float* a, size_t prev, size_t axis, size_t post, float* out, 
 #pragma unroll
         for (int u = 0; u < 8; ++u) acc[0].push(x[u]);
       }
-      for (; k < k1; ++k) acc[0].push(base[k * post]);
+      float x[7];  // the rest of the slice, its loads together too
+#pragma unroll
+      for (int u = 0; u < 7; ++u) x[u] = k + u < k1 ? base[(k + u) * post] : 0.f;
+#pragma unroll
+      for (int u = 0; u < 7; ++u)
+        if (k + u < k1) acc[0].push(x[u]);
     }
   }
 #pragma unroll
@@ -411,11 +429,12 @@ k_cols_block(const float* a, size_t prev, size_t axis, size_t post, float* out, 
   }
   __syncthreads();
   // warp v < VW merges column v of every lane, slices in order
-  if (w < VW) {
+  if (w < VW) {  // (at least VW warps)
     const int col = lane * VW + w;
     Acc<OP, COMP> r;
     r.init();
-    for (int ww = 0; ww < kColsBlockWarps; ++ww) r.merge(sh_s[ww][col], sh_c[ww][col]);
+#pragma unroll
+    for (int ww = 0; ww < NW; ++ww) r.merge(sh_s[ww][col], sh_c[ww][col]);
     float val = r.value();
     if (OP == VKC_SUM || OP == VKC_PROD) val *= scale;
     res[col] = val;
@@ -423,13 +442,23 @@ k_cols_block(const float* a, size_t prev, size_t axis, size_t post, float* out, 
   __syncthreads();
   if (!cin) return;
   if (rebroadcast) {
-    for (size_t k = w; k < axis; k += kColsBlockWarps)
+    for (size_t k = w; k < axis; k += NW)
 #pragma unroll
       for (int v = 0; v < VW; ++v) out[(i * axis + k) * post + j + v] = res[lane * VW + v];
   } else if (w == 0) {
 #pragma unroll
     for (int v = 0; v < VW; ++v) out[i * post + j + v] = res[lane * VW + v];
   }
+}
+
+template <int OP, bool COMP>
+int combine_splits(vkc_device_t dev, unsigned grid, const float2* partials, size_t prev, size_t axis, size_t post,
+                   int splits, float* out, int rebroadcast, float scale) {
+  const cudaError_t e =
+      vkc::launch_second(k_combine_splits<OP, COMP>, dim3(grid), dim3(kThreads), dev->stream, prev * axis * post,
+                         partials, prev, axis, post, splits, out, rebroadcast, scale);
+  if (e != cudaSuccess) return vkc::set_error(VKC_ERR_CUDA, "reduce_combine launch: %s", cudaGetErrorString(e));
+  return vkc::check_launch("reduce_combine");
 }
 
 template <int OP, bool COMP>
@@ -460,17 +489,15 @@ int reduce_axis_impl(vkc_device_t dev, const float* a, size_t prev, size_t axis,
                                                                           rebroadcast, scale);
       return vkc::check_launch("reduce_rows_block");
     }
-    double* partials = nullptr;
-    int r = vkc::scratch_alloc(dev, sizeof(double) * 2 * prev * splits, (void**)&partials);
+    float2* partials = nullptr;
+    int r = vkc::scratch_alloc(dev, sizeof(float2) * prev * splits, (void**)&partials);
     if (r != VKC_OK) return r;
     k_rows_block<OP, COMP><<<(unsigned)(prev * splits), kThreads, 0, dev->stream>>>(a, prev, axis, splits, out,
                                                                                   partials, rebroadcast, scale);
     r = vkc::check_launch("reduce_rows_block");
     if (r == VKC_OK) {
       unsigned g2 = (unsigned)((prev + kThreads - 1) / kThreads);
-      k_combine_splits<OP, COMP><<<g2, kThreads, 0, dev->stream>>>(partials, prev, axis, 1, splits, out,
-                                                                   rebroadcast, scale);
-      r = vkc::check_launch("reduce_combine");
+      r = combine_splits<OP, COMP>(dev, g2, partials, prev, axis, 1, splits, out, rebroadcast, scale);
     }
     vkc::scratch_free(dev, partials);
     return r;
@@ -485,24 +512,35 @@ int reduce_axis_impl(vkc_device_t dev, const float* a, size_t prev, size_t axis,
     size_t maxs = std::max<size_t>(1, axis / 32);
     splits = (int)std::min<size_t>(std::min<size_t>(want, maxs), 65535);
   }
-  if (splits > 1 && prev * axis * post <= kColsBlockMaxElems) {
+  // warps of k_cols_block: at least 8 rows of the axis each, and no more than
+  // give every SM its threads
+  int warps = 1;
+  while (warps < kColsBlockWarps && (size_t)warps * 16 <= axis && prev * post * warps * 2 <= target_threads) warps *= 2;
+  if (warps >= 4 && prev * axis * post <= kColsBlockMaxElems) {
     // 32 columns per block (scalar loads) unless 128-column blocks still
     // cover every SM: the compensated sum's ~8 instructions per element
     // would otherwise pile onto a few SMs
     const bool vec4 = vec && prev * (post / 128) >= (size_t)dev->sm_count;
     const size_t cols = vec4 ? 128 : 32;
     const size_t blocks = prev * ((post + cols - 1) / cols);
+    auto launch = [&](auto kern) {
+      kern<<<(unsigned)blocks, warps * 32, 0, dev->stream>>>(a, prev, axis, post, out, rebroadcast, scale);
+    };
     if (vec4)
-      k_cols_block<OP, COMP, 4><<<(unsigned)blocks, kColsBlockWarps * 32, 0, dev->stream>>>(a, prev, axis, post, out,
-                                                                                        rebroadcast, scale);
+      warps == 32   ? launch(k_cols_block<OP, COMP, 4, 32>)
+      : warps == 16 ? launch(k_cols_block<OP, COMP, 4, 16>)
+      : warps == 8  ? launch(k_cols_block<OP, COMP, 4, 8>)
+                    : launch(k_cols_block<OP, COMP, 4, 4>);
     else
-      k_cols_block<OP, COMP, 1><<<(unsigned)blocks, kColsBlockWarps * 32, 0, dev->stream>>>(a, prev, axis, post, out,
-                                                                                        rebroadcast, scale);
+      warps == 32   ? launch(k_cols_block<OP, COMP, 1, 32>)
+      : warps == 16 ? launch(k_cols_block<OP, COMP, 1, 16>)
+      : warps == 8  ? launch(k_cols_block<OP, COMP, 1, 8>)
+                    : launch(k_cols_block<OP, COMP, 1, 4>);
     return vkc::check_launch("reduce_cols_block");
   }
-  double* partials = nullptr;
+  float2* partials = nullptr;
   if (splits > 1) {
-    int r = vkc::scratch_alloc(dev, sizeof(double) * 2 * prev * splits * post, (void**)&partials);
+    int r = vkc::scratch_alloc(dev, sizeof(float2) * prev * splits * post, (void**)&partials);
     if (r != VKC_OK) return r;
   }
   dim3 grid((unsigned)((cols_threads + kThreads - 1) / kThreads), (unsigned)splits);
@@ -515,9 +553,7 @@ int reduce_axis_impl(vkc_device_t dev, const float* a, size_t prev, size_t axis,
   int r = vkc::check_launch("reduce_cols");
   if (r == VKC_OK && splits > 1) {
     unsigned g2 = (unsigned)((prev * post + kThreads - 1) / kThreads);
-    k_combine_splits<OP, COMP><<<g2, kThreads, 0, dev->stream>>>(partials, prev, axis, post, splits, out,
-                                                                 rebroadcast, scale);
-    r = vkc::check_launch("reduce_combine");
+    r = combine_splits<OP, COMP>(dev, g2, partials, prev, axis, post, splits, out, rebroadcast, scale);
   }
   vkc::scratch_free(dev, partials);
   return r;
@@ -620,10 +656,7 @@ int reduce_all_noalloc_impl(vkc_device_t dev, const float* a, size_t n, float* o
   k_reduce_all<OP, COMP, NACC><<<(unsigned)grid, kThreads, 0, dev->stream>>>(a, n, partials, out, scale);
   int r = vkc::check_launch("reduce_all_noalloc");
   if (r != VKC_OK) return r;
-  const bool fp64 = (OP == VKC_SUM || OP == VKC_PROD) && n >= (size_t(1) << 24);
-  if (fp64) k_reduce_partials<OP, COMP, true><<<1, 1024, 0, dev->stream>>>(partials, (int)grid, out, scale);
-  else k_reduce_partials<OP, COMP, false><<<1, 1024, 0, dev->stream>>>(partials, (int)grid, out, scale);
-  return vkc::check_launch("reduce_partials_noalloc");
+  return reduce_partials<OP, COMP>(dev, partials, grid, n, out, scale);
 }
 
 }  // namespace
