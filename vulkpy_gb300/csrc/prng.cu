@@ -183,14 +183,160 @@ __device__ __forceinline__ uint32_t next(uint4& s) {
 // [0,1) float from the top 23 bits (prng_xoshiro128pp_float.comp:33).
 __device__ __forceinline__ float to_unit(uint32_t r) { return __uint_as_float((r >> 9) | 0x3f800000u) - 1.0f; }
 
-// Box-Muller pair (prng_box_muller.comp:26-31).
-__device__ __forceinline__ void box_muller(float u0, float u1, float mean, float stddev, float& z0, float& z1) {
-  const float r = sqrtf(-2.0f * logf(1.0f - u0)) * stddev;
-  const float angle = 6.28318530718f * u1;
-  float s, c;
-  sincosf(angle, &s, &c);
-  z0 = __fmaf_rn(r, s, mean);
-  z1 = __fmaf_rn(r, c, mean);
+// Box-Muller (prng_box_muller.comp:26-31): r = sqrt(-2 log(1 - u0)) * stddev,
+// angle = fl(6.28318530718f u1), mean + r sin(angle), mean + r cos(angle).
+//
+// The generator's arguments are narrow (1 - u0 in [2^-23, 1], a multiple of
+// 2^-23; angle in [0, 2 pi]), so the functions are written for them, without
+// the general ones' checks and slow paths, and two pairs go together through
+// packed float32 arithmetic (fma.rn.f32x2).  The kernel is bound by its
+// instructions, the integer ones above all (the generator's own 20 per pair):
+// 2^27 normals took 225 us with logf / sqrtf / sincosf (102 instructions per
+// pair even with these functions in scalar form: 215 us), 177 us so; the
+// store alone takes 79.  Polynomials are minimax fits (Lawson's iteration)
+// made for this file; log within 0.9 ulp and sin, cos within 1.5 ulp over all
+// their arguments.
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2(float a) { return f2(a, a); }
+__device__ __forceinline__ void f2_get(F2 x, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+
+// w = 2^e m with m in [sqrt(1/2), sqrt(2)): e and m - 1.
+__device__ __forceinline__ void log_parts(float w, float& e, float& m) {
+  const int b = __float_as_int(w) - 0x3f3504f3;
+  e = (float)(b >> 23);
+  m = __int_as_float((b & 0x007fffff) + 0x3f3504f3);
+}
+
+// log(w), w in [2^-23, 1]: log(1 + f) = f + f^2 (-1/2 + f P(f)), plus e ln 2
+// in two parts (e times the first is exact).
+__device__ __forceinline__ F2 log_unit(F2 w) {
+  float w0, w1, e0, e1, m0, m1;
+  f2_get(w, w0, w1);
+  log_parts(w0, e0, m0);
+  log_parts(w1, e1, m1);
+  const F2 e = f2(e0, e1), f = f2_add(f2(m0, m1), f2(-1.0f));
+  F2 p = f2_fma(f2(-0.07634501f), f, f2(0.12761581f));
+  p = f2_fma(p, f, f2(-0.13160183f));
+  p = f2_fma(p, f, f2(0.14201757f));
+  p = f2_fma(p, f, f2(-0.16623357f));
+  p = f2_fma(p, f, f2(0.20001227f));
+  p = f2_fma(p, f, f2(-0.2500082f));
+  p = f2_fma(p, f, f2(0.3333333f));
+  const F2 g = f2_fma(f2_mul(f, f), f2_fma(f, p, f2(-0.5f)), f);
+  return f2_fma(e, f2(0x1.62e4p-1f), f2_fma(e, f2(0x1.7f7d1cp-20f), g));
+}
+
+// sqrt(-2 x), x in [-2^4, 0]: one Newton step from the reciprocal root (0
+// gives 1e-18, as if x were -5e-37).
+__device__ __forceinline__ F2 sqrt_minus2(F2 x) {
+  F2 a = f2_mul(x, f2(-2.0f));
+  float a0, a1, y0, y1;
+  f2_get(a, a0, a1);
+  a0 = fmaxf(a0, 1e-36f);
+  a1 = fmaxf(a1, 1e-36f);
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y0) : "f"(a0));
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y1) : "f"(a1));
+  a = f2(a0, a1);
+  const F2 y = f2(y0, y1), g = f2_mul(a, y), mg = f2_mul(g, f2(-1.0f));
+  return f2_fma(f2_fma(mg, g, a), f2_mul(y, f2(0.5f)), g);
+}
+
+// sin of y = a - kf pi (|y| <= pi/2 and a little), negated where the low bit of
+// kt is set.  pi in three parts; the first product leaves an exact difference.
+__device__ __forceinline__ F2 sin_reduced(F2 a, F2 kf, F2 kt) {
+  F2 y = f2_fma(kf, f2(-0x1.921fb6p+1f), a);
+  y = f2_fma(kf, f2(0x1.777a5cp-24f), y);
+  y = f2_fma(kf, f2(0x1.ee59dap-49f), y);
+  const F2 z = f2_mul(y, y);
+  F2 p = f2_fma(f2(0x1.5dbceap-19f), z, f2(-0x1.9f6feep-13f));
+  p = f2_fma(p, z, f2(0x1.110ed4p-7f));
+  p = f2_fma(p, z, f2(-0x1.55554cp-3f));
+  const F2 r = f2_fma(f2_mul(y, z), p, y);
+  float r0, r1, t0, t1;
+  f2_get(r, r0, r1);
+  f2_get(kt, t0, t1);
+  return f2(__uint_as_float(__float_as_uint(r0) ^ (__float_as_uint(t0) << 31)),
+            __uint_as_float(__float_as_uint(r1) ^ (__float_as_uint(t1) << 31)));
+}
+
+// sin and cos of a in [0, 2 pi].  cos(a) = -sin(a - (n + 1/2) pi) (-1)^n, so
+// both are sines of arguments near a zero and keep their relative accuracy.
+__device__ __forceinline__ void sincos_turn(F2 a, F2& s, F2& c) {
+  const F2 inv = f2(0x1.45f306p-2f);
+  // adding 1.5 * 2^23 rounds to a whole number k, which is then in the low bits
+  F2 t = f2_fma(a, inv, f2(12582912.f));
+  s = sin_reduced(a, f2_add(t, f2(-12582912.f)), t);
+  // one more: the sign is (-1)^(n + 1)
+  t = f2_add(f2_fma(a, inv, f2(-0.5f)), f2(12582913.f));
+  c = sin_reduced(a, f2_add(f2_add(t, f2(-12582913.f)), f2(0.5f)), t);
+}
+
+// Two pairs: from raw outputs (r0a, r1a) and (r0b, r1b).  1 - u0 and u1 are
+// exact multiples of 2^-23.
+__device__ __forceinline__ void box_muller2(uint32_t r0a, uint32_t r1a, uint32_t r0b, uint32_t r1b, float mean,
+                                            float stddev, float2& za, float2& zb) {
+  const F2 k0 = f2((float)(r0a >> 9), (float)(r0b >> 9)), k1 = f2((float)(r1a >> 9), (float)(r1b >> 9));
+  const F2 w = f2_fma(k0, f2(-0x1p-23f), f2(1.0f));
+  const F2 r = f2_mul(sqrt_minus2(log_unit(w)), f2(stddev));
+  F2 s, c;
+  sincos_turn(f2_mul(k1, f2(6.28318530718f * 0x1p-23f)), s, c);
+  const F2 z0 = f2_fma(r, s, f2(mean)), z1 = f2_fma(r, c, f2(mean));
+  f2_get(z0, za.x, zb.x);
+  f2_get(z1, za.y, zb.y);
+}
+
+// Steps [b0, b1) of the pair of states (sa, sb) that writes out[step * size +
+// ta] and the element after it, which is there up to step `full`; `pair8`:
+// the two as one 8-byte store.
+__device__ __forceinline__ void normal_steps(uint4& sa, uint4& sb, float* out, uint64_t ta, uint32_t size, uint64_t b0,
+                                             uint64_t b1, uint64_t full, float mean, float stddev, bool pair8) {
+  float* p = out + b0 * size + ta;
+  auto put = [&](float* q, uint64_t step, float2 z) {
+    if (pair8 && step < full) {
+      *reinterpret_cast<float2*>(q) = z;
+    } else {
+      q[0] = z.x;
+      if (step < full) q[1] = z.y;
+    }
+  };
+  uint64_t step = b0;
+  for (; step + 2 <= b1; step += 2, p += 2 * (size_t)size) {
+    const uint32_t r0a = next(sa), r1a = next(sb), r0b = next(sa), r1b = next(sb);
+    float2 za, zb;
+    box_muller2(r0a, r1a, r0b, r1b, mean, stddev, za, zb);
+    put(p, step, za);
+    put(p + size, step + 1, zb);
+  }
+  if (step < b1) {
+    const uint32_t r0 = next(sa), r1 = next(sb);
+    float2 z, unused;
+    box_muller2(r0, r1, r0, r1, mean, stddev, z, unused);
+    put(p, step, z);
+  }
 }
 
 // x times one power of a map, from its byte tables (16 x 256 entries).
@@ -292,23 +438,21 @@ k_generate(uint4* state, uint32_t size, void* out, size_t n, uint32_t low, uint3
   state[t] = s;
 }
 
+// 128 threads: 2^20 states fill the GPU 2.25 times over, and smaller blocks
+// leave less of it idle at the end (256 threads: 185 us, 128: 177 us).
+constexpr int kNormalThreads = 128;
 // Normal numbers with an even number of states: thread p owns states 2p and
 // 2p+1, which produce both halves of every Box-Muller pair it writes.
 // `m` is the length of the uniform stream (n, or n+1 for odd n).
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kNormalThreads)
 k_normal_pairs(uint4* state, uint32_t size, float* out, size_t n, size_t m, float mean, float stddev) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t ta = 2 * p;
   if (ta >= size || (size_t)ta >= m) return;
   uint4 sa = state[ta], sb = state[ta + 1];
-  for (size_t k0 = ta; k0 < m; k0 += size) {
-    const float u0 = to_unit(next(sa));
-    const float u1 = to_unit(next(sb));  // k0 + 1 < m: m is even
-    float z0, z1;
-    box_muller(u0, u1, mean, stddev, z0, z1);
-    out[k0] = z0;
-    if (k0 + 1 < n) out[k0 + 1] = z1;
-  }
+  const uint64_t cnt = (m - ta + size - 1) / size;  // pair steps; m is even
+  const uint64_t full = n > (size_t)ta + 1 ? (n - ta - 2) / size + 1 : 0;  // those with both elements in the output
+  normal_steps(sa, sb, out, ta, size, 0, cnt, full, mean, stddev, ((uintptr_t)out & 7u) == 0);
   state[ta] = sa;
   state[ta + 1] = sb;
 }
@@ -329,19 +473,21 @@ k_normal_pairs_seg(const uint4* __restrict__ state_in, uint4* __restrict__ state
   if (b0 >= cnt) return;
   const uint64_t b1 = min(cnt, b0 + L);
   uint4 sa = advance(pows, state_in[ta], b0), sb = advance(pows, state_in[ta + 1], b0);
-  for (uint64_t step = b0; step < b1; ++step) {
-    const size_t k0 = step * size + ta;
-    const float u0 = to_unit(next(sa));
-    const float u1 = to_unit(next(sb));
-    float z0, z1;
-    box_muller(u0, u1, mean, stddev, z0, z1);
-    out[k0] = z0;
-    if (k0 + 1 < n) out[k0 + 1] = z1;
-  }
+  const uint64_t full = n > (size_t)ta + 1 ? (n - ta - 2) / size + 1 : 0;  // as k_normal_pairs
+  normal_steps(sa, sb, out, ta, size, b0, b1, full, mean, stddev, ((uintptr_t)out & 7u) == 0);
   if (b1 == cnt) {
     state_out[ta] = sa;
     state_out[ta + 1] = sb;
   }
+}
+
+// Of uniforms given by the caller (any float32 values).
+__device__ __forceinline__ void box_muller_any(float u0, float u1, float mean, float stddev, float& z0, float& z1) {
+  const float r = sqrtf(-2.0f * logf(1.0f - u0)) * stddev;
+  float s, c;
+  sincosf(6.28318530718f * u1, &s, &c);
+  z0 = fmaf(r, s, mean);
+  z1 = fmaf(r, c, mean);
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -351,7 +497,7 @@ k_box_muller(const float* u, float* out, size_t n, float mean, float stddev) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += stride) {
     const size_t j = 2 * i;
     float z0, z1;
-    box_muller(u[j], u[j + 1], mean, stddev, z0, z1);
+    box_muller_any(u[j], u[j + 1], mean, stddev, z0, z1);
     out[j] = z0;
     if (j + 1 < n) out[j + 1] = z1;
   }
@@ -495,8 +641,8 @@ VKC_EXPORT int vkc_xoshiro_normal(vkc_device_t dev, uint32_t* state, uint32_t si
             reinterpret_cast<const uint4*>(state), state_out, size, out, n, m, mean, stddev, pows, L, G);
       });
     }
-    unsigned grid = (pairs + kThreads - 1) / kThreads;
-    k_normal_pairs<<<grid, kThreads, 0, dev->stream>>>(reinterpret_cast<uint4*>(state), size, out, n, m, mean,
+    unsigned grid = (pairs + kNormalThreads - 1) / kNormalThreads;
+    k_normal_pairs<<<grid, kNormalThreads, 0, dev->stream>>>(reinterpret_cast<uint4*>(state), size, out, n, m, mean,
                                                         stddev);
     return vkc::check_launch("xoshiro_normal");
   }
