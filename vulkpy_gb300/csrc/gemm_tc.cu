@@ -306,6 +306,7 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
                                | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
     int it = 0, acc_it = 0, lo_it = 0;
     bool ok = true;
+    const uint64_t desc0 = sw128_desc(base);
     for (int u = (int)blockIdx.x; u < units && ok; u += (int)gridDim.x) {
       const PUnit p = unit_of<BN>(u, splits, kps, nk, m_blocks, n_blocks);
       if constexpr (PARTS == 3) {
@@ -321,6 +322,8 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           const int lb = lo_it & 1;
           if (*abort_flag || (lo_first && !mbar_wait(loe_bar(lb), ((lo_it >> 1) & 1) ^ 1))) { ok = false; break; }
           const uint32_t d_lo = tmem + (uint32_t)((2 + lb) * BN);
+          const uint64_t ds = desc_at(desc0, (uint32_t)s * Cfg::kStageBytes);
+          constexpr uint32_t PB = Cfg::kABytes + Cfg::kBBytes;  // part to part
 #pragma unroll
           for (int i = 0; i < 5; ++i) {
             // the tiles this product is the first to read
@@ -332,7 +335,7 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             tc_fence_after();
 #pragma unroll
             for (int k = 0; k < kBK / 16; ++k)
-              mma_bf16(d_lo, sw128_desc(part_a(s, pa[i]) + 32u * k), sw128_desc(part_b(s, pb[i]) + 32u * k), idesc,
+              mma_bf16(d_lo, desc_at(ds, pa[i] * PB + 32u * k), desc_at(ds, pb[i] * PB + Cfg::kABytes + 32u * k), idesc,
                        (i == 0 && k == 0 && lo_first) ? 0u : 1u);
             if (rel[i] >= 0) mma_commit(empty_bar(s * 5 + rel[i]));
           }
@@ -345,8 +348,8 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             tc_fence_after();
 #pragma unroll
             for (int k = sub * STEPS; k < (sub + 1) * STEPS; ++k)
-              mma_bf16(tmem + (uint32_t)(b * BN), sw128_desc(part_a(s, 0) + 32u * k),
-                       sw128_desc(part_b(s, 0) + 32u * k), idesc, k == sub * STEPS ? 0u : 1u);
+              mma_bf16(tmem + (uint32_t)(b * BN), desc_at(ds, 32u * k), desc_at(ds, Cfg::kABytes + 32u * k), idesc,
+                       k == sub * STEPS ? 0u : 1u);
             mma_commit(accf_bar(b));  // the small products issued so far are complete with it
           }
           if (!ok) break;
@@ -366,15 +369,17 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           const int s = it % STAGES;
           if (*abort_flag || !mbar_wait(full_bar(s), (it / STAGES) & 1)) { ok = false; break; }
           tc_fence_after();
+          const uint64_t ds = desc_at(desc0, (uint32_t)s * Cfg::kStageBytes);
+          constexpr uint32_t LO = Cfg::kABytes + Cfg::kBBytes;  // hi to lo
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k) {
-            const uint64_t a = sw128_desc(stage_a(s) + 32u * k);
-            const uint64_t bb = sw128_desc(stage_b(s) + 32u * k);
+            const uint64_t a = desc_at(ds, 32u * k);
+            const uint64_t bb = desc_at(ds, Cfg::kABytes + 32u * k);
             const uint32_t first = (kb == g0 && k == 0) ? 0u : 1u;
             if (PARTS == 2) {
               // small cross terms first, the dominant hi*hi term last
-              mma_bf16(d, a, sw128_desc(stage_blo(s) + 32u * k), idesc, first);
-              mma_bf16(d, sw128_desc(stage_alo(s) + 32u * k), bb, idesc, 1);
+              mma_bf16(d, a, desc_at(ds, LO + Cfg::kABytes + 32u * k), idesc, first);
+              mma_bf16(d, desc_at(ds, LO + 32u * k), bb, idesc, 1);
               mma_bf16(d, a, bb, idesc, 1);
             } else {
               mma_bf16(d, a, bb, idesc, first);

@@ -139,14 +139,42 @@ struct TileTable {
   TileOp op[2 * kMaxGroup];
 };
 
+// Two values as bf16 pairs: hi, lo = bf16(x - hi), or hi, mid and lo.
+template <bool THREE>
+__device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
+  if (THREE) {
+    __nv_bfloat16 h0, m0, l0, h1, m1, l1;
+    split_bf16_3(x0, h0, m0, l0);
+    split_bf16_3(x1, h1, m1, l1);
+    h = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
+    m = (uint32_t)__bfloat16_as_ushort(m0) | ((uint32_t)__bfloat16_as_ushort(m1) << 16);
+    l = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
+  } else {
+    // cvt.rn.bf16x2.f32 rounds both (upper half first); a bf16 is the upper
+    // half of its float32
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(x1), "f"(x0));
+    const float r0 = x0 - __uint_as_float(h << 16), r1 = x1 - __uint_as_float(h & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(l) : "f"(r1), "f"(r0));
+  }
+}
+
 // One 128 x 64 tile per block iteration: load (coalesced along whichever
 // index is contiguous) into shared memory, then write 16-byte chunks of hi
 // (and lo = bf16(x - hi), or mid and lo) at their swizzled positions.  Rows
 // >= rows and k >= K are written as zeros.  THREE: three parts; `repair` is
 // then the count of tiles left to k_gemm_repair_grouped, zeroed here.
+//
+// The pass streams (each element read and written once), but it was bound by
+// its instructions, 38 per element: bounds and 64-bit offsets for every load
+// and four-byte shared-memory reads with two-way bank conflicts (the 64-model
+// step's four passes 87 + 47 + 47 + 52 us, 4.2 TB/s).  So tiles inside the
+// matrix load through a stepped pointer, the shared tile's 16-byte chunks
+// are XOR-swizzled by row so that both stores and the 16-byte reads are free
+// of conflicts, and two values are rounded by one conversion (now TILEUS).
 template <bool THREE>
-__global__ void __launch_bounds__(256, 3) k_tile_operands(const __grid_constant__ TileTable tab, uint32_t* repair) {
-  __shared__ float s[kTileRows][kTileK + 1];
+__global__ void __launch_bounds__(256, 4) k_tile_operands(const __grid_constant__ TileTable tab, uint32_t* repair) {
+  // element (r, k): chunk (k >> 2) ^ (r & 7) of row r, word k & 3
+  __shared__ __align__(16) float s[kTileRows * kTileK];
   const int tid = threadIdx.x;
   if (THREE && blockIdx.x == 0 && tid == 0) *repair = 0u;
   for (int t = blockIdx.x; t < tab.total; t += gridDim.x) {
@@ -154,36 +182,54 @@ __global__ void __launch_bounds__(256, 3) k_tile_operands(const __grid_constant_
     const int local = t - op.tile0;
     const int rt = local / op.kt, kt = local % op.kt;
     const int64_t r0 = (int64_t)rt * kTileRows, k0 = (int64_t)kt * kTileK;
-    __syncthreads();
+    const int64_t ld = op.ld;
+    const int rows = (int)min((int64_t)kTileRows, op.rows - r0), ks = (int)min((int64_t)kTileK, op.k - k0);
+    const bool whole = rows == kTileRows && ks == kTileK;
     // all 32 loads of a thread are issued before the shared-memory stores,
     // so a tile waits for memory once
     constexpr int kPer = kTileRows * kTileK / 256;
     float v[kPer];
     if (op.k_contig) {
+      // a warp reads 32 k of one row: rows tid / 64 + 4 i, k = tid % 64
+      const int k = tid & 63, rb = tid >> 6;
+      const float* p = op.src + (r0 + rb) * ld + k0 + k;
+      if (whole) {
 #pragma unroll
-      for (int i = 0; i < kPer; ++i) {
-        const int e = i * 256 + tid;
-        const int r = e >> 6, k = e & 63;
-        const int64_t gr = r0 + r, gk = k0 + k;
-        v[i] = (gr < op.rows && gk < op.k) ? __ldg(op.src + gr * op.ld + gk) : 0.f;
+        for (int i = 0; i < kPer; ++i, p += 4 * ld) v[i] = __ldg(p);
+      } else {
+#pragma unroll
+        for (int i = 0; i < kPer; ++i, p += 4 * ld) v[i] = (rb + 4 * i < rows && k < ks) ? __ldg(p) : 0.f;
       }
+      __syncthreads();  // the previous tile's reads
 #pragma unroll
       for (int i = 0; i < kPer; ++i) {
-        const int e = i * 256 + tid;
-        s[e >> 6][e & 63] = v[i];
+        const int r = rb + 4 * i;
+        s[r * kTileK + ((((k >> 2) ^ (r & 7)) << 2) | (k & 3))] = v[i];
       }
     } else {
+      // a warp reads 8 rows of 4 k's (32 contiguous bytes each): rows
+      // 8 (w & 3) + lane % 8 + 32 (i & 3), k = 4 (w >> 2) + lane / 8 + 8 (i >> 2)
+      const int lane = tid & 31, w = tid >> 5;
+      const int r = 8 * (w & 3) + (lane & 7), kq = 4 * (w >> 2) + (lane >> 3);
+      const float* p = op.src + (k0 + kq) * ld + r0 + r;
+      if (whole) {
 #pragma unroll
-      for (int i = 0; i < kPer; ++i) {
-        const int e = i * 256 + tid;
-        const int k = e >> 7, r = e & 127;
-        const int64_t gr = r0 + r, gk = k0 + k;
-        v[i] = (gr < op.rows && gk < op.k) ? __ldg(op.src + gk * op.ld + gr) : 0.f;
+        for (int i = 0; i < kPer; ++i) {
+          v[i] = __ldg(p + 32 * (i & 3));
+          if ((i & 3) == 3) p += 8 * ld;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+          v[i] = (r + 32 * (i & 3) < rows && kq + 8 * (i >> 2) < ks) ? __ldg(p + 32 * (i & 3)) : 0.f;
+          if ((i & 3) == 3) p += 8 * ld;
+        }
       }
+      __syncthreads();
 #pragma unroll
       for (int i = 0; i < kPer; ++i) {
-        const int e = i * 256 + tid;
-        s[e & 127][e >> 7] = v[i];
+        const int rr = r + 32 * (i & 3), k = kq + 8 * (i >> 2);
+        s[rr * kTileK + ((((k >> 2) ^ (rr & 7)) << 2) | (k & 3))] = v[i];
       }
     }
     __syncthreads();
@@ -195,34 +241,20 @@ __global__ void __launch_bounds__(256, 3) k_tile_operands(const __grid_constant_
     for (int i = 0; i < 4; ++i) {
       const int cidx = i * 256 + tid;  // 128 rows x 8 chunks of 8 elements
       const int r = cidx >> 3, c = cidx & 7;
-      uint32_t h[4], l[4];
+      // lanes with c >= 4 read their second half first: eight lanes' 16-byte
+      // reads then cover all banks
+      const int odd = (c >> 2) & 1;
+      const float4* row = reinterpret_cast<const float4*>(s + r * kTileK);
+      const float4 a = row[(2 * c + odd) ^ (r & 7)], b = row[(2 * c + 1 - odd) ^ (r & 7)];
+      const float4 x = odd ? b : a, y = odd ? a : b;
+      uint32_t h[4], m[4], l[4];
+      split_pair<THREE>(x.x, x.y, h[0], m[0], l[0]);
+      split_pair<THREE>(x.z, x.w, h[1], m[1], l[1]);
+      split_pair<THREE>(y.x, y.y, h[2], m[2], l[2]);
+      split_pair<THREE>(y.z, y.w, h[3], m[3], l[3]);
       const size_t off = (size_t)r * 128 + (size_t)(((c ^ (r & 7)) << 4));
-      if (THREE) {
-        uint32_t m[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          __nv_bfloat16 h0, m0, l0, h1, m1, l1;
-          split_bf16_3(s[r][c * 8 + 2 * j], h0, m0, l0);
-          split_bf16_3(s[r][c * 8 + 2 * j + 1], h1, m1, l1);
-          h[j] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
-          m[j] = (uint32_t)__bfloat16_as_ushort(m0) | ((uint32_t)__bfloat16_as_ushort(m1) << 16);
-          l[j] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
-        }
-        *reinterpret_cast<uint4*>(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
-        *reinterpret_cast<uint4*>(mid + off) = make_uint4(m[0], m[1], m[2], m[3]);
-        *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
-        continue;
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float x0 = s[r][c * 8 + 2 * j], x1 = s[r][c * 8 + 2 * j + 1];
-        const __nv_bfloat16 h0 = __float2bfloat16_rn(x0), h1 = __float2bfloat16_rn(x1);
-        const __nv_bfloat16 l0 = __float2bfloat16_rn(x0 - __bfloat162float(h0));
-        const __nv_bfloat16 l1 = __float2bfloat16_rn(x1 - __bfloat162float(h1));
-        h[j] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
-        l[j] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
-      }
       *reinterpret_cast<uint4*>(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
+      if (THREE) *reinterpret_cast<uint4*>(mid + off) = make_uint4(m[0], m[1], m[2], m[3]);
       if (lo) *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
     }
   }
@@ -392,77 +424,82 @@ k_gemm_tc_grouped(const __grid_constant__ TcTable tab, uint32_t* err, uint32_t* 
     // ---------------- MMA issuer
     uint32_t g = 0, acc = 0;  // g: K blocks (stage ring), acc: accumulations (TMEM ring)
     uint32_t lo_it = 0;       // PARTS == 3: accumulations of small products
+    const uint64_t desc0 = sw128_desc(base);
     bool ok = true;
     for (int t = blockIdx.x; t < tab.total && ok; t += gridDim.x) {
       const TcProb& P = tab.p[find_problem(tab.p, tab.count, t)];
       const int bn = tile_bn(P, ((t - P.tile0) % P.tiles_n) * BN);
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) |
                              ((uint32_t)(kTileRows >> 4) << 24);
+      const int kt = P.kt, klast = P.klast;
+      const bool swap = P.swap != 0;
       if constexpr (PARTS == 3) {
         // stage tiles: 0 a_hi, 1 b_hi, 2 a_lo, 3 b_lo, 4 a_mid, 5 b_mid; the
         // products in k_gemm_tcp's order (hi*mid before mid*hi in terms of
         // op(A), op(B), which change sides in a swapped problem)
-        for (int kb = 0; kb < P.kt && ok; ++kb, ++g, ++acc) {
+        for (int kb = 0; kb < kt && ok; ++kb, ++g, ++acc) {
           const int s = g % S, b = acc & 1, lb = 2 + (lo_it & 1);
-          const bool lo_first = kb % kLoSpan == 0, lo_last = kb % kLoSpan == kLoSpan - 1 || kb == P.kt - 1;
+          const bool lo_first = kb % kLoSpan == 0, lo_last = kb % kLoSpan == kLoSpan - 1 || kb == kt - 1;
           if (*abort_flag || (lo_first && !mbar_wait(acce_bar(lb), ((lo_it >> 1) & 1) ^ 1)) ||
               !mbar_wait(acce_bar(b), ((acc >> 1) & 1) ^ 1) || !mbar_wait(full_bar(s), (g / S) & 1)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const int ksteps = kb == P.kt - 1 ? P.klast : kTileK / 16;
+          const int ksteps = kb == kt - 1 ? klast : kTileK / 16;
           const uint32_t d_lo = tmem + (uint32_t)(lb * BN), d_hi = tmem + (uint32_t)(b * BN);
+          const uint64_t ds = desc_at(desc0, (uint32_t)s * Cfg::kStageBytes);
           constexpr int ta[5] = {4, 0, 4, 0, 2}, tb[5] = {5, 5, 1, 3, 1};          // mm hm mh hl lh
           constexpr int sa[5] = {4, 4, 0, 2, 0}, sb[5] = {5, 1, 5, 1, 3};          // swapped sides
 #pragma unroll
           for (int i = 0; i < 5; ++i) {
-            const uint32_t wa = (uint32_t)(P.swap ? sa[i] : ta[i]), wb = (uint32_t)(P.swap ? sb[i] : tb[i]);
-            for (int k = 0; k < ksteps; ++k)
-              mma_bf16(d_lo, sw128_desc(stage(s, wa) + 32u * k), sw128_desc(stage(s, wb) + 32u * k), idesc,
-                       (i == 0 && k == 0 && lo_first) ? 0u : 1u);
+            const uint64_t da = desc_at(ds, (uint32_t)(swap ? sa[i] : ta[i]) * kTileBytes);
+            const uint64_t db = desc_at(ds, (uint32_t)(swap ? sb[i] : tb[i]) * kTileBytes);
+#pragma unroll
+            for (int k = 0; k < kTileK / 16; ++k)
+              if (k < ksteps)
+                mma_bf16(d_lo, desc_at(da, 32u * k), desc_at(db, 32u * k), idesc,
+                         (i == 0 && k == 0 && lo_first) ? 0u : 1u);
           }
-          for (int k = 0; k < ksteps; ++k)
-            mma_bf16(d_hi, sw128_desc(stage(s, 0) + 32u * k), sw128_desc(stage(s, 1) + 32u * k), idesc, k ? 1u : 0u);
+#pragma unroll
+          for (int k = 0; k < kTileK / 16; ++k)
+            if (k < ksteps)
+              mma_bf16(d_hi, desc_at(ds, 32u * k), desc_at(ds, kTileBytes + 32u * k), idesc, k ? 1u : 0u);
           mma_commit(empty_bar(s));
           mma_commit(accf_bar(b));
           if (lo_last) ++lo_it;
         }
         continue;
       }
-      const int span = X3 ? kDrainX3 : P.kt;  // K blocks per TMEM accumulation
-      for (int g0 = 0; g0 < P.kt && ok; g0 += span, ++acc) {
+      const int span = X3 ? kDrainX3 : kt;  // K blocks per TMEM accumulation
+      // cross terms in k_gemm_tcp's order: op(A)_hi op(B)_lo, op(A)_lo
+      // op(B)_hi, then hi*hi (a swapped problem has op(B) on the A side, so
+      // its cross terms come in the other order)
+      const uint32_t xa = swap ? 2u : 0u, xb = swap ? 1u : 3u, ya = swap ? 0u : 2u, yb = swap ? 3u : 1u;
+      for (int g0 = 0; g0 < kt && ok; g0 += span, ++acc) {
         const int b = acc % kAccBufs;
         if (*abort_flag || !mbar_wait(acce_bar(b), ((acc / kAccBufs) & 1) ^ 1)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d = tmem + (uint32_t)(b * BN);
-        const int g1 = min(P.kt, g0 + span);
+        const int g1 = min(kt, g0 + span);
         for (int kb = g0; kb < g1; ++kb, ++g) {
           const int s = g % S;
           if (*abort_flag || !mbar_wait(full_bar(s), (g / S) & 1)) { ok = false; break; }
           tc_fence_after();
-          const int ksteps = kb == P.kt - 1 ? P.klast : kTileK / 16;
+          const int ksteps = kb == kt - 1 ? klast : kTileK / 16;
+          const uint64_t da = desc_at(desc0, (uint32_t)s * Cfg::kStageBytes), db = desc_at(da, kTileBytes);
+          const uint64_t dxa = desc_at(da, xa * kTileBytes), dxb = desc_at(da, xb * kTileBytes);
+          const uint64_t dya = desc_at(da, ya * kTileBytes), dyb = desc_at(da, yb * kTileBytes);
 #pragma unroll
           for (int k = 0; k < kTileK / 16; ++k) {
             if (k >= ksteps) break;
-            const uint64_t a = sw128_desc(stage(s, 0) + 32u * k);
-            const uint64_t bb = sw128_desc(stage(s, 1) + 32u * k);
             const uint32_t first = (kb == g0 && k == 0) ? 0u : 1u;
             if (X3) {
-              // the same order of products as k_gemm_tcp: op(A)_hi op(B)_lo,
-              // op(A)_lo op(B)_hi, then hi*hi (a swapped problem has op(B)
-              // on the A side, so its cross terms come in the other order)
-              const uint64_t alo = sw128_desc(stage(s, 2) + 32u * k), blo = sw128_desc(stage(s, 3) + 32u * k);
-              if (P.swap) {
-                mma_bf16(d, alo, bb, idesc, first);
-                mma_bf16(d, a, blo, idesc, 1);
-              } else {
-                mma_bf16(d, a, blo, idesc, first);
-                mma_bf16(d, alo, bb, idesc, 1);
-              }
-              mma_bf16(d, a, bb, idesc, 1);
+              mma_bf16(d, desc_at(dxa, 32u * k), desc_at(dxb, 32u * k), idesc, first);
+              mma_bf16(d, desc_at(dya, 32u * k), desc_at(dyb, 32u * k), idesc, 1);
+              mma_bf16(d, desc_at(da, 32u * k), desc_at(db, 32u * k), idesc, 1);
             } else {
-              mma_bf16(d, a, bb, idesc, first);
+              mma_bf16(d, desc_at(da, 32u * k), desc_at(db, 32u * k), idesc, first);
             }
           }
           mma_commit(empty_bar(s));

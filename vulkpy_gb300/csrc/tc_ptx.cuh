@@ -77,6 +77,19 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
   return d;
 }
 
+// The descriptor of a tile `bytes` (a multiple of 16) after that of `d`: one
+// addition, since addresses stay below 2^18.  One thread issues all MMAs, and
+// deriving two descriptors from an address for each costs it more cycles than
+// a small MMA runs.
+__device__ __forceinline__ uint64_t desc_at(uint64_t d, uint32_t bytes) {
+  uint32_t lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(d));
+  lo += bytes >> 4;
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate) {
   asm volatile(
