@@ -170,7 +170,8 @@ __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& h, uint
 // step's four passes 87 + 47 + 47 + 52 us, 4.2 TB/s).  So tiles inside the
 // matrix load through a stepped pointer, the shared tile's 16-byte chunks
 // are XOR-swizzled by row so that both stores and the 16-byte reads are free
-// of conflicts, and two values are rounded by one conversion (now TILEUS).
+// of conflicts, and two values are rounded by one conversion (63 + 32 + 34 + 38
+// us with four blocks per SM).
 template <bool THREE>
 __global__ void __launch_bounds__(256, 4) k_tile_operands(const __grid_constant__ TileTable tab, uint32_t* repair) {
   // element (r, k): chunk (k >> 2) ^ (r & 7) of row r, word k & 3
