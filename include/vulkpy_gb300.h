@@ -67,7 +67,8 @@ enum vkc_reduce_precision {
 /* matmul arithmetic */
 enum vkc_matmul_precision {
   VKC_MM_FP32 = 0,   /* fp32 (the drop-in default): FMAs, or exact three-part
-                      * bf16 operands on tcgen05 where there is enough work */
+                      * bf16 operands on tcgen05 (vkc_matmul: with enough
+                      * work; the others: from m n k = 2^30 on)               */
   VKC_MM_BF16 = 1,   /* tcgen05 bf16 x bf16 -> fp32 accumulate                */
   VKC_MM_BF16X3 = 2  /* tcgen05 split-bf16: hi*hi + hi*lo + lo*hi, fp32 acc   */
 };
@@ -328,7 +329,8 @@ int vkc_gemm(vkc_device_t dev, int precision, int trans_a, int trans_b,
  * per 128-row tile) and the split-K count; splits = 0 removes an entry.  The
  * table written by vulkpy_gb300/autotune.py is loaded at import; shapes
  * without an entry use 256-wide tiles and an occupancy heuristic for splits.
- * get: the plan a shape will use.  tune_set/tune_get are the same with
+ * fp32: tile_n = 256 sets the split count of the FMA GEMM, 128 that of the
+ * three-part tensor-core product too.  get: the plan a shape will use.  tune_set/tune_get are the same with
  * tile_n = 256 / without it.  No reference counterpart (matmul.comp has no
  * tiling). */
 int vkc_gemm_plan_set(int precision, int64_t m, int64_t n, int64_t k, int splits, int tile_n);

@@ -32,9 +32,13 @@ def vk():
 def plans():
     """vkc_gemm_plan_set, and the shipped table again afterwards."""
     from vulkpy_gb300 import _lib, autotune
-    yield lambda m, n, k, s: _lib.lib.vkc_gemm_plan_set(_lib.MM_FP32, m, n, k, s, 256)
+    yield lambda m, n, k, s: _lib.lib.vkc_gemm_plan_set(_lib.MM_FP32, m, n, k, s, 128)
     _lib.lib.vkc_gemm_tune_clear()
     autotune.load_table()
+
+
+def _matmul(vk, gpu, A, B):
+    return np.asarray(vk.Array(gpu, data=A) @ vk.Array(gpu, data=B)).copy()
 
 
 def _gemm(vk, gpu, A, B, ta, tb, alpha=1.0, beta=0.0, C0=None):
@@ -63,12 +67,23 @@ def _operands(rng, M, N, K, ta, tb):
 def test_accuracy_at_tile_edges(gpu, vk, plans, m, n, k, splits):
     rng = np.random.default_rng(m + 3 * n + 7 * k)
     plans(m, n, k, splits)
-    for ta, tb in ((0, 0), (1, 1)):
-        A, B = _operands(rng, m, n, k, ta, tb)
-        C0 = rng.standard_normal((m, n)).astype(np.float32)
-        e = (A.T if ta else A).astype(np.float64) @ (B.T if tb else B).astype(np.float64)
-        assert rel_fro(_gemm(vk, gpu, A, B, ta, tb), e) < BOUND
-        assert rel_fro(_gemm(vk, gpu, A, B, ta, tb, 0.5, 2.0, C0), 0.5 * e + 2.0 * C0) < BOUND
+    A, B = _operands(rng, m, n, k, 0, 0)
+    assert rel_fro(_matmul(vk, gpu, A, B), A.astype(np.float64) @ B) < BOUND
+    assert gpu.check_errors() == 0
+
+
+# vkc_gemm takes the path from m n k = 2^30 on: transposes, alpha, beta
+@pytest.mark.parametrize("m,n,k", [(1025, 1030, 1100), (513, 4099, 520), (2100, 513, 1024)])
+@pytest.mark.parametrize("splits", [1, 2])
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_gemm_forms(gpu, vk, plans, m, n, k, splits, ta, tb):
+    rng = np.random.default_rng(m + 3 * n + 7 * k)
+    plans(m, n, k, splits)
+    A, B = _operands(rng, m, n, k, ta, tb)
+    C0 = rng.standard_normal((m, n)).astype(np.float32)
+    e = (A.T if ta else A).astype(np.float64) @ (B.T if tb else B).astype(np.float64)
+    assert rel_fro(_gemm(vk, gpu, A, B, ta, tb), e) < BOUND
+    assert rel_fro(_gemm(vk, gpu, A, B, ta, tb, 0.5, 2.0, C0), 0.5 * e + 2.0 * C0) < BOUND
     assert gpu.check_errors() == 0
 
 
@@ -123,11 +138,21 @@ def test_values_outside_the_split(gpu, vk, plans, kind, splits):
     plans(m, n, k, splits)
     A, B = _operands(rng, m, n, k, 0, 0)
     _poison(A, B, kind)
-    _same(_gemm(vk, gpu, A, B, 0, 0), A, B)
+    _same(_matmul(vk, gpu, A, B), A, B)
+    assert gpu.check_errors() == 0
+
+
+@pytest.mark.parametrize("kind", ["inf", "nan", "huge", "large", "tiny"])
+@pytest.mark.parametrize("splits", [1, 2])
+def test_values_outside_the_split_in_gemm(gpu, vk, plans, kind, splits):
+    rng = np.random.default_rng(12)
+    m, n, k = 1040, 1030, 1010
+    plans(m, n, k, splits)
+    A, B = _operands(rng, m, n, k, 0, 0)
+    _poison(A, B, kind)
     _same(_gemm(vk, gpu, np.ascontiguousarray(A.T), np.ascontiguousarray(B.T), 1, 1), A, B)
     # beta: C is read once, by whichever kernel computes the result
-    C0 = np.full((m, n), 3.0, np.float32)
-    got = _gemm(vk, gpu, A, B, 0, 0, 1.0, 1.0, C0)
+    got = _gemm(vk, gpu, A, B, 0, 0, 1.0, 1.0, np.full((m, n), 3.0, np.float32))
     clean = np.ones((m, n), bool)
     clean[[1, 40], :] = False
     clean[:, 2] = False
@@ -144,7 +169,7 @@ def test_grouped_equals_single_with_unusual_values(gpu, vk, plans, kind):
     vkc_gemm's bits, recomputed results included."""
     rng = np.random.default_rng(3)
     As, Bs, ref = [], [], []
-    for m, n, k in ((150, 140, 200), (64, 300, 130), (50, 129, 64), (41, 3, 777), (130, 64, 512), (45, 70, 20)):
+    for m, n, k in ((1040, 1030, 1010), (64, 4200, 4100), (50, 129, 64), (2100, 520, 1000)):
         plans(m, n, k, 1)
         A, B = _operands(rng, m, n, k, 0, 0)
         if k > 64:

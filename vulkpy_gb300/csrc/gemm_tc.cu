@@ -799,6 +799,22 @@ inline int64_t cta_tiles(int64_t M, int64_t N, int bn) {
   return ((M + kBM - 1) / kBM) * ((N + bn - 1) / bn);
 }
 
+// K ranges of the three-part product: an entry set with tile width 128, else
+// as many as fill the GPU once with at least two K blocks each (within 5% of
+// the best of 1 .. 16 over 107 shapes from 128 x 128 to 4096^2).
+constexpr int kMmFp32Tc = 8;  // its entries' precision in the table
+int fp32_tc_splits(vkc_device_t dev, int64_t M, int64_t N, int64_t K) {
+  const int nk = (int)std::max<int64_t>(1, (K + kBK - 1) / kBK);
+  {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    auto it = g_tune.find(tune_key(kMmFp32Tc, bucket(M), bucket(N), bucket(K)));
+    if (it != g_tune.end()) return std::max(1, std::min(it->second & 0xffff, nk));
+  }
+  const int64_t tiles = cta_tiles(M, N, 128);
+  if (tiles * 2 > dev->sm_count || nk < 4) return 1;
+  return (int)std::max<int64_t>(1, std::min<int64_t>({dev->sm_count / tiles, nk / 2, 16}));
+}
+
 TcPlan choose_plan(vkc_device_t dev, int precision, int64_t M, int64_t N, int64_t K) {
   const int nk = (int)std::max<int64_t>(1, (K + kBK - 1) / kBK);
   {
@@ -1098,8 +1114,16 @@ VKC_EXPORT int vkc_gemm_plan_set(int precision, int64_t m, int64_t n, int64_t k,
   VKC_REQUIRE(tile_n == 128 || tile_n == 256, "tile width must be 128 or 256");
   std::lock_guard<std::mutex> lk(vkc::g_tune_mu);
   auto key = vkc::tune_key(precision, vkc::bucket(m), vkc::bucket(n), vkc::bucket(k));
-  if (splits == 0) vkc::g_tune.erase(key);
-  else vkc::g_tune[key] = splits | (tile_n << 16);
+  // fp32: width 256 sets the FMA GEMM's ranges, width 128 the tensor path's too
+  const bool fp32 = precision == VKC_MM_FP32;
+  auto tc = vkc::tune_key(vkc::kMmFp32Tc, vkc::bucket(m), vkc::bucket(n), vkc::bucket(k));
+  if (splits == 0) {
+    vkc::g_tune.erase(key);
+    if (fp32) vkc::g_tune.erase(tc);
+  } else {
+    vkc::g_tune[key] = splits | (tile_n << 16);
+    if (fp32 && tile_n == 128) vkc::g_tune[tc] = splits;
+  }
   return VKC_OK;
 }
 
@@ -1200,7 +1224,8 @@ int gemm_tc(vkc_device_t dev, int precision, bool ta, bool tb, int64_t M, int64_
 }
 
 int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t K, float alpha, const float* A,
-              int64_t lda, const float* B, int64_t ldb, float beta, float* C, int64_t ldc, GemmEpilogue epi) {
+              int64_t lda, const float* B, int64_t ldb, float beta, float* C, int64_t ldc, GemmEpilogue epi,
+              bool layer) {
   GemmEpilogue plain = epi;
   plain.dmask = nullptr;
   plain.dact = VKC_ACT_NONE;
@@ -1209,7 +1234,7 @@ int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t 
     return r == VKC_OK ? act_deriv_after(dev, epi, C, M, N, ldc) : r;
   };
   const int ranges = simt_splits(dev, M, N, K);
-  if (!fp32_on_tensor_cores(M, N, K, ranges)) return simt();
+  if (!(layer ? layer_fp32_on_tensor_cores(M, N, K, ranges) : fp32_on_tensor_cores(M, N, K, ranges))) return simt();
   const int64_t Kp = (K + kBK - 1) / kBK * kBK;
   const int64_t tiles = cta_tiles(M, N, 128);
   const size_t elems = 3 * (size_t)(M + N) * Kp;
@@ -1227,7 +1252,7 @@ int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t 
   CUtensorMap ma, mb;
   if (r == VKC_OK) r = make_map(&ma, a, 3 * M, Kp, kBM);
   if (r == VKC_OK) r = make_map(&mb, b, 3 * N, Kp, 128);
-  const int splits = std::min<int>(ranges, (int)(Kp / kBK));
+  const int splits = fp32_tc_splits(dev, M, N, K);
   if (r == VKC_OK)
     // K in short ranges: two hi*hi accumulations per K block (256^3 in 4
     // ranges, U[0,1) data: error 8.0e-8 -> 5.5e-8, where FMAs in 16 ranges of

@@ -40,10 +40,24 @@ inline bool fp32_on_tensor_cores(int64_t M, int64_t N, int64_t K, int splits) {
   return chain + (splits > 1 ? 32 : 0) >= 96 || M * N >= (1 << 24);
 }
 
+// The same for the products of layers: vkc_gemm, the grouped GEMM and the
+// Dense calls, which agree with one another bit for bit.  A layer's call is
+// bound by the host up to about 2^30 (256 x 784 -> 1024 -> 1024 -> 10 run call
+// by call: 176 us a step with FMAs, 191 with the tensor path's extra launches;
+// 4096 x 2048 -> 2048 forward and backward: 2410 us with FMAs, 637 on the
+// tensor cores).  In a network a ReLU passes another rounding on as another
+// sign wherever a value is within it of zero, so below that line trained
+// models keep the values of the FMA path too.
+inline bool layer_fp32_on_tensor_cores(int64_t M, int64_t N, int64_t K, int splits) {
+  return fp32_on_tensor_cores(M, N, K, splits) && M * N * K >= (int64_t(1) << 30);
+}
+
 // C = act(alpha * op(A) op(B) + beta * C + bias) (* act'(dmask)) in fp32: on
-// the tensor cores or with FMAs, by fp32_on_tensor_cores.
+// the tensor cores or with FMAs, by fp32_on_tensor_cores (layer: by
+// layer_fp32_on_tensor_cores).
 int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t K, float alpha, const float* A,
-              int64_t lda, const float* B, int64_t ldb, float beta, float* C, int64_t ldc, GemmEpilogue epi);
+              int64_t lda, const float* B, int64_t ldb, float beta, float* C, int64_t ldc, GemmEpilogue epi,
+              bool layer = true);
 
 // C *= act'(epi.dmask) as a launch of its own, after a GEMM that could not
 // apply it (nn.cu).

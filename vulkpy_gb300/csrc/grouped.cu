@@ -1198,10 +1198,10 @@ int gemm_grouped(vkc_device_t dev, int precision, const vkc_gemm_problem* proble
   std::vector<int> order = work_order(problems, count);
   std::vector<int> tc, simt;
   // K = 0 has no tensor-core work: C = act(beta*C + bias) through the SIMT path
-  // fp32: as vkc_gemm without a split of K decides
+  // fp32: as vkc_gemm and the Dense calls decide
   for (int i : order) {
     const vkc_gemm_problem& q = problems[i];
-    const bool on_tc = precision == VKC_MM_FP32 ? fp32_on_tensor_cores(q.m, q.n, q.k, 1) : q.k > 0;
+    const bool on_tc = precision == VKC_MM_FP32 ? layer_fp32_on_tensor_cores(q.m, q.n, q.k, 1) : q.k > 0;
     (on_tc ? tc : simt).push_back(i);
   }
   // Another problem may read an updated value as its operand (dx = dy W

@@ -4,9 +4,12 @@
 #include "gemm_simt.cuh"
 #include "gemm_tc.cuh"
 
-VKC_EXPORT int vkc_gemm(vkc_device_t dev, int precision, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k,
-                        float alpha, const float* a, int64_t lda, const float* b, int64_t ldb, float beta, float* c,
-                        int64_t ldc) {
+namespace {
+
+// layer: the fp32 arithmetic of layers (vkc_gemm) or of a product by itself (vkc_matmul).
+int gemm_entry(vkc_device_t dev, int precision, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k, float alpha,
+               const float* a, int64_t lda, const float* b, int64_t ldb, float beta, float* c, int64_t ldc,
+               bool layer) {
   VKC_BIND(dev);
   VKC_REQUIRE(m >= 0 && n >= 0 && k >= 0, "negative matmul size");
   if (m == 0 || n == 0) return VKC_OK;
@@ -22,7 +25,7 @@ VKC_EXPORT int vkc_gemm(vkc_device_t dev, int precision, int trans_a, int trans_
   switch (precision) {
     case VKC_MM_FP32:
       return vkc::gemm_fp32(dev, trans_a != 0, trans_b != 0, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc,
-                            vkc::GemmEpilogue{});
+                            vkc::GemmEpilogue{}, layer);
     case VKC_MM_BF16:
     case VKC_MM_BF16X3:
       return vkc::gemm_tc(dev, precision, trans_a != 0, trans_b != 0, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc,
@@ -32,7 +35,15 @@ VKC_EXPORT int vkc_gemm(vkc_device_t dev, int precision, int trans_a, int trans_
   }
 }
 
+}  // namespace
+
+VKC_EXPORT int vkc_gemm(vkc_device_t dev, int precision, int trans_a, int trans_b, int64_t m, int64_t n, int64_t k,
+                        float alpha, const float* a, int64_t lda, const float* b, int64_t ldb, float beta, float* c,
+                        int64_t ldc) {
+  return gemm_entry(dev, precision, trans_a, trans_b, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, true);
+}
+
 VKC_EXPORT int vkc_matmul(vkc_device_t dev, int precision, const float* a, const float* b, float* c, int64_t m,
                           int64_t k, int64_t n) {
-  return vkc_gemm(dev, precision, 0, 0, m, n, k, 1.0f, a, k > 0 ? k : 1, b, n, 0.0f, c, n);
+  return gemm_entry(dev, precision, 0, 0, m, n, k, 1.0f, a, k > 0 ? k : 1, b, n, 0.0f, c, n, false);
 }
