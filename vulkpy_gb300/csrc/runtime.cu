@@ -608,6 +608,8 @@ VKC_EXPORT int vkc_side_begin(vkc_device_t dev) {
   VKC_REQUIRE(dev->stream == dev->own_stream, "branch: not on the device's own stream");
   VKC_CUDA(cudaEventRecord(dev->side_fork, dev->stream));
   VKC_CUDA(cudaStreamWaitEvent(dev->side_stream, dev->side_fork, 0));
+  // in a capture the bias branch must have forked too before it is joined
+  if (!dev->side_pending) VKC_CUDA(cudaStreamWaitEvent(dev->bias_stream, dev->side_fork, 0));
   VKC_CUDA(cudaEventRecord(dev->bias_join, dev->bias_stream));
   VKC_CUDA(cudaStreamWaitEvent(dev->side_stream, dev->bias_join, 0));
   dev->stream = dev->side_stream;

@@ -126,23 +126,56 @@ class GroupedSequence:
         dys = [Array(gpu, shape=p.shape) for p in preds]
         for y in ys:
             y._dptr()
-        check(lib.vkc_mse_grouped(gpu._dev.h, _ptrs([p._dptr() for p in preds]), _ptrs([y._dptr() for y in ys]),
-                                  _ptrs([d._buf.ptr or 0 for d in dys]),
-                                  (C.c_int64 * n)(*[p.shape[0] for p in preds]),
-                                  (C.c_int64 * n)(*[p.shape[1] for p in preds]), losses._buf.ptr or 0, n))
-        losses._written()
+        px, py = _ptrs([p._dptr() for p in preds]), _ptrs([y._dptr() for y in ys])
+        batch = (C.c_int64 * n)(*[p.shape[0] for p in preds])
+        cols = (C.c_int64 * n)(*[p.shape[1] for p in preds])
+        check(lib.vkc_mse_grouped(gpu._dev.h, px, py, _ptrs([d._buf.ptr or 0 for d in dys]), batch, cols, None, n))
         for d in dys:
             d._written()
-        # ---- backward
-        for l in range(nl - 1, -1, -1):
+        # The loss values and the bias gradients and steps are needed by
+        # nothing in the backward: on the device's own stream they run on the
+        # side branch, beside the tiling passes and GEMMs, and join at the
+        # end.  What the branch reads (the gradients passed down) is kept
+        # until then: freed on the main stream before, it could be handed to
+        # the next allocation.
+        keep = [dys]
+        side = gpu._dev.own_stream()
+        if side:
+            check(lib.vkc_side_defer(gpu._dev.h, 1))
+        try:
+            self._beside(side, lambda: check(lib.vkc_mse_grouped(
+                gpu._dev.h, px, py, None, batch, cols, losses._buf.ptr or 0, n)))
+            losses._written()
+            self._backward(acts, dys, keep, side)
+        finally:
+            if side:
+                check(lib.vkc_side_defer(gpu._dev.h, 0))
+            del keep
+        return preds, losses
+
+    def _beside(self, side: bool, run):
+        """``run()`` on the side branch (after everything issued so far)."""
+        h = self.gpu._dev.h
+        if not side:
+            run()
+            return
+        check(lib.vkc_side_begin(h))
+        try:
+            run()
+        finally:
+            check(lib.vkc_side_end(h))
+
+    def _backward(self, acts, dys, keep, side: bool):
+        gpu = self.gpu
+        n = len(self.models)
+        for l in range(len(self._plan[0]) - 1, -1, -1):
             dense = [self._plan[m][l][0] for m in range(n)]
             # bias gradients (overwrite: db = 0 + sum_b dy), then b += (-lr) db
-            check(lib.vkc_colsum_update_grouped(gpu._dev.h, _ptrs([dy._dptr() for dy in dys]),
-                                                _ptrs([d.b.grad._dptr() for d in dense]),
-                                                (C.c_int64 * n)(*[dy.shape[0] for dy in dys]),
-                                                (C.c_int64 * n)(*[d.output_dim for d in dense]), n, 1,
-                                                _ptrs([d.b.value._dptr() for d in dense]),
-                                                (C.c_float * n)(*[-d.b.opt_state.opt.lr for d in dense])))
+            self._beside(side, lambda: check(lib.vkc_colsum_update_grouped(
+                gpu._dev.h, _ptrs([dy._dptr() for dy in dys]), _ptrs([d.b.grad._dptr() for d in dense]),
+                (C.c_int64 * n)(*[dy.shape[0] for dy in dys]), (C.c_int64 * n)(*[d.output_dim for d in dense]), n, 1,
+                _ptrs([d.b.value._dptr() for d in dense]),
+                (C.c_float * n)(*[-d.b.opt_state.opt.lr for d in dense]))))
             probs = []
             upds = []
             nxt = []
@@ -176,5 +209,5 @@ class GroupedSequence:
             if l > 0:
                 for dx in nxt:
                     dx._written()
+                keep.append(nxt)
                 dys = nxt
-        return preds, losses
