@@ -211,3 +211,8 @@ def shape_arg(shape) -> "C.Array":
 
 def exported_symbols() -> list[str]:
     return sorted(_SIGS)
+
+
+from . import _hot  # noqa: E402  (linked against the library loaded above)
+
+_hot.set_check(check)

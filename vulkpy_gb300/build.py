@@ -12,6 +12,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
@@ -19,6 +20,7 @@ CSRC = HERE / "csrc"
 INCLUDE = HERE.parent / "include"
 BUILD = HERE / "_build"
 LIB = HERE / "libvulkpy_gb300.so"
+HOT = HERE / "_hot.so"        # the CPython binding of the per-operation calls
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = [
@@ -80,6 +82,17 @@ def build(verbose: bool = False, jobs: int | None = None) -> Path:
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
         os.replace(tmp, LIB)
+    src = CSRC / "hot.c"
+    if _stale(HOT, src, sorted(INCLUDE.glob("*.h"))):
+        tmp = HOT.with_suffix(".so.tmp")
+        cmd = [os.environ.get("CC", "gcc"), "-O2", "-std=c11", "-shared", "-fPIC", f"-I{sysconfig.get_paths()['include']}",
+               str(src), "-o", str(tmp), f"-L{HERE}", f"-l:{LIB.name}", "-Wl,-rpath,$ORIGIN"]
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"compiling hot.c failed:\n{r.stdout}\n{r.stderr}")
+        os.replace(tmp, HOT)
     return LIB
 
 

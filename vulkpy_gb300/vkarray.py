@@ -32,8 +32,8 @@ from typing import Iterable, List, Optional, Sequence, Tuple, Union
 import numpy as np
 
 from . import _lib
-from ._lib import lib, check, shape_arg
-from .util import debug_enabled
+from ._lib import _hot, lib, check, shape_arg
+from .util import _DEBUG, debug_enabled
 from .vktyping import KeyType, ValueType, Resource, ArrayProtocol
 
 __all__ = ["GPU", "U32Array", "Shape", "Array", "zeros", "Job"]
@@ -58,6 +58,7 @@ class _Device:
         h = C.c_void_p()
         check(lib.vkc_device_open(int(idx), float(priority), C.byref(h)))
         self.h = h
+        self.hv = h.value   # the handle as an int (per-operation calls)
         self.idx = idx
         self.seq = 0        # ops issued
         self.done = 0       # ops known to be complete
@@ -112,7 +113,7 @@ class _Device:
     # -- freeing ------------------------------------------------------------
     def release(self, ptr: int, graph) -> None:
         """Free a device buffer, stream-ordered, respecting open branches and
-        graph captures (see _DevBuf)."""
+        graph captures (see _alloc)."""
         if graph is not None and self.capture is not graph:
             return                                  # owned by its graph
         if len(self.streams) > 1:                   # a branch is open
@@ -338,7 +339,7 @@ def _host_buffer(shape, dtype) -> Tuple[np.ndarray, bool]:
     return np.empty(shape, dtype=dtype), False
 
 
-class _DevBuf:
+def _alloc(dev: _Device, nbytes: int) -> "_hot.Buf":
     """Device allocation, freed stream-ordered when garbage collected.
 
     While a graph is being captured on the device, new allocations become
@@ -346,32 +347,75 @@ class _DevBuf:
     live at the end of the capture they belong to the graph (re-made at the
     same address on every launch, released when the graph is).  Frees of
     older buffers during a capture are deferred until it ends."""
+    cap = dev.capture
+    b = _hot.alloc(dev, dev.hv, nbytes, cap)
+    if cap is not None and nbytes:
+        cap._allocated.add(b.ptr)
+    return b
 
-    __slots__ = ("dev", "ptr", "nbytes", "graph", "h2d_job")
 
-    def __init__(self, dev: _Device, nbytes: int, src: Optional[np.ndarray] = None, pinned: bool = False):
-        self.dev = dev
-        self.nbytes = nbytes
-        self.graph = dev.capture
-        self.h2d_job = None
-        p = C.c_void_p()
-        if src is not None and nbytes > 0 and pinned and self.graph is None:
-            # pinned source: queued on the copy stream, no host wait
-            j = C.c_void_p()
-            check(lib.vkc_upload_async(dev.h, src.ctypes.data, nbytes, C.byref(p), C.byref(j)))
-            self.h2d_job = j.value
-        elif src is not None and nbytes > 0:
-            check(lib.vkc_upload(dev.h, src.ctypes.data, nbytes, C.byref(p)))
-        else:
-            check(lib.vkc_alloc(dev.h, nbytes, C.byref(p)))
-        self.ptr = p.value
-        if self.graph is not None and self.ptr:
-            self.graph._allocated.add(self.ptr)
+def _upload(dev: _Device, nbytes: int, src: np.ndarray, pinned: bool) -> "_hot.Buf":
+    """A device buffer holding a copy of ``src``."""
+    if nbytes <= 0:
+        return _alloc(dev, nbytes)
+    cap = dev.capture
+    p, job = C.c_void_p(), None
+    if pinned and cap is None:
+        # pinned source: queued on the copy stream, no host wait
+        j = C.c_void_p()
+        check(lib.vkc_upload_async(dev.h, src.ctypes.data, nbytes, C.byref(p), C.byref(j)))
+        job = j.value
+    else:
+        check(lib.vkc_upload(dev.h, src.ctypes.data, nbytes, C.byref(p)))
+    if cap is not None and p.value:
+        cap._allocated.add(p.value)
+    return _hot.adopt(dev, dev.hv, p.value, nbytes, cap, job)
+
+
+class _UploadJob:
+    """A pending pinned upload: its raw job handle and the source it reads."""
+
+    __slots__ = ("j", "src")
+
+    def __init__(self, j, src):
+        self.j, self.src = j, src
+
+    def wait(self):
+        j, self.j = self.j, None
+        try:
+            check(lib.vkc_job_wait(j, -1))
+        finally:
+            lib.vkc_job_destroy(j)
 
     def __del__(self):
         try:
-            if self.ptr:
-                self.dev.release(self.ptr, self.graph)
+            if self.j is not None:
+                lib.vkc_job_destroy(self.j)
+        except Exception:  # interpreter shutdown
+            pass
+
+
+class _ReadBackJob:
+    """A pending read-back: its raw job handle and the host mirror it writes
+    (which may go back to the pinned pool only after the copy)."""
+
+    __slots__ = ("j", "host")
+
+    def __init__(self, j, host):
+        self.j, self.host = j, host
+
+    def wait(self):
+        j, self.j = self.j, None
+        try:
+            check(lib.vkc_job_wait(j, -1))
+        finally:
+            lib.vkc_job_destroy(j)
+
+    def __del__(self):
+        try:
+            if self.j is not None:
+                lib.vkc_job_wait(self.j, -1)
+                lib.vkc_job_destroy(self.j)
         except Exception:  # interpreter shutdown
             pass
 
@@ -407,52 +451,63 @@ def _prod(shape) -> int:
 class _GPUArray(Resource):
     _dtype = np.float32
 
+    # what a new array starts with; an instance holds only what differs
+    _buf: Optional["_hot.Buf"] = None
+    _job_seq: Optional[int] = None    # sequence number of the op that wrote it last
+    _host: Optional[np.ndarray] = None
+    _host_pinned = False
+    _host_valid = False
+    _dev_valid = True
+    _h2d_job: Optional[_UploadJob] = None    # pending pinned upload
+    _d2h_job: Optional[_ReadBackJob] = None  # pending read-back (prefetch)
+    _d2h_fresh = False  # no op has written the array since that read-back
+
     def __init__(self, gpu: GPU):
         self._gpu: GPU = gpu
-        self.job: Optional[Job] = None
-        self._keep: List[Resource] = []
-        self._buf: Optional[_DevBuf] = None
-        self._host: Optional[np.ndarray] = None
-        self._host_pinned = False
-        self._host_valid = False
-        self._dev_valid = True
-        self._h2d_job = None  # raw job handle of a pending pinned upload
-        self._h2d_src = None  # the pinned source that upload reads
-        self._d2h_job = None  # raw job handle of a pending read-back (prefetch)
-        self._d2h_fresh = False  # no op has written the array since that read-back
+
+    @property
+    def job(self) -> Optional[Job]:
+        """Completion marker of the op that wrote the array last, or None."""
+        seq = self._job_seq
+        return None if seq is None else Job(self._gpu._dev, seq)
+
+    @job.setter
+    def job(self, job: Optional[Job]):
+        self._job_seq = None if job is None else job.seq
+
+    @property
+    def _keep(self) -> List[Resource]:
+        return self.__dict__.setdefault("_kept", [])
+
+    @_keep.setter
+    def _keep(self, v: List[Resource]):
+        self.__dict__["_kept"] = v
+
+    def _done(self):
+        """Nothing queued writes the array any more."""
+        self._job_seq = None
+        self.__dict__.pop("_kept", None)
 
     # -- construction helpers
     def _init_storage(self, shape, data: Optional[np.ndarray]):
-        self.shape = tuple(int(s) for s in shape)
-        self._size = _prod(self.shape)
+        self.shape = shape = tuple(int(s) for s in shape)
+        self._size = _prod(shape)
         nbytes = self._size * 4  # float32 and uint32 elements
-        pinned = data is not None and _is_pinned(data)
-        self._buf = _DevBuf(self._gpu._dev, nbytes, data, pinned)
+        dev = self._gpu._dev
+        if data is None:
+            self._buf = _alloc(dev, nbytes)
+            return
+        self._buf = _upload(dev, nbytes, data, _is_pinned(data))
         if self._buf.h2d_job is not None:
-            self._h2d_job, self._h2d_src = self._buf.h2d_job, data
-
-    def __del__(self):
-        try:
-            if self._d2h_job is not None:
-                # the copy still writes into the host mirror: let it finish
-                # before the mirror can go back to the pinned pool
-                j, self._d2h_job = self._d2h_job, None
-                lib.vkc_job_wait(j, -1)
-                lib.vkc_job_destroy(j)
-            if self._h2d_job is not None:
-                lib.vkc_job_destroy(self._h2d_job)
-                self._h2d_job = None
-        except Exception:  # interpreter shutdown
-            pass
+            self._h2d_job = _UploadJob(self._buf.h2d_job, data)
 
     # -- synchronisation
     def wait(self):
         """Wait for the last op that wrote this array (vkarray.py:153-161)."""
-        if self.job is not None:
-            self.job.wait()
-            self.job = None
+        if self._job_seq is not None:
+            self._gpu._dev.wait_seq(self._job_seq)
+        self._done()
         self._wait_h2d()
-        self._keep = []
 
     def prefetch(self):
         """Start copying this array to the host now, without waiting: the copy
@@ -472,20 +527,16 @@ class _GPUArray(Resource):
             self._host = self._host.reshape(self.shape)
         j = C.c_void_p()
         check(lib.vkc_d2h_async(dev.h, self._host.ctypes.data, self._buf.ptr, self._buf.nbytes, C.byref(j)))
-        self._d2h_job = j.value
+        self._d2h_job = _ReadBackJob(j.value, self._host)
         self._d2h_fresh = True
 
     def _wait_d2h(self):
         if self._d2h_job is not None:
             j, self._d2h_job = self._d2h_job, None
-            try:
-                check(lib.vkc_job_wait(j, -1))
-            finally:
-                lib.vkc_job_destroy(j)
+            j.wait()
             if self._d2h_fresh:
                 self._host_valid = True
-                self.job = None
-                self._keep = []
+                self._done()
 
     def flush(self):
         """Upload pending host-side writes now."""
@@ -494,11 +545,7 @@ class _GPUArray(Resource):
     def _wait_h2d(self):
         if self._h2d_job is not None:
             j, self._h2d_job = self._h2d_job, None
-            try:
-                check(lib.vkc_job_wait(j, -1))
-            finally:
-                lib.vkc_job_destroy(j)
-                self._h2d_src = None
+            j.wait()
 
     def _ensure_device(self):
         """Make the device copy current (upload the host mirror if newer)."""
@@ -510,7 +557,7 @@ class _GPUArray(Resource):
         if self._host_pinned:
             j = C.c_void_p()
             check(lib.vkc_h2d(self._gpu._dev.h, self._buf.ptr, h.ctypes.data, nbytes, C.byref(j)))
-            self._h2d_job = j.value
+            self._h2d_job = _UploadJob(j.value, h)
         else:
             # pageable source: staged before the call returns
             check(lib.vkc_h2d(self._gpu._dev.h, self._buf.ptr, h.ctypes.data, nbytes, None))
@@ -534,30 +581,39 @@ class _GPUArray(Resource):
             else:
                 dev.synchronize()
             dev.done = max(dev.done, issued)
-            self.job = None
-            self._keep = []
+            self._done()
             self._host_valid = True
         return self._host
 
     def _dptr(self) -> int:
         """Device pointer for reading (uploads pending host writes first)."""
-        self._ensure_device()
+        return self._dbuf().ptr or 0
+
+    def _dbuf(self) -> "_hot.Buf":
+        """Device buffer for reading (as _dptr)."""
+        if not self._dev_valid:
+            self._ensure_device()
         cap = self._gpu._dev.capture
         if cap is not None:
             cap._touch(self, write=False)
-        return self._buf.ptr or 0
+        return self._buf
 
     def _written(self):
         """Record that an op on the stream (re)wrote this array."""
         self._dev_valid = True
         self._host_valid = False
         self._d2h_fresh = False
-        dev = self._gpu._dev
+        self._fresh(self._gpu._dev)
+
+    def _fresh(self, dev: _Device):
+        """As _written, for an array that an op has just made."""
         if dev.capture is not None:
             dev.capture._touch(self, write=True)
-            self.job = None
-            return
-        self.job = dev.issued()
+            self._job_seq = None
+        elif _DEBUG["sync"]:
+            self._job_seq = dev.issued().seq
+        else:
+            dev.seq = self._job_seq = dev.seq + 1
 
     # -- host access
     @property
@@ -603,7 +659,7 @@ class _GPUArray(Resource):
             if _is_pinned(src):
                 j = C.c_void_p()
                 check(lib.vkc_h2d(dev.h, self._buf.ptr, src.ctypes.data, self._buf.nbytes, C.byref(j)))
-                self._h2d_job, self._h2d_src = j.value, src
+                self._h2d_job = _UploadJob(j.value, src)
             else:
                 check(lib.vkc_h2d(dev.h, self._buf.ptr, src.ctypes.data, self._buf.nbytes, None))
             self._written()
@@ -737,7 +793,16 @@ class Array(_GPUArray):
         return self._gpu._dev.h
 
     def _new(self, shape) -> "Array":
-        return Array(self._gpu, shape=shape)
+        return self._make(tuple(shape), _prod(shape))
+
+    def _make(self, shape: tuple, size: int) -> "Array":
+        """A new array of ``size`` elements for an op's result."""
+        a = Array.__new__(Array)
+        a._gpu = gpu = self._gpu
+        a.shape = shape
+        a._size = size
+        a._buf = _alloc(gpu._dev, 4 * size)
+        return a
 
     def _check_shape(self, other):
         if tuple(self.shape) != tuple(other.shape):
@@ -745,35 +810,31 @@ class Array(_GPUArray):
 
     # ------------------------------------------------------------ binary ops
     def _op(self, other, op: int) -> "Array":
+        dev = self._gpu._dev
         if not isinstance(other, Array):
-            ret = self._new(self.shape)
-            check(lib.vkc_binary_scalar(self._h, op, self._dptr(), float(other), ret._buf.ptr or 0, self._size))
-            ret._written()
-            return ret
-        if tuple(self.shape) == tuple(other.shape):
-            ret = self._new(self.shape)
-            check(lib.vkc_binary(self._h, op, self._dptr(), other._dptr(), ret._buf.ptr or 0, self._size))
-            ret._written()
-            return ret
-        shape, sa, sb, sc, nd = _bcast_plan(tuple(self.shape), tuple(other.shape))
-        ret = self._new(shape)
-        check(lib.vkc_broadcast_binary(self._h, op, self._dptr(), sa, other._dptr(), sb, ret._buf.ptr or 0, sc, nd))
-        ret._written()
+            ret = self._make(tuple(self.shape), self._size)
+            _hot.binary_scalar(dev.hv, op, self._dbuf(), float(other), ret._buf, self._size)
+        elif tuple(self.shape) == tuple(other.shape):
+            ret = self._make(tuple(self.shape), self._size)
+            _hot.binary(dev.hv, op, self._dbuf(), other._dbuf(), ret._buf, self._size)
+        else:
+            shape, size, sa, sb, sc, nd, _ = _bcast_plan(tuple(self.shape), tuple(other.shape))
+            ret = self._make(shape, size)
+            _hot.broadcast_binary(dev.hv, op, self._dbuf(), sa, other._dbuf(), sb, ret._buf, sc, nd)
+        ret._fresh(dev)
         return ret
 
     def _iop(self, other, op: int) -> "Array":
+        hv = self._gpu._dev.hv
         if not isinstance(other, Array):
-            check(lib.vkc_binary_scalar(self._h, op, self._dptr(), float(other), self._buf.ptr or 0, self._size))
+            _hot.binary_scalar(hv, op, self._dbuf(), float(other), self._buf, self._size)
         elif tuple(self.shape) == tuple(other.shape):
-            check(lib.vkc_binary(self._h, op, self._dptr(), other._dptr(), self._buf.ptr or 0, self._size))
+            _hot.binary(hv, op, self._dbuf(), other._dbuf(), self._buf, self._size)
         else:
-            shape = tuple(np.broadcast_shapes(self.shape, other.shape))
+            shape, _, sa, sb, sc, nd, _ = _bcast_plan(tuple(self.shape), tuple(other.shape))
             if shape != tuple(self.shape):
                 raise ValueError(f"Incompatible shape. {shape} vs {self.shape}")
-            nd = len(shape)
-            check(lib.vkc_broadcast_binary(
-                self._h, op, self._dptr(), shape_arg(shape), other._dptr(),
-                shape_arg(_pad(other.shape, nd)), self._buf.ptr or 0, shape_arg(shape), nd))
+            _hot.broadcast_binary(hv, op, self._dbuf(), sa, other._dbuf(), sb, self._buf, sc, nd)
         self._written()
         return self
 
@@ -804,13 +865,14 @@ class Array(_GPUArray):
     # ------------------------------------------------------------ unary ops
     def _unary(self, name: str, inplace: bool) -> "Array":
         op = _lib.UNARY[name]
+        dev = self._gpu._dev
         if inplace:
-            check(lib.vkc_unary(self._h, op, self._dptr(), self._buf.ptr or 0, self._size))
+            _hot.unary(dev.hv, op, self._dbuf(), self._buf, self._size)
             self._written()
             return self
-        ret = self._new(self.shape)
-        check(lib.vkc_unary(self._h, op, self._dptr(), ret._buf.ptr or 0, self._size))
-        ret._written()
+        ret = self._make(tuple(self.shape), self._size)
+        _hot.unary(dev.hv, op, self._dbuf(), ret._buf, self._size)
+        ret._fresh(dev)
         return ret
 
     def abs(self, inplace: bool = False): return self._unary("abs", inplace)
@@ -839,6 +901,12 @@ class Array(_GPUArray):
         """Element-wise clamp (vkarray.py:1110-1191); array bounds broadcast."""
         lo_arr = isinstance(min, Array)
         hi_arr = isinstance(max, Array)
+        if not (lo_arr or hi_arr or inplace):
+            out = self._make(tuple(self.shape), self._size)
+            dev = self._gpu._dev
+            _hot.clamp(dev.hv, self._dbuf(), None, None, float(min), float(max), out._buf, self._size)
+            out._fresh(dev)
+            return out
         shapes = [tuple(self.shape)]
         if lo_arr:
             shapes.append(tuple(min.shape))
@@ -879,14 +947,16 @@ class Array(_GPUArray):
         N = _prod(other.shape[1:])
         ret = self._new(shape)
         prec = _MATMUL_PRECISION[self._gpu.matmul_precision]
-        check(lib.vkc_matmul(self._h, prec, self._dptr(), other._dptr(), ret._buf.ptr or 0, M, K, N))
-        ret._written()
+        dev = self._gpu._dev
+        _hot.matmul(dev.hv, prec, self._dbuf(), other._dbuf(), ret._buf, M, K, N)
+        ret._fresh(dev)
         return ret
 
     # ------------------------------------------------------------ reductions
     def _reduce(self, op: int, axis, keepdims: bool, rebroadcast: bool, scale: float = 1.0) -> "Array":
         if self._size == 0:
             raise ValueError("reduction of an empty array")
+        dev = self._gpu._dev
         if rebroadcast:
             if not isinstance(axis, (int, np.integer)):
                 raise ValueError("When `rebroadcast` is specified, `axis` must be `int`")
@@ -895,14 +965,13 @@ class Array(_GPUArray):
             n = int(self.shape[a])
             post = _prod(self.shape[a + 1:])
             ret = self._new(self.shape)
-            check(lib.vkc_reduce_axis(self._h, op, self._dptr(), prev, n, post, ret._buf.ptr or 0, 1, scale))
-            ret._written()
+            _hot.reduce_axis(dev.hv, op, self._dbuf(), prev, n, post, ret._buf, 1, scale)
+            ret._fresh(dev)
             return ret
         if axis is None:
             ret = self._new((1,))
-            check(lib.vkc_reduce_all(self._h, op, self._gpu.reduce_precision, self._dptr(), self._size,
-                                     ret._buf.ptr or 0, scale))
-            ret._written()
+            _hot.reduce_all(dev.hv, op, self._gpu.reduce_precision, self._dbuf(), self._size, ret._buf, scale)
+            ret._fresh(dev)
             if keepdims:
                 ret.reshape((1,) * len(self.shape))
             return ret
@@ -923,8 +992,8 @@ class Array(_GPUArray):
             new_shape = shape[:first] + shape[last + 1:]
             ret = self._new(tuple(new_shape))
             s = scale if i == len(runs) - 1 else 1.0
-            check(lib.vkc_reduce_axis(self._h, op, tmp._dptr(), prev, n, post, ret._buf.ptr or 0, 0, s))
-            ret._written()
+            _hot.reduce_axis(dev.hv, op, tmp._dbuf(), prev, n, post, ret._buf, 0, s)
+            ret._fresh(dev)
             tmp = ret
             shape = new_shape
         if keepdims:
@@ -955,7 +1024,7 @@ class Array(_GPUArray):
             raise ValueError("attempt to get argmax/argmin of an empty sequence")
         if axis is None:
             ret = U32Array(self._gpu, shape=(1,))
-            check(lib.vkc_arg_reduce_all(self._h, op, self._dptr(), self._size, ret._buf.ptr or 0))
+            _hot.arg_reduce_all(self._gpu._dev.hv, op, self._dbuf(), self._size, ret._buf)
             ret._written()
             if keepdims:
                 ret.reshape((1,) * len(self.shape))
@@ -967,8 +1036,8 @@ class Array(_GPUArray):
         new_shape = shape[:a] + ([1] if keepdims else []) + shape[a + 1:]
         ret = U32Array(self._gpu, shape=tuple(new_shape))
         if ret._size:
-            check(lib.vkc_arg_reduce_axis(self._h, op, self._dptr(), _prod(shape[:a]), int(shape[a]),
-                                          _prod(shape[a + 1:]), ret._buf.ptr or 0))
+            _hot.arg_reduce_axis(self._gpu._dev.hv, op, self._dbuf(), _prod(shape[:a]), int(shape[a]),
+                                 _prod(shape[a + 1:]), ret._buf)
             ret._written()
         return ret
 
@@ -1022,14 +1091,14 @@ class Array(_GPUArray):
         n_idx = indices._size
         if axis is None:
             ret = self._new(indices.shape)
-            check(lib.vkc_gather(self._h, self._dptr(), self._size, indices._dptr(), n_idx, ret._buf.ptr or 0))
+            _hot.gather(self._gpu._dev.hv, self._dbuf(), self._size, indices._dbuf(), n_idx, ret._buf)
         else:
             a = _normalize_axes(axis, len(self.shape))[0]
             prev_shape = tuple(self.shape[:a])
             post_shape = tuple(self.shape[a + 1:])
             ret = self._new(tuple(indices.shape) + prev_shape + post_shape)
-            check(lib.vkc_gather_axis(self._h, self._dptr(), _prod(prev_shape), int(self.shape[a]),
-                                      _prod(post_shape), indices._dptr(), n_idx, ret._buf.ptr or 0))
+            _hot.gather_axis(self._gpu._dev.hv, self._dbuf(), _prod(prev_shape), int(self.shape[a]),
+                             _prod(post_shape), indices._dbuf(), n_idx, ret._buf)
         ret._written()
         return ret
 
@@ -1085,12 +1154,13 @@ def matmul_grouped(a_list: Sequence["Array"], b_list: Sequence["Array"], precisi
 
 @functools.lru_cache(maxsize=256)
 def _bcast_plan(a_shape: tuple, b_shape: tuple):
-    """Result shape and the C shape arguments of a broadcast binary op (the
-    ctypes arrays are read-only for the library, so one set per pair of
-    shapes serves every call)."""
+    """Result shape and size of a broadcast binary op, and the addresses of its
+    C shape arguments (the ctypes arrays, last, are read-only for the
+    library, so one set per pair of shapes serves every call)."""
     shape = tuple(int(v) for v in np.broadcast_shapes(a_shape, b_shape))
     nd = len(shape)
-    return shape, shape_arg(_pad(a_shape, nd)), shape_arg(_pad(b_shape, nd)), shape_arg(shape), nd
+    keep = (shape_arg(_pad(a_shape, nd)), shape_arg(_pad(b_shape, nd)), shape_arg(shape))
+    return (shape, _prod(shape)) + tuple(C.addressof(k) for k in keep) + (nd, keep)
 
 
 def _pad(shape, nd) -> tuple:
