@@ -32,7 +32,9 @@ int gemm_tc(vkc_device_t dev, int precision, bool ta, bool tb, int64_t M, int64_
 // 64 10.9 -> 9.4, 128^3 17.5 -> 10.4, 300^3 (19 ranges of 16) 12.6 -> 11.2,
 // 256^3 (16 ranges of 16) 9.3 -> 10.9, 1024 x 1024 x 48 9.2 -> 9.6, 4096 x
 // 4096 x 16 30.6 -> 27.9.  Run call by call the third launch costs another 1.5
-// us of host time, hence 96 steps rather than 64.
+// us of host time, hence 96 steps rather than 64.  Unsplit products up to K =
+// 256 whose small tiles fit the GPU at once go to k_gemm_small all the same
+// (128^3 4.0 us).
 inline bool fp32_on_tensor_cores(int64_t M, int64_t N, int64_t K, int splits) {
   if (M < 2 || N < 2 || K < 16) return false;                            // vectors are bound by reading the matrix
   if (M > (1 << 22) || N > (1 << 22) || K >= (1ll << 31)) return false;  // 32-bit tile and row coordinates
