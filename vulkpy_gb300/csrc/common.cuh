@@ -103,6 +103,23 @@ inline unsigned wave_grid(const vkc_device* dev, K* kernel, size_t work_items, i
   return (unsigned)(want < cap ? want : cap);
 }
 
+// Loads kernels on the device (once; `done` has a bit per device).  A kernel is
+// otherwise loaded at its first launch, and the host then waits for the work
+// running before it: a call of several launches loads all of them first, so
+// that its first run is asynchronous too.
+template <class... K>
+inline void load_kernels(vkc_device_t dev, std::atomic<uint64_t>& done, K*... kernels) {
+  const uint64_t bit = uint64_t(1) << (dev->index & 63);
+  if (done.load(std::memory_order_acquire) & bit) return;
+  cudaFuncAttributes at;
+  const bool ok = ((cudaFuncGetAttributes(&at, (const void*)kernels) == cudaSuccess) && ...);
+  if (!ok) {
+    cudaGetLastError();  // the launch will say what is wrong
+    return;
+  }
+  done.fetch_or(bit, std::memory_order_release);
+}
+
 // Stream-ordered scratch allocation on the device's current stream.
 int scratch_alloc(vkc_device_t dev, size_t bytes, void** p);
 void scratch_free(vkc_device_t dev, void* p);

@@ -1248,6 +1248,12 @@ int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t 
     clear_error();
     return simt();
   }
+  {
+    static std::atomic<uint64_t> loaded{0};
+    load_kernels(dev, loaded, k_split_pair<3>, k_gemm_tcp<3, 128, 2, 1>, k_gemm_tcp<3, 128, 2, 2>,
+                 k_splitk_reduce4<true>, k_splitk_reduce<true>, k_gemm_repair<false, false>, k_gemm_repair<false, true>,
+                 k_gemm_repair<true, false>, k_gemm_repair<true, true>);
+  }
   auto* a = static_cast<__nv_bfloat16*>(scratch);
   auto* b = a + 3 * (size_t)M * Kp;
   auto* repair = reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + list);

@@ -1051,6 +1051,10 @@ int grouped_tc(vkc_device_t dev, const vkc_gemm_problem* probs, const vkc_gemm_u
       if (r == VKC_OK) continue;
     }
     if (r != VKC_OK) return r;
+    if (PARTS == 3) {
+      static std::atomic<uint64_t> loaded{0};
+      load_kernels(dev, loaded, k_tile_operands<true>, k_gemm_tc_grouped<3>, k_gemm_repair_grouped);
+    }
     uint8_t* sbase = static_cast<uint8_t*>(scratch);
     uint32_t* repair = PARTS == 3 ? reinterpret_cast<uint32_t*>(sbase + list) : nullptr;
     SimtTable rt{};  // PARTS == 3: the problems as the repair kernel needs them
