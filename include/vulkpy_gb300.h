@@ -197,11 +197,13 @@ int vkc_set_cluster_splitk(int enable);
  * vkc_side_defer(dev, 0) joins them all back into the device's stream (the
  * gradients are complete on it from then on).  A training step defers
  * across its backward pass, so the weight GEMMs of every layer overlap the
- * chain of input-gradient GEMMs.  No reference counterpart. */
+ * chain of input-gradient GEMMs.  Holds for the calling thread's calls.  No
+ * reference counterpart. */
 int vkc_side_defer(vkc_device_t dev, int defer);
-/* Work on the side branch: after vkc_side_begin(dev) the device's calls go
- * to the side stream, which first waits for everything issued so far on the
- * device's stream and on the bias-sum branch; vkc_side_end(dev) returns to
+/* Work on the side branch: after vkc_side_begin(dev) the calling thread's
+ * calls go to the side stream, which first waits for everything issued so far
+ * on the device's stream and on the bias-sum branch (other threads' calls go
+ * on to the device's stream); vkc_side_end(dev), by the same thread, returns to
  * the device's stream and joins the branch back (or, under vkc_side_defer,
  * leaves it for that join).  Sequence.train runs each layer's optimizer
  * step there as soon as the layer's gradients are issued.  Only from the

@@ -17,12 +17,50 @@
 
 #define VKC_EXPORT extern "C" __attribute__((visibility("default")))
 
+namespace vkc {
+// Whether this thread's calls go to a branch of a device (BranchScope,
+// vkc_side_begin) and whether it defers the joins (vkc_side_defer).
+struct ThreadBranch {
+  const void* of = nullptr;        // the device's CurrentStream
+  cudaStream_t stream = nullptr;
+  const void* deferred = nullptr;  // the device whose joins wait
+};
+inline thread_local ThreadBranch t_branch;
+
+// The stream that calls on a device go to: the shared one (the device's own
+// or the user's), or while this thread works on a branch, the branch's.  A
+// branch is the thread's and not the device's: the interpreter runs other
+// threads in the middle of a training step, and what they queue must not
+// land on the step's branch, which their later calls are not ordered after.
+struct CurrentStream {
+  cudaStream_t shared = nullptr;
+  operator cudaStream_t() const { return t_branch.of == this ? t_branch.stream : shared; }
+};
+
+class BranchScope {
+ public:
+  BranchScope(const CurrentStream& current, cudaStream_t stream) : before_(t_branch) {
+    t_branch.of = &current;
+    t_branch.stream = stream;
+  }
+  ~BranchScope() {
+    t_branch.of = before_.of;
+    t_branch.stream = before_.stream;
+  }
+  BranchScope(const BranchScope&) = delete;
+  BranchScope& operator=(const BranchScope&) = delete;
+
+ private:
+  ThreadBranch before_;
+};
+}  // namespace vkc
+
 struct vkc_device {
   int index = 0;
   int sm_count = 0;
   int cc_major = 0, cc_minor = 0;
   cudaStream_t own_stream = nullptr;   // compute stream created at open
-  cudaStream_t stream = nullptr;       // current compute stream (own or user's)
+  vkc::CurrentStream stream;           // current compute stream (own, user's or this thread's branch)
   cudaStream_t copy_stream = nullptr;  // uploads into fresh buffers
   cudaMemPool_t upload_pool = nullptr; // their buffers (reused only by later uploads)
   // Upload buffers the caller freed, each with an event on the compute stream
@@ -41,8 +79,7 @@ struct vkc_device {
   cudaStream_t side_stream = nullptr;  // independent work forked from `stream` inside one call
   cudaStream_t bias_stream = nullptr;  // a second such branch (the Dense backward's bias sums)
   cudaEvent_t side_fork = nullptr, side_join = nullptr, bias_join = nullptr;
-  int side_defer = 0;    // vkc_side_defer: leave the branches open until vkc_side_defer(dev, 0)
-  int side_pending = 0;  // branches forked and not yet joined back
+  std::atomic<int> side_pending{0};    // branches forked and not yet joined back
   uint32_t* err_word = nullptr;        // device error flags (bit0: gather index)
   uint32_t* done_ctr = nullptr;        // arrival counter of last-block reductions (zero between kernels)
   uint32_t* xo_jump_pows = nullptr;    // xoshiro jump-map powers (lazy)

@@ -125,13 +125,16 @@ int dense_backward_gemms(vkc_device_t dev, int precision, const float* x, const 
     VKC_CUDA(cudaStreamWaitEvent(dev->bias_stream, dev->side_fork, 0));
     // bias stream: the bias sum; side stream: the weight GEMM when dx is
     // wanted; main: dx, or the weight GEMM (the first layer has no dx)
-    dev->stream = dev->bias_stream;
-    int r = colsum_into(dev, dy, db, batch, out_dim, overwrite);
-    dev->stream = dev->side_stream;
-    if (r == VKC_OK && dx)
+    int r;
+    {
+      vkc::BranchScope branch(dev->stream, dev->bias_stream);
+      r = colsum_into(dev, dy, db, batch, out_dim, overwrite);
+    }
+    if (r == VKC_OK && dx) {
+      vkc::BranchScope branch(dev->stream, dev->side_stream);
       r = gemm_any(dev, precision, true, false, out_dim, in_dim, batch, 1.0f, dy, out_dim, x, in_dim, wbeta, dw,
                    in_dim, vkc::GemmEpilogue{});
-    dev->stream = main;
+    }
     if (r == VKC_OK && dx)
       r = gemm_any(dev, precision, false, false, batch, in_dim, out_dim, 1.0f, dy, out_dim, w, in_dim, 0.0f, dx,
                    in_dim, dx_epi);
@@ -142,7 +145,7 @@ int dense_backward_gemms(vkc_device_t dev, int precision, const float* x, const 
     // so the branches of several layers overlap the input-gradient chain; the
     // join is recorded even after an error, so a capture stays joined
     dev->side_pending = 1;
-    if (!dev->side_defer) {
+    if (vkc::t_branch.deferred != dev) {
       const int rj = vkc_side_defer(dev, 0);
       if (r == VKC_OK) r = rj;
     }
@@ -542,16 +545,16 @@ VKC_EXPORT int vkc_dense_stack_forward(vkc_device_t dev, int precision, int laye
   if (fork) {
     VKC_CUDA(cudaEventRecord(dev->side_fork, main));
     VKC_CUDA(cudaStreamWaitEvent(dev->side_stream, dev->side_fork, 0));
-    dev->stream = dev->side_stream;
   }
-  for (int l = 1; l < layers && r == VKC_OK; ++l)
-    r = vkc::tc_split_operands(dev, w[l], dims[l + 1], dims[l], true, w_hi[(size_t)l], w_lo[(size_t)l], nullptr, 0, 0,
-                               true, nullptr, nullptr, dims[l], kp[(size_t)l]);
+  {
+    vkc::BranchScope branch(dev->stream, fork ? dev->side_stream : main);
+    for (int l = 1; l < layers && r == VKC_OK; ++l)
+      r = vkc::tc_split_operands(dev, w[l], dims[l + 1], dims[l], true, w_hi[(size_t)l], w_lo[(size_t)l], nullptr, 0, 0,
+                                 true, nullptr, nullptr, dims[l], kp[(size_t)l]);
+  }
   cudaError_t ej = cudaSuccess;
-  if (fork) {
-    dev->stream = main;
+  if (fork)
     ej = cudaEventRecord(dev->side_join, dev->side_stream);  // recorded even after an error: a capture stays joined
-  }
   if (r == VKC_OK)
     r = vkc::tc_split_operands(dev, x, batch, dims[0], true, a_hi[0], a_lo[0], w[0], dims[1], dims[0], true, w_hi[0],
                                w_lo[0], dims[0], kp[0]);

@@ -172,7 +172,7 @@ VKC_EXPORT int vkc_device_open(int index, float priority, vkc_device_t* out) {
     delete dev;
     return set_error(VKC_ERR_CUDA, "device setup: %s", cudaGetErrorString(e));
   }
-  dev->stream = dev->own_stream;
+  dev->stream.shared = dev->own_stream;
 
   // Keep freed blocks cached in the pool instead of returning them to the OS:
   // arrays are short-lived and large (up to GiBs), re-mapping is expensive.
@@ -261,7 +261,7 @@ VKC_EXPORT int vkc_device_stream(vkc_device_t dev, void** stream) {
 
 VKC_EXPORT int vkc_device_set_stream(vkc_device_t dev, void* stream) {
   VKC_REQUIRE(dev, "device handle is NULL");
-  dev->stream = stream ? (cudaStream_t)stream : dev->own_stream;
+  dev->stream.shared = stream ? (cudaStream_t)stream : dev->own_stream;
   return VKC_OK;
 }
 
@@ -590,16 +590,21 @@ VKC_EXPORT int vkc_set_pdl(int enable) {
 VKC_EXPORT int vkc_side_defer(vkc_device_t dev, int defer) {
   VKC_BIND(dev);
   if (defer) {
-    dev->side_defer = 1;
+    vkc::t_branch.deferred = dev;
     return VKC_OK;
   }
-  dev->side_defer = 0;
-  if (!dev->side_pending) return VKC_OK;
-  dev->side_pending = 0;
+  if (vkc::t_branch.deferred == dev) vkc::t_branch.deferred = nullptr;
+  if (!dev->side_pending.exchange(0)) return VKC_OK;
   VKC_CUDA(cudaEventRecord(dev->side_join, dev->side_stream));
   VKC_CUDA(cudaEventRecord(dev->bias_join, dev->bias_stream));
-  VKC_CUDA(cudaStreamWaitEvent(dev->stream, dev->side_join, 0));
-  VKC_CUDA(cudaStreamWaitEvent(dev->stream, dev->bias_join, 0));
+  // branches fork from the device's own stream only; the caller's calls may
+  // have moved to another one since
+  const cudaStream_t current = dev->stream;
+  for (cudaStream_t s : {dev->own_stream, current}) {
+    VKC_CUDA(cudaStreamWaitEvent(s, dev->side_join, 0));
+    VKC_CUDA(cudaStreamWaitEvent(s, dev->bias_join, 0));
+    if (s == current) break;
+  }
   return VKC_OK;
 }
 
@@ -612,7 +617,8 @@ VKC_EXPORT int vkc_side_begin(vkc_device_t dev) {
   if (!dev->side_pending) VKC_CUDA(cudaStreamWaitEvent(dev->bias_stream, dev->side_fork, 0));
   VKC_CUDA(cudaEventRecord(dev->bias_join, dev->bias_stream));
   VKC_CUDA(cudaStreamWaitEvent(dev->side_stream, dev->bias_join, 0));
-  dev->stream = dev->side_stream;
+  vkc::t_branch.of = &dev->stream;
+  vkc::t_branch.stream = dev->side_stream;
   dev->side_pending = 1;
   return VKC_OK;
 }
@@ -620,8 +626,9 @@ VKC_EXPORT int vkc_side_begin(vkc_device_t dev) {
 VKC_EXPORT int vkc_side_end(vkc_device_t dev) {
   VKC_BIND(dev);
   VKC_REQUIRE(dev->stream == dev->side_stream, "branch: vkc_side_end without vkc_side_begin");
-  dev->stream = dev->own_stream;
-  if (!dev->side_defer) return vkc_side_defer(dev, 0);
+  vkc::t_branch.of = nullptr;
+  dev->side_pending = 1;  // again: another thread's join may have come between
+  if (vkc::t_branch.deferred != dev) return vkc_side_defer(dev, 0);
   return VKC_OK;
 }
 
