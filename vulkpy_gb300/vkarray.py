@@ -59,6 +59,9 @@ class _Device:
         check(lib.vkc_device_open(int(idx), float(priority), C.byref(h)))
         self.h = h
         self.hv = h.value   # the handle as an int (per-operation calls)
+        s = C.c_void_p()
+        check(lib.vkc_device_stream(h, C.byref(s)))
+        self._own = s.value  # the device's own stream
         self.idx = idx
         self.seq = 0        # ops issued
         self.done = 0       # ops known to be complete
@@ -141,8 +144,13 @@ class _Device:
 
     # -- branches -----------------------------------------------------------
     def own_stream(self) -> bool:
-        """True when work goes to the device's own stream (no branch open)."""
-        return len(self.streams) == 1
+        """True when work goes to the device's own stream: no branch is open,
+        and the caller has set no other stream (vkc_device_set_stream)."""
+        if len(self.streams) != 1:
+            return False
+        s = C.c_void_p()
+        check(lib.vkc_device_stream(self.h, C.byref(s)))
+        return s.value == self._own
 
     def branch_enter(self):
         parent = self.streams[-1]
