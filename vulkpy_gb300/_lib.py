@@ -213,6 +213,7 @@ def exported_symbols() -> list[str]:
     return sorted(_SIGS)
 
 
-from . import _hot  # noqa: E402  (linked against the library loaded above)
+from . import _hot  # noqa: E402
 
-_hot.set_check(check)
+# the per-operation calls go to the library loaded above, whichever file it is
+_hot.bind(lambda name: C.cast(getattr(lib, name), C.c_void_p).value, check)

@@ -86,7 +86,7 @@ def build(verbose: bool = False, jobs: int | None = None) -> Path:
     if _stale(HOT, src, sorted(INCLUDE.glob("*.h"))):
         tmp = HOT.with_suffix(".so.tmp")
         cmd = [os.environ.get("CC", "gcc"), "-O2", "-std=c11", "-shared", "-fPIC", f"-I{sysconfig.get_paths()['include']}",
-               str(src), "-o", str(tmp), f"-L{HERE}", f"-l:{LIB.name}", "-Wl,-rpath,$ORIGIN"]
+               str(src), "-o", str(tmp)]
         if verbose:
             print(" ".join(cmd), flush=True)
         r = subprocess.run(cmd, capture_output=True, text=True)

@@ -4,20 +4,37 @@
  * calls around 2 us of launch.  Each function takes the arguments of the
  * vkc_ function of its name, device handle first (an int); device pointers are
  * Buf objects, ints or None.  A status other than VKC_OK raises through the
- * Python function given to set_check.  The interpreter lock is released
- * around every library call, as ctypes does. */
+ * Python function given to bind.  The interpreter lock is released around
+ * every library call, as ctypes does.
+ *
+ * The module is not linked with the library: bind takes the functions'
+ * addresses from the one that ctypes has loaded (VULKPY_GB300_LIB may name
+ * another file than the one beside this module), so a process has one copy
+ * of the library's state. */
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <structmember.h>
 
 #include "../../include/vulkpy_gb300.h"
 
-static PyObject* g_check = NULL; /* check(status): raises */
+/* The functions of the library that are called here. */
+#define FUNCTIONS(X)                                                                                              \
+  X(alloc) X(free) X(unary) X(binary) X(binary_scalar) X(broadcast_binary) X(clamp) X(reduce_all) X(reduce_axis) \
+  X(arg_reduce_all) X(arg_reduce_axis) X(gather) X(gather_axis) X(matmul)
+static struct {
+#define X(name) __typeof__(&vkc_##name) name;
+  FUNCTIONS(X)
+#undef X
+} lib;
+
+static PyObject* g_check = NULL; /* check(status): raises; NULL until bind */
 static PyObject *g_capture, *g_streams, *g_release;
+
+static PyObject* unbound(void) { return PyErr_Format(PyExc_RuntimeError, "no library bound"); }
 
 static PyObject* finish(int st) {
   if (st == VKC_OK) Py_RETURN_NONE;
-  PyObject* r = g_check ? PyObject_CallFunction(g_check, "i", st) : NULL;
+  PyObject* r = PyObject_CallFunction(g_check, "i", st);
   if (r) {
     Py_DECREF(r);
     PyErr_Format(PyExc_RuntimeError, "library status %d", st);
@@ -56,6 +73,7 @@ static Buf* buf_alloc(PyObject* dev, void* h, Py_ssize_t nbytes, PyObject* graph
 /* alloc(dev, handle, nbytes, graph) -> Buf on the device's current stream */
 static PyObject* hot_alloc(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   if (n != 4) return PyErr_Format(PyExc_TypeError, "alloc takes 4 arguments");
+  if (!g_check) return unbound();
   void* h = PyLong_AsVoidPtr(a[1]);
   const Py_ssize_t nbytes = PyLong_AsSsize_t(a[2]);
   if (PyErr_Occurred()) return NULL;
@@ -65,7 +83,7 @@ static PyObject* hot_alloc(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   int st;
   void* p = NULL;
   Py_BEGIN_ALLOW_THREADS
-  st = vkc_alloc((vkc_device_t)h, (size_t)nbytes, &p);
+  st = lib.alloc((vkc_device_t)h, (size_t)nbytes, &p);
   Py_END_ALLOW_THREADS
   if (st != VKC_OK) {
     Py_DECREF(b);
@@ -78,6 +96,7 @@ static PyObject* hot_alloc(PyObject* self, PyObject* const* a, Py_ssize_t n) {
 /* adopt(dev, handle, ptr, nbytes, graph, h2d_job) -> Buf owning ptr */
 static PyObject* hot_adopt(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   if (n != 6) return PyErr_Format(PyExc_TypeError, "adopt takes 6 arguments");
+  if (!g_check) return unbound();
   void* h = PyLong_AsVoidPtr(a[1]);
   void* p = a[2] == Py_None ? NULL : PyLong_AsVoidPtr(a[2]);
   const Py_ssize_t nbytes = PyLong_AsSsize_t(a[3]);
@@ -114,7 +133,7 @@ static void buf_release(Buf* b) {
   }
   if (plain) {
     Py_BEGIN_ALLOW_THREADS
-    vkc_free((vkc_device_t)b->h, p);
+    lib.free((vkc_device_t)b->h, p);
     Py_END_ALLOW_THREADS
   } else {
     PyErr_Clear();
@@ -186,6 +205,7 @@ static void* ptr_of(PyObject* o) {
 #define HOT(name, count, decl, call)                                              \
   static PyObject* hot_##name(PyObject* self, PyObject* const* a, Py_ssize_t n) { \
     if (n != count) return PyErr_Format(PyExc_TypeError, #name " takes %d arguments", count); \
+    if (!g_check) return unbound();                                               \
     vkc_device_t dev = DEV;                                                       \
     decl;                                                                         \
     if (PyErr_Occurred()) return NULL;                                            \
@@ -196,33 +216,48 @@ static void* ptr_of(PyObject* o) {
     return finish(st);                                                            \
   }
 
-HOT(unary, 5, int op = INT(1); void* x = PTR(2); void* y = PTR(3); size_t m = SIZE(4), vkc_unary(dev, op, x, y, m))
+HOT(unary, 5, int op = INT(1); void* x = PTR(2); void* y = PTR(3); size_t m = SIZE(4), lib.unary(dev, op, x, y, m))
 HOT(binary, 6, int op = INT(1); void* x = PTR(2); void* y = PTR(3); void* z = PTR(4); size_t m = SIZE(5),
-    vkc_binary(dev, op, x, y, z, m))
+    lib.binary(dev, op, x, y, z, m))
 HOT(binary_scalar, 6, int op = INT(1); void* x = PTR(2); float s = FLT(3); void* z = PTR(4); size_t m = SIZE(5),
-    vkc_binary_scalar(dev, op, x, s, z, m))
+    lib.binary_scalar(dev, op, x, s, z, m))
 HOT(broadcast_binary, 9,
     int op = INT(1); void* x = PTR(2); void* sx = PTR(3); void* y = PTR(4); void* sy = PTR(5); void* z = PTR(6);
-    void* sz = PTR(7); int nd = INT(8), vkc_broadcast_binary(dev, op, x, sx, y, sy, z, sz, nd))
+    void* sz = PTR(7); int nd = INT(8), lib.broadcast_binary(dev, op, x, sx, y, sy, z, sz, nd))
 HOT(clamp, 8, void* x = PTR(1); void* lo = PTR(2); void* hi = PTR(3); float l = FLT(4); float u = FLT(5);
-    void* z = PTR(6); size_t m = SIZE(7), vkc_clamp(dev, x, lo, hi, l, u, z, m))
+    void* z = PTR(6); size_t m = SIZE(7), lib.clamp(dev, x, lo, hi, l, u, z, m))
 HOT(reduce_all, 7, int op = INT(1); int prec = INT(2); void* x = PTR(3); size_t m = SIZE(4); void* z = PTR(5);
-    float s = FLT(6), vkc_reduce_all(dev, op, prec, x, m, z, s))
+    float s = FLT(6), lib.reduce_all(dev, op, prec, x, m, z, s))
 HOT(reduce_axis, 9, int op = INT(1); void* x = PTR(2); size_t p = SIZE(3); size_t m = SIZE(4); size_t q = SIZE(5);
-    void* z = PTR(6); int re = INT(7); float s = FLT(8), vkc_reduce_axis(dev, op, x, p, m, q, z, re, s))
+    void* z = PTR(6); int re = INT(7); float s = FLT(8), lib.reduce_axis(dev, op, x, p, m, q, z, re, s))
 HOT(arg_reduce_all, 5, int op = INT(1); void* x = PTR(2); size_t m = SIZE(3); void* z = PTR(4),
-    vkc_arg_reduce_all(dev, op, x, m, z))
+    lib.arg_reduce_all(dev, op, x, m, z))
 HOT(arg_reduce_axis, 7, int op = INT(1); void* x = PTR(2); size_t p = SIZE(3); size_t m = SIZE(4);
-    size_t q = SIZE(5); void* z = PTR(6), vkc_arg_reduce_axis(dev, op, x, p, m, q, z))
+    size_t q = SIZE(5); void* z = PTR(6), lib.arg_reduce_axis(dev, op, x, p, m, q, z))
 HOT(gather, 6, void* x = PTR(1); size_t m = SIZE(2); void* i = PTR(3); size_t k = SIZE(4); void* z = PTR(5),
-    vkc_gather(dev, x, m, i, k, z))
+    lib.gather(dev, x, m, i, k, z))
 HOT(gather_axis, 8, void* x = PTR(1); size_t p = SIZE(2); size_t m = SIZE(3); size_t q = SIZE(4); void* i = PTR(5);
-    size_t k = SIZE(6); void* z = PTR(7), vkc_gather_axis(dev, x, p, m, q, i, k, z))
+    size_t k = SIZE(6); void* z = PTR(7), lib.gather_axis(dev, x, p, m, q, i, k, z))
 HOT(matmul, 8, int prec = INT(1); void* x = PTR(2); void* y = PTR(3); void* z = PTR(4); int64_t m = I64(5);
-    int64_t k = I64(6); int64_t q = I64(7), vkc_matmul(dev, prec, x, y, z, m, k, q))
+    int64_t k = I64(6); int64_t q = I64(7), lib.matmul(dev, prec, x, y, z, m, k, q))
 
-static PyObject* hot_set_check(PyObject* self, PyObject* f) {
-  Py_XSETREF(g_check, Py_NewRef(f));
+/* bind(address, check): address(name) is that of the library's vkc_<name> */
+static PyObject* hot_bind(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+  if (n != 2) return PyErr_Format(PyExc_TypeError, "bind takes 2 arguments");
+  __typeof__(lib) l;
+#define X(name)                                                  \
+  {                                                              \
+    PyObject* r = PyObject_CallFunction(a[0], "s", "vkc_" #name); \
+    void* p = r ? PyLong_AsVoidPtr(r) : NULL;                    \
+    Py_XDECREF(r);                                               \
+    if (PyErr_Occurred()) return NULL;                           \
+    if (!p) return PyErr_Format(PyExc_ValueError, "vkc_" #name " is NULL"); \
+    l.name = (__typeof__(l.name))p;                              \
+  }
+  FUNCTIONS(X)
+#undef X
+  lib = l;
+  Py_XSETREF(g_check, Py_NewRef(a[1]));
   Py_RETURN_NONE;
 }
 
@@ -230,7 +265,7 @@ static PyObject* hot_set_check(PyObject* self, PyObject* f) {
 static PyMethodDef methods[] = {M(alloc), M(adopt), M(unary), M(binary), M(binary_scalar), M(broadcast_binary),
                                 M(clamp), M(reduce_all), M(reduce_axis), M(arg_reduce_all), M(arg_reduce_axis),
                                 M(gather), M(gather_axis), M(matmul),
-                                {"set_check", hot_set_check, METH_O, NULL},
+                                M(bind),
                                 {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_hot", "Binding of the per-operation calls.", -1, methods};
 
