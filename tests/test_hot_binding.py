@@ -23,3 +23,12 @@ def test_one_copy_of_the_library(tmp_path):
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
     assert r.stdout.split() == [str(other)]
+
+
+def test_binding_is_named_for_the_interpreter():
+    """An interpreter with another ABI must not load it."""
+    import sysconfig
+    _lib = pytest.importorskip("vulkpy_gb300._lib")
+    name = os.path.basename(_lib._hot.__file__)
+    assert name == "_hot" + sysconfig.get_config_var("EXT_SUFFIX") != "_hot.so"
+    assert not os.path.exists(os.path.join(os.path.dirname(_lib._hot.__file__), "_hot.so"))

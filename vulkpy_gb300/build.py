@@ -20,7 +20,9 @@ CSRC = HERE / "csrc"
 INCLUDE = HERE.parent / "include"
 BUILD = HERE / "_build"
 LIB = HERE / "libvulkpy_gb300.so"
-HOT = HERE / "_hot.so"        # the CPython binding of the per-operation calls
+# the CPython binding of the per-operation calls, named for the interpreter it
+# is compiled for (another one does not load it)
+HOT = HERE / ("_hot" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = [
@@ -82,6 +84,7 @@ def build(verbose: bool = False, jobs: int | None = None) -> Path:
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
         os.replace(tmp, LIB)
+    (HERE / "_hot.so").unlink(missing_ok=True)  # any interpreter would load it
     src = CSRC / "hot.c"
     if _stale(HOT, src, sorted(INCLUDE.glob("*.h"))):
         tmp = HOT.with_suffix(".so.tmp")
