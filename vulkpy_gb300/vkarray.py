@@ -404,13 +404,15 @@ class _UploadJob:
 
 
 class _ReadBackJob:
-    """A pending read-back: its raw job handle and the host mirror it writes
-    (which may go back to the pinned pool only after the copy)."""
+    """A pending read-back: its raw job handle, the device buffer it reads and
+    the host mirror it writes.  The copy runs on a stream of its own, so both
+    are kept until it is done: the buffer freed on the compute stream before
+    could be handed to the next allocation."""
 
-    __slots__ = ("j", "host")
+    __slots__ = ("j", "buf", "host")
 
-    def __init__(self, j, host):
-        self.j, self.host = j, host
+    def __init__(self, j, buf, host):
+        self.j, self.buf, self.host = j, buf, host
 
     def wait(self):
         j, self.j = self.j, None
@@ -535,7 +537,7 @@ class _GPUArray(Resource):
             self._host = self._host.reshape(self.shape)
         j = C.c_void_p()
         check(lib.vkc_d2h_async(dev.h, self._host.ctypes.data, self._buf.ptr, self._buf.nbytes, C.byref(j)))
-        self._d2h_job = _ReadBackJob(j.value, self._host)
+        self._d2h_job = _ReadBackJob(j.value, self._buf, self._host)
         self._d2h_fresh = True
 
     def _wait_d2h(self):
