@@ -81,12 +81,14 @@ class Graph:
             a._ensure_device()
         check(lib.vkc_graph_launch(self._h))
         self._launched = True
+        seq = self._dev.seq + 1  # one op for all the arrays
         for r in self._written.values():
             a = r()
             if a is not None:
                 a._dev_valid = True
                 a._host_valid = False
-                a.job = self._dev.issued()
+                a._job_seq = seq
+        self._dev.issued()
 
     def __del__(self):
         # The garbage collector may run this in the middle of another
