@@ -27,3 +27,12 @@ def test_launch_is_one_operation(gpu):
     for i, a in enumerate(arrays):
         a.wait()
         assert np.all(np.asarray(a) == 2.0 * (i + 1))
+
+
+def test_a_read_back_begun_before_a_launch_is_not_used(gpu):
+    """As for any other write after a prefetch."""
+    g, (a,) = _doubling_graph(gpu, 1)
+    g.launch()
+    a.prefetch()
+    g.launch()
+    assert np.all(np.asarray(a) == 4.0)

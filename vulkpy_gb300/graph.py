@@ -87,6 +87,7 @@ class Graph:
             if a is not None:
                 a._dev_valid = True
                 a._host_valid = False
+                a._d2h_fresh = False  # a read-back begun before has the values of before
                 a._job_seq = seq
         self._dev.issued()
 
