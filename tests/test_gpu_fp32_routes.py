@@ -95,6 +95,24 @@ def test_without_room_for_the_copies(gpu, vk, no_plans):
     assert rel_fro(np.asarray(c), exp) < 1e-6
 
 
+def test_without_room_for_the_partial_sums(gpu, vk, no_plans):
+    """300 x 300 x 400 in three K ranges: the operand copies can be had, the
+    ranges' partial sums cannot; the FMA GEMM needs neither."""
+    from vulkpy_gb300 import _lib
+    A, B = _operands(np.random.default_rng(3), 300, 300, 400, 0, 0)
+    a, b = vk.Array(gpu, data=A), vk.Array(gpu, data=B)
+    exp = A.astype(np.float64) @ B
+    try:
+        assert _lib.lib.vkc_inject_alloc_failure(2) == 0   # the third allocation: after the copies'
+        launches, c = _launches(gpu, lambda: a @ b)
+    finally:
+        _lib.lib.vkc_inject_alloc_failure(-1)
+    assert launches == 2                                   # the operand pre-pass, and the FMA GEMM
+    assert rel_fro(np.asarray(c), exp) < 1e-6
+    launches, c = _launches(gpu, lambda: a @ b)
+    assert launches == 3 and rel_fro(np.asarray(c), exp) < BOUND
+
+
 def _grouped(vk, gpu, A, B):
     """A @ B as a grouped product of one problem: launches and result."""
     from vulkpy_gb300 import _lib

@@ -1271,6 +1271,11 @@ int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t 
         dev, ma, mb, ma, mb, M, N, K, alpha, beta, C, ldc, epi, splits, nullptr,
         RepairOperands{A, B, lda, ldb, K, ta ? 1 : 0, tb ? 1 : 0}, repair);
   scratch_free(dev, scratch);
+  if (r == VKC_ERR_OOM) {
+    // no room for the ranges' partial sums, so the GEMM was not launched
+    clear_error();
+    return simt();
+  }
   return r;
 }
 
