@@ -250,17 +250,15 @@ __device__ __forceinline__ F2 log_unit(F2 w) {
   return f2_fma(e, f2(0x1.62e4p-1f), f2_fma(e, f2(0x1.7f7d1cp-20f), g));
 }
 
-// sqrt(-2 x), x in [-2^4, 0]: one Newton step from the reciprocal root (0
-// gives 1e-18, as if x were -5e-37).
+// sqrt(-2 x), x in [-2^4, 0]: one Newton step from the reciprocal root (of
+// 1e-36 for x = 0, so that 0 gives 0 and not 0 times infinity; the smallest
+// other x is -2^-23).
 __device__ __forceinline__ F2 sqrt_minus2(F2 x) {
-  F2 a = f2_mul(x, f2(-2.0f));
+  const F2 a = f2_mul(x, f2(-2.0f));
   float a0, a1, y0, y1;
   f2_get(a, a0, a1);
-  a0 = fmaxf(a0, 1e-36f);
-  a1 = fmaxf(a1, 1e-36f);
-  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y0) : "f"(a0));
-  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y1) : "f"(a1));
-  a = f2(a0, a1);
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y0) : "f"(fmaxf(a0, 1e-36f)));
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y1) : "f"(fmaxf(a1, 1e-36f)));
   const F2 y = f2(y0, y1), g = f2_mul(a, y), mg = f2_mul(g, f2(-1.0f));
   return f2_fma(f2_fma(mg, g, a), f2_mul(y, f2(0.5f)), g);
 }
