@@ -1,7 +1,11 @@
-"""The radius of the normal generator's pairs, over all its 2^23 arguments.  A state (0, 1, 0, w) gives the raw output rotl(w, 7), so that any
+"""The functions inside the normal generator, each over all its 2^23
+arguments.  A state (0, 1, 0, w) gives the raw output rotl(w, 7), so that any
 pair of uniforms can be put in.
 
-Bound, in ulps of the exact value: 1.5 (logf's 1 ulp, half of it after the square root, which is one of the
+Bounds, in ulps of the exact value: sin and cos 1.55 (the reduced argument is
+rounded once, half an ulp, which is one of the result's where that lies a
+binade below; half an ulp for the result; 0.05 for the polynomial), the radius
+1.5 (logf's 1 ulp, half of it after the square root, which is one of the
 result's in a lower binade; half an ulp for the result)."""
 import numpy as np
 import pytest
@@ -49,3 +53,18 @@ def test_radius_zero_gives_the_mean(gpu, every):
     for mean in (0.0, 1.5, 1e-20):
         for z in _pairs(gpu, np.zeros(len(k1), np.uint32), k1, mean=mean, stddev=3.0):
             np.testing.assert_array_equal(z, np.float32(mean))
+
+
+def test_sin_and_cos(gpu, every):
+    half = np.full(1, N // 2, np.uint32)
+    r = _pairs(gpu, half, np.zeros(1, np.uint32))[1][0]
+    sd = np.float32(1.0) / r
+    while _pairs(gpu, half, np.zeros(1, np.uint32), stddev=float(sd))[1][0] != 1.0:   # fl(r stddev) = 1
+        sd = np.nextafter(sd, np.float32(9))
+        assert sd < 2 / r
+    s, c = _pairs(gpu, np.full(N, N // 2, np.uint32), every, stddev=float(sd))
+    a = (np.float32(6.28318530718) * (every.astype(np.float32) / np.float32(N))).astype(np.float64)
+    assert s[0] == 0.0 and c[0] == 1.0
+    assert _ulps(s[1:], np.sin(a[1:])).max() < 1.55
+    assert _ulps(c, np.cos(a)).max() < 1.55
+    assert np.abs(s).max() <= 1.0 and np.abs(c).max() <= 1.0

@@ -194,8 +194,9 @@ __device__ __forceinline__ float to_unit(uint32_t r) { return __uint_as_float((r
 // 2^27 normals took 225 us with logf / sqrtf / sincosf (102 instructions per
 // pair even with these functions in scalar form: 215 us), 177 us so; the
 // store alone takes 79.  Polynomials are minimax fits (Lawson's iteration)
-// made for this file; log within 0.9 ulp and sin, cos within 1.5 ulp over all
-// their arguments.
+// made for this file.  Over all 2^23 arguments, in ulps of the exact value: log
+// within 0.9, sin within 1.42 and cos within 1.46 (sincosf: 1.45 and 1.47),
+// r / stddev within 0.98 (0.97).
 struct F2 {
   unsigned long long v;
 };
@@ -263,34 +264,38 @@ __device__ __forceinline__ F2 sqrt_minus2(F2 x) {
   return f2_fma(f2_fma(mg, g, a), f2_mul(y, f2(0.5f)), g);
 }
 
-// sin of y = a - kf pi (|y| <= pi/2 and a little), negated where the low bit of
-// kt is set.  pi in three parts; the first product leaves an exact difference.
-__device__ __forceinline__ F2 sin_reduced(F2 a, F2 kf, F2 kt) {
-  F2 y = f2_fma(kf, f2(-0x1.921fb6p+1f), a);
-  y = f2_fma(kf, f2(0x1.777a5cp-24f), y);
-  y = f2_fma(kf, f2(0x1.ee59dap-49f), y);
-  const F2 z = f2_mul(y, y);
-  F2 p = f2_fma(f2(0x1.5dbceap-19f), z, f2(-0x1.9f6feep-13f));
-  p = f2_fma(p, z, f2(0x1.110ed4p-7f));
-  p = f2_fma(p, z, f2(-0x1.55554cp-3f));
-  const F2 r = f2_fma(f2_mul(y, z), p, y);
-  float r0, r1, t0, t1;
-  f2_get(r, r0, r1);
-  f2_get(kt, t0, t1);
-  return f2(__uint_as_float(__float_as_uint(r0) ^ (__float_as_uint(t0) << 31)),
-            __uint_as_float(__float_as_uint(r1) ^ (__float_as_uint(t1) << 31)));
-}
-
-// sin and cos of a in [0, 2 pi].  cos(a) = -sin(a - (n + 1/2) pi) (-1)^n, so
-// both are sines of arguments near a zero and keep their relative accuracy.
+// sin and cos of a in [0, 2 pi]: a = n pi/2 + y with n the nearest whole
+// number, sin and cos of y (|y| <= pi/4) by their odd and even polynomials,
+// and the quadrant's exchange and signs.  pi/2 in three parts (Cody and Waite,
+// Software Manual for the Elementary Functions, 1980); the first product
+// leaves an exact difference, y is rounded once.
 __device__ __forceinline__ void sincos_turn(F2 a, F2& s, F2& c) {
-  const F2 inv = f2(0x1.45f306p-2f);
-  // adding 1.5 * 2^23 rounds to a whole number k, which is then in the low bits
-  F2 t = f2_fma(a, inv, f2(12582912.f));
-  s = sin_reduced(a, f2_add(t, f2(-12582912.f)), t);
-  // one more: the sign is (-1)^(n + 1)
-  t = f2_add(f2_fma(a, inv, f2(-0.5f)), f2(12582913.f));
-  c = sin_reduced(a, f2_add(f2_add(t, f2(-12582913.f)), f2(0.5f)), t);
+  // adding 1.5 * 2^23 rounds to a whole number, which is then in the low bits
+  const F2 t = f2_fma(a, f2(0x1.45f306p-1f), f2(12582912.f));
+  const F2 n = f2_add(t, f2(-12582912.f));
+  F2 y = f2_fma(n, f2(-0x1.921fb6p+0f), a);
+  y = f2_fma(n, f2(0x1.777a5cp-25f), y);
+  y = f2_fma(n, f2(0x1.ee59dap-50f), y);
+  const F2 z = f2_mul(y, y);
+  F2 p = f2_fma(f2(-0x1.995372p-13f), z, f2(0x1.110832p-7f));
+  p = f2_fma(p, z, f2(-0x1.555548p-3f));
+  F2 q = f2_fma(f2(0x1.99e0ecp-16f), z, f2(-0x1.6c0c1ap-10f));
+  q = f2_fma(q, z, f2(0x1.55554ap-5f));
+  q = f2_fma(q, z, f2(-0.5f));
+  float sy[2], cy[2], tt[2];
+  f2_get(f2_fma(f2_mul(y, z), p, y), sy[0], sy[1]);
+  f2_get(f2_fma(q, z, f2(1.0f)), cy[0], cy[1]);
+  f2_get(t, tt[0], tt[1]);
+  float so[2], co[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t k = __float_as_uint(tt[i]);
+    const float v = k & 1u ? cy[i] : sy[i], w = k & 1u ? sy[i] : cy[i];
+    so[i] = __uint_as_float(__float_as_uint(v) ^ ((k << 30) & 0x80000000u));
+    co[i] = __uint_as_float(__float_as_uint(w) ^ (((k + 1u) << 30) & 0x80000000u));
+  }
+  s = f2(so[0], so[1]);
+  c = f2(co[0], co[1]);
 }
 
 // Two pairs: from raw outputs (r0a, r1a) and (r0b, r1b).  1 - u0 and u1 are
