@@ -218,8 +218,10 @@ k_gemm_simt(int64_t M, int64_t N, int64_t K, float alpha, const float* __restric
 // 10.1, 1000 x 1000 x 64 11.7 -> 8.6.
 constexpr int kSmallT = 32, kSmallK = 64, kSmallThreads = 128;
 
+// (TB: five blocks per SM; without a bound the compiler holds back its loads to
+// fit more)
 template <bool TA, bool TB>
-__global__ void __launch_bounds__(kSmallThreads)
+__global__ void __launch_bounds__(kSmallThreads, TB ? 5 : 0)
 k_gemm_small(int M, int N, int K, float alpha, const float* __restrict__ A, int64_t lda, const float* __restrict__ B,
              int64_t ldb, float beta, float* C, int64_t ldc, GemmEpilogue epi) {
   __shared__ float As[kSmallK][kSmallT + 1];
@@ -229,15 +231,31 @@ k_gemm_small(int M, int N, int K, float alpha, const float* __restrict__ A, int6
   constexpr int kPer = kSmallT * kSmallK / kSmallThreads;  // 16
   float ra[kPer], rb[kPer];
   // a warp reads along each operand's contiguous index: run c = tid + 128 i,
-  // K contiguous: k = c % 64, row c / 64; else row c % 32, k = c / 32
+  // A K contiguous: k = c % 64, row c / 64; else row c % 32, k = c / 32.  B K
+  // contiguous: 8 k of 4 columns per warp, so that its stores (rows of 36
+  // words, 16-byte aligned for the reads) fall in 32 banks; along K they
+  // would meet four to a bank (1300 x 900 x 600: 78 -> 70 us).
+  const int bk = tid & 7, bn = ((tid & 31) >> 3) + 4 * (tid >> 5);  // TB: k bk + 8 i, columns bn, bn + 16
+  const float* bp0 = B + (int64_t)(n0 + bn) * ldb + bk;
+  const float* bp1 = bp0 + 16 * ldb;
   auto load = [&](int k0) {
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
       const int c = tid + kSmallThreads * i;
       const int ka = k0 + (TA ? c >> 5 : c & 63), m = m0 + (TA ? c & 31 : c >> 6);
       ra[i] = m < M && ka < K ? A[TA ? (int64_t)ka * lda + m : (int64_t)m * lda + ka] : 0.f;
-      const int kb = k0 + (TB ? c & 63 : c >> 5), n = n0 + (TB ? c >> 6 : c & 31);
-      rb[i] = n < N && kb < K ? B[TB ? (int64_t)n * ldb + kb : (int64_t)kb * ldb + n] : 0.f;
+      if (!TB) {
+        const int kb = k0 + (c >> 5), n = n0 + (c & 31);
+        rb[i] = n < N && kb < K ? B[(int64_t)kb * ldb + n] : 0.f;
+      }
+    }
+    if (TB) {
+#pragma unroll
+      for (int i = 0; i < kPer / 2; ++i) {
+        const int k = k0 + 8 * i;
+        rb[i] = n0 + bn < N && k + bk < K ? bp0[k] : 0.f;
+        rb[i + kPer / 2] = n0 + bn + 16 < N && k + bk < K ? bp1[k] : 0.f;
+      }
     }
   };
   float acc[2][4] = {};
@@ -248,7 +266,8 @@ k_gemm_small(int M, int N, int K, float alpha, const float* __restrict__ A, int6
     for (int i = 0; i < kPer; ++i) {
       const int c = tid + kSmallThreads * i;
       As[TA ? c >> 5 : c & 63][TA ? c & 31 : c >> 6] = ra[i];
-      Bs[TB ? c & 63 : c >> 5][TB ? c >> 6 : c & 31] = rb[i];
+      if (TB) Bs[bk + 8 * (i % (kPer / 2))][bn + 16 * (i / (kPer / 2))] = rb[i];
+      else Bs[c >> 5][c & 31] = rb[i];
     }
     __syncthreads();
     if (k0 + kSmallK < K) load(k0 + kSmallK);
@@ -285,10 +304,13 @@ k_gemm_small(int M, int N, int K, float alpha, const float* __restrict__ A, int6
   }
 }
 
-// The small kernel where the plan does not split K and its tiles fit the GPU
-// at once (8 blocks per SM: 1000 x 1000 x 64 11.7 -> 8.6 us; the 128 x 128 tile
-// reads less, and fills the GPU from there on).  A split plan keeps its ranges:
-// they are the more exact sum, and take 9.0 us at 256^3 against 9.7.
+// The small kernel where the plan does not split K and there are at most eight
+// tiles per SM (1000 x 1000 x 64 11.7 -> 8.6 us; the 128 x 128 tile reads less,
+// and fills the GPU from there on).  No bound on K: with so few results a long
+// one comes with a narrow matrix, whose 128 x 128 tiles are mostly padding (9900
+// x 17 x 6000 704 -> 264 us), and 1500 x 800 x 800 takes 92-96 us against 94-102.
+// A split plan keeps its ranges: they are the more exact sum, and take 9.0 us
+// at 256^3 against 9.7.
 inline bool gemm_is_small(vkc_device_t dev, int64_t M, int64_t N, int64_t K, int splits) {
   const int64_t tiles = ((M + kSmallT - 1) / kSmallT) * ((N + kSmallT - 1) / kSmallT);
   return K > 0 && K < (1 << 30) && splits == 1 && tiles <= (int64_t)dev->sm_count * 8;
