@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 from oracle.ops import rel_fro
-from test_gpu_fp32_tensor import BOUND, _operands, _poison, _same, plans, vk  # noqa: F401  (fixtures)
+from test_gpu_fp32_tensor import BOUND, _gemm, _operands, _poison, _same, plans, vk  # noqa: F401  (fixtures)
 
 pytestmark = pytest.mark.gpu
 
@@ -74,6 +74,42 @@ def test_values_outside_the_split(gpu, vk, plans, kind, splits):
     launches, got = _product(vk, gpu, A, B)
     assert launches == 3
     _same(got, A, B)
+    assert gpu.check_errors() == 0
+
+
+# partial sums recomputed inside the GEMM: each form, with operands that the
+# 16-byte loads can and cannot read, remainders of rows, columns and K
+@pytest.mark.parametrize("kind", ["nan", "large"])
+@pytest.mark.parametrize("m,n,k", [(1040, 1032, 1016), (1041, 1031, 1015)])
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_partial_sums_outside_the_split(gpu, vk, plans, kind, m, n, k, ta, tb):
+    plans(m, n, k, 3)
+    A, B = _operands(np.random.default_rng(13), m, n, k, 0, 0)
+    _poison(A, B, kind)
+    launches, got = _launches(gpu, lambda: _gemm(vk, gpu, np.ascontiguousarray(A.T) if ta else A,
+                                                 np.ascontiguousarray(B.T) if tb else B, ta, tb))
+    assert launches == 3
+    _same(got, A, B)
+    assert gpu.check_errors() == 0
+
+
+def test_partial_sums_outside_the_split_on_every_cta(gpu, vk, plans):
+    """More units per CTA than the mask of units to recompute has bits: rows at
+    both ends of the matrix, in either K range."""
+    m, n, k = 9300, 9200, 128
+    plans(m, n, k, 2)
+    rng = np.random.default_rng(14)
+    A, B = _operands(rng, m, n, k, 0, 0)
+    A[5, 100] = np.nan
+    A[9299, 3] = np.float32(2.0 ** 103)
+    launches, got = _product(vk, gpu, A, B)
+    assert launches == 3
+    assert np.all(np.isnan(got[5]))
+    rows = np.unique(np.concatenate([np.arange(0, 140), rng.integers(140, m, 200), np.arange(m - 140, m)]))
+    rows = rows[rows != 5]
+    e = A[rows].astype(np.float64) @ B
+    scale = np.abs(A[rows]).astype(np.float64) @ np.abs(B)
+    assert np.all(np.abs(got[rows] - e) <= (k + 2) * 2.0 ** -24 * scale)
     assert gpu.check_errors() == 0
 
 

@@ -37,10 +37,6 @@ __device__ __forceinline__ void split_bf16_3(float x, __nv_bfloat16& h, __nv_bfl
   if (!(fabsf(x) < 0x1p103f)) h = __ushort_as_bfloat16(0x7fffu);
 }
 
-__device__ __forceinline__ bool all_finite(float a, float b, float c, float d) {
-  return (a * 0.f + b * 0.f) + (c * 0.f + d * 0.f) == 0.f;
-}
-
 // Whether the first `cols` of a lane's N accumulators are finite.
 template <int N>
 __device__ __forceinline__ bool lane_finite(const float (&r)[N], int cols) {
@@ -50,29 +46,28 @@ __device__ __forceinline__ bool lane_finite(const float (&r)[N], int cols) {
   return t == 0.f;
 }
 
-// W neighbouring results (m, n..n+W-1) by one thread, eight k's loads ahead of
-// their (ordered) FMAs.
-template <int W>
-__device__ __noinline__ void repair_dots(const RepairOperands& o, int64_t m, int64_t n, float (&acc)[W]) {
-  const float* a = o.a + (o.ta ? m : m * o.lda);
-  const float* b = o.b + (o.tb ? n * o.ldb : n);
-  const int64_t sa = o.ta ? o.lda : 1, sb = o.tb ? 1 : o.ldb, sw = o.tb ? o.ldb : 1;
-#pragma unroll
-  for (int w = 0; w < W; ++w) acc[w] = 0.f;
-  for (int64_t k0 = 0; k0 < o.k; k0 += 8) {
-    float av[8], bv[8][W];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      const bool in = k0 + t < o.k;
-      av[t] = in ? a[(k0 + t) * sa] : 0.f;
-#pragma unroll
-      for (int w = 0; w < W; ++w) bv[t][w] = in ? b[(k0 + t) * sb + w * sw] : 0.f;
-    }
-#pragma unroll
-    for (int t = 0; t < 8; ++t)
-#pragma unroll
-      for (int w = 0; w < W; ++w) acc[w] = fmaf(av[t], bv[t][w], acc[w]);
-  }
+// The tile at (m0, n0) of the partial sums over k in [k0, k1), into out (M x N),
+// by the 256 threads of Sync.
+//
+// The partial sums are the place for it, since the K ranges share the work: a
+// thread per result in the reduction was a chain of all of K (256 x 256 with K =
+// 16384 of NaN 2150 us, so 155, FMAs alone 119), and a warp of the GEMM's
+// epilogue per 32 rows 1210 us.
+template <class Sync>
+__device__ __forceinline__ void repair_partial(const RepairOperands& o, int64_t M, int64_t N, int64_t m0, int64_t n0,
+                                               int64_t k0, int64_t k1, float* out, SimtSmem& sm) {
+  const float* a = o.a + (o.ta ? k0 * o.lda : k0);
+  const float* b = o.b + (o.tb ? k0 : k0 * o.ldb);
+  const GemmEpilogue none{};
+  Sync::sync();  // the previous tile's reads of `sm`
+  if (!o.ta && !o.tb)
+    simt_tile<false, false, Sync>(M, N, k1 - k0, 1.f, a, o.lda, b, o.ldb, 0.f, out, N, none, nullptr, m0, n0, sm);
+  else if (!o.tb)
+    simt_tile<true, false, Sync>(M, N, k1 - k0, 1.f, a, o.lda, b, o.ldb, 0.f, out, N, none, nullptr, m0, n0, sm);
+  else if (!o.ta)
+    simt_tile<false, true, Sync>(M, N, k1 - k0, 1.f, a, o.lda, b, o.ldb, 0.f, out, N, none, nullptr, m0, n0, sm);
+  else
+    simt_tile<true, true, Sync>(M, N, k1 - k0, 1.f, a, o.lda, b, o.ldb, 0.f, out, N, none, nullptr, m0, n0, sm);
 }
 
 // The 128 x 128 tiles that a GEMM launch left (list[0] of them, numbered along

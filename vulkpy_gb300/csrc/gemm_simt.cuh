@@ -48,15 +48,20 @@ __device__ __forceinline__ float act_deriv(float v, float y, int act) {
 // One 128 x 128 output tile at (m0, n0).  `mask` (may be NULL, same layout
 // as C) multiplies the result by the derivative of activation `mact` at
 // mask[m, n].  The caller synchronises the block before reusing `sm` for
-// another tile.
-template <bool TA, bool TB>
+// another tile.  Sync: the 256 threads that compute it (BlockSync: the block).
+struct BlockSync {
+  static __device__ __forceinline__ int thread() { return threadIdx.x; }
+  static __device__ __forceinline__ void sync() { __syncthreads(); }
+};
+
+template <bool TA, bool TB, class Sync = BlockSync>
 __device__ __forceinline__ void simt_tile(int64_t M, int64_t N, int64_t K, float alpha, const float* __restrict__ A,
                                           int64_t lda, const float* __restrict__ B, int64_t ldb, float beta, float* C,
                                           int64_t ldc, GemmEpilogue epi, const float* __restrict__ mask, int64_t m0,
                                           int64_t n0, SimtSmem& sm, int mact = VKC_ACT_RELU) {
   auto& As = sm.As;
   auto& Bs = sm.Bs;
-  const int tid = threadIdx.x;
+  const int tid = Sync::thread();
   const int tx = tid & 15, ty = tid >> 4;
 
   // Per K step each thread loads 8 elements of the A tile and 8 of the B
@@ -134,7 +139,7 @@ __device__ __forceinline__ void simt_tile(int64_t M, int64_t N, int64_t K, float
   load_a(0);
   load_b(0);
   store(0);
-  __syncthreads();
+  Sync::sync();
   for (int64_t ks = 0; ks < ksteps; ++ks) {
     const int buf = ks & 1;
     if (ks + 1 < ksteps) {
@@ -156,7 +161,7 @@ __device__ __forceinline__ void simt_tile(int64_t M, int64_t N, int64_t K, float
     }
     if (ks + 1 < ksteps) {
       store(buf ^ 1);
-      __syncthreads();
+      Sync::sync();
     }
   }
 

@@ -21,7 +21,7 @@
 // cannot hold (inf, NaN, |x| >= 2^103) become NaN in hi, so every result they
 // reach is not finite; tiles with results that are not finite are recomputed
 // from the fp32 operands with ordered FMAs (k_gemm_repair; with split K the
-// reduction recomputes single results).
+// tiles of partial sums, at the end of the GEMM itself).
 //
 // k_gemm_tcp is persistent (one CTA per SM; each CTA loads every operand tile
 // it multiplies into its own shared memory) with two TMEM accumulators, so a
@@ -87,7 +87,8 @@ struct PCfg {
   // full[kRing], empty[kRing], accf[2], acce[2], drain, red[2], epi, loe[2],
   // then tmem slot, abort flag and two tile flags
   static constexpr uint32_t kSlotOff = kBarOff + 8u * (2 * kRing + 10);
-  static constexpr uint32_t kEpiOff = (kSlotOff + 16 + 127) / 128 * 128;  // per-warp epilogue stages
+  static constexpr uint32_t kRedoOff = kSlotOff + 16;  // PARTS == 3: units to recompute (two words)
+  static constexpr uint32_t kEpiOff = (kRedoOff + (PARTS == 3 ? 8 : 0) + 127) / 128 * 128;  // per-warp epilogue stages
   static constexpr uint32_t kSmem = kEpiOff + kEpiWarps * kEpiStageBytes + 1024 /*alignment slack*/;
 };
 
@@ -158,14 +159,40 @@ __device__ __forceinline__ void cluster_reduce_rows(const float* partial, int sp
 // map_a / map_b: the hi copies (PARTS == 3: the three copies one after the
 // other as 3 M and 3 N rows); map_alo / map_blo: the lo copies (PARTS == 2).
 // repair (PARTS == 3): count of tiles of C left to k_gemm_repair, then their
-// numbers.
-template <int PARTS, int BN, int STAGES, int DRAIN>
+// numbers; SPLIT (PARTS == 3): partial sums, with ro, the fp32 operands, for
+// those that are not finite (an instantiation of its own: in one kernel the
+// form without split took 2% longer, 4096^3 600 -> 615 us).
+// The epilogue warps, for simt_tile.
+struct EpiWarpsSync {
+  static __device__ __forceinline__ int thread() { return (int)threadIdx.x - 64; }
+  static __device__ __forceinline__ void sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+};
+static_assert(kEpiWarps * 32 == kGemmThreads && kThreadsP == kGemmThreads + 64, "EpiWarpsSync");
+
+// The units of this CTA marked in `redo` (k_gemm_tcp), by its epilogue warps.
+// Out of line, so that the GEMM's registers and code are as without it.
+template <int BN>
+__device__ __noinline__ void repair_units(const RepairOperands& ro, const uint32_t* redo, int M, int N, int K, int splits,
+                                          int kps, int m_blocks, int n_blocks, float* partial, SimtSmem& sm) {
+  const int nk = (K + kBK - 1) / kBK, units = m_blocks * n_blocks * splits;
+  for (int i = 0, u = (int)blockIdx.x; u < units; ++i, u += (int)gridDim.x) {
+    const int bit = min(i, 63);
+    if (!(redo[bit >> 5] >> (bit & 31) & 1u)) continue;
+    const PUnit p = unit_of<BN>(u, splits, kps, nk, m_blocks, n_blocks);
+    const int64_t k0 = (int64_t)p.kb0 * kBK;
+    repair_partial<EpiWarpsSync>(ro, M, N, p.m0, p.n0, k0, min((int64_t)K, k0 + (int64_t)p.nkb * kBK),
+                                 partial + (int64_t)p.z * M * N, sm);
+  }
+}
+
+template <int PARTS, int BN, int STAGES, int DRAIN, bool SPLIT = false>
 __global__ void __launch_bounds__(kThreadsP, 1)
 k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
            const __grid_constant__ CUtensorMap map_alo, const __grid_constant__ CUtensorMap map_blo, int M, int N,
            int K, float alpha, float beta, float* __restrict__ C, int64_t ldc, const float* __restrict__ bias, int act,
            uint32_t* err, float* __restrict__ partial, int splits, int kps, int m_blocks, int n_blocks,
-           int cl_reduce, const float* __restrict__ dmask, int dact, uint32_t* __restrict__ repair) {
+           int cl_reduce, const float* __restrict__ dmask, int dact, uint32_t* __restrict__ repair,
+           const __grid_constant__ RepairOperands ro) {
   using Cfg = PCfg<PARTS, BN, STAGES>;
   constexpr bool X3 = PARTS > 1;      // a split mode: accumulations drained into fp32 registers
   constexpr int R = Cfg::kRing;
@@ -189,6 +216,8 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   auto loe_bar = [&](int b) { return bars + 8u * (2 * R + 8 + b); };  // PARTS == 3: small-term accumulator read
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + Cfg::kSlotOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  // PARTS == 3: bit i: this CTA's i-th unit's partial sums are not all finite (bit 63: one from the 64th on)
+  uint32_t* redo = reinterpret_cast<uint32_t*>(gbase + Cfg::kRedoOff);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -212,6 +241,7 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     }
     mbar_init(epi_bar, kEpiWarps);
     abort_flag[0] = abort_flag[1] = abort_flag[2] = 0;
+    if (PARTS == 3 && SPLIT) redo[0] = redo[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -484,7 +514,7 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       }
       if (!ok) break;
       if (ngroups == 0) continue;
-      const bool raw_out = partial != nullptr;
+      const bool raw_out = PARTS == 3 ? SPLIT : partial != nullptr;
       bool skip = false;
       if (PARTS == 3 && !raw_out) {
         // A tile with a result that is not finite is left to k_gemm_repair
@@ -501,6 +531,12 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         ++red_it;
         if (skip && warp == 2 && lane == 0)
           repair[1 + atomicAdd(repair, 1u)] = (uint32_t)((p.m0 / kBM) * n_blocks + p.n0 / BN);
+      } else if (PARTS == 3) {
+        const bool bad = p.m0 + q * 32 + lane < M && !lane_finite(acc, N - (p.n0 + h * CW));
+        if (__any_sync(0xffffffffu, bad) && lane == 0) {
+          const int i = min((u - (int)blockIdx.x) / (int)gridDim.x, 63);
+          atomicOr(redo + (i >> 5), 1u << (i & 31));
+        }
       }
       float* cbase = raw_out ? partial + (int64_t)p.z * M * N : C;
       const int64_t ld = raw_out ? (int64_t)N : ldc;
@@ -565,6 +601,9 @@ k_gemm_tcp(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
   }
+  if (PARTS == 3 && SPLIT && warp >= 2 && !*abort_flag && (redo[0] | redo[1]))
+    // the copies and MMAs are done with shared memory
+    repair_units<BN>(ro, redo, M, N, K, splits, kps, m_blocks, n_blocks, partial, *reinterpret_cast<SimtSmem*>(gbase));
   // no CTA leaves while a peer may still arrive on its barriers
   if (cl_reduce) cluster_sync_all();
 }
@@ -867,13 +906,10 @@ __device__ __forceinline__ void split_out1(const SplitOut& so, int64_t r, int64_
 
 // Four columns per thread (N % 4 == 0, ldc % 4 == 0, 16-byte aligned C);
 // the split loads are issued four at a time ahead of their (ordered) adds.
-// REPAIR: a quad with a sum that is not finite is recomputed from the
-// operands `ro`.
-template <bool REPAIR>
 __global__ void __launch_bounds__(256)
 k_splitk_reduce4(const float* __restrict__ partial, int splits, int64_t M, int64_t N, float alpha, float beta,
                  float* __restrict__ C, int64_t ldc, const float* __restrict__ bias, int act,
-                 const float* __restrict__ dmask, int dact, SplitOut so, RepairOperands ro) {
+                 const float* __restrict__ dmask, int dact, SplitOut so) {
   pdl_wait();
   pdl_trigger();
   const int64_t total = M * N, quads = total / 4;
@@ -893,11 +929,6 @@ k_splitk_reduce4(const float* __restrict__ partial, int splits, int64_t M, int64
     }
     for (; z < splits; ++z) add4(s, __ldcs(p + (int64_t)z * quads));
     const int64_t r = i / N, col = i - r * N;
-    if (REPAIR && !all_finite(s.x, s.y, s.z, s.w)) {
-      float v[4];
-      repair_dots<4>(ro, r, col, v);
-      s = make_float4(v[0], v[1], v[2], v[3]);
-    }
     float4* cp = reinterpret_cast<float4*>(C + r * ldc + col);
     const float4 c0 = beta != 0.f ? *cp : make_float4(0.f, 0.f, 0.f, 0.f);
     float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -920,11 +951,10 @@ k_splitk_reduce4(const float* __restrict__ partial, int splits, int64_t M, int64
   }
 }
 
-template <bool REPAIR>
 __global__ void __launch_bounds__(256)
 k_splitk_reduce(const float* __restrict__ partial, int splits, int64_t M, int64_t N, float alpha, float beta,
                 float* __restrict__ C, int64_t ldc, const float* __restrict__ bias, int act,
-                const float* __restrict__ dmask, int dact, SplitOut so, RepairOperands ro) {
+                const float* __restrict__ dmask, int dact, SplitOut so) {
   pdl_wait();
   pdl_trigger();
   const int64_t total = M * N;
@@ -933,11 +963,6 @@ k_splitk_reduce(const float* __restrict__ partial, int splits, int64_t M, int64_
     float s = partial[i];
     for (int z = 1; z < splits; ++z) s += partial[(int64_t)z * total + i];
     const int64_t r = i / N, col = i - r * N;
-    if (REPAIR && !isfinite(s)) {
-      float v[1];
-      repair_dots<1>(ro, r, col, v);
-      s = v[0];
-    }
     float* c = C + r * ldc + col;
     float v = splitk_epilogue(s, alpha, beta, beta != 0.f ? *c : 0.f, bias != nullptr, bias ? bias[col] : 0.f, act);
     if (dmask) v = act_deriv(v, dmask[r * ldc + col], dact);
@@ -947,22 +972,15 @@ k_splitk_reduce(const float* __restrict__ partial, int splits, int64_t M, int64_
 }
 
 int splitk_reduce(vkc_device_t dev, const float* partial, int splits, int64_t M, int64_t N, float alpha, float beta,
-                  float* C, int64_t ldc, const GemmEpilogue& epi, const SplitOut* out = nullptr,
-                  const RepairOperands& ro = RepairOperands{}) {
+                  float* C, int64_t ldc, const GemmEpilogue& epi, const SplitOut* out = nullptr) {
   const SplitOut so = out ? *out : SplitOut{nullptr, nullptr, 0};
   const bool vec = N % 4 == 0 && ldc % 4 == 0 && ((uintptr_t)C & 15u) == 0 && ((uintptr_t)epi.dmask & 15u) == 0;
   auto launch = [&](auto kern, unsigned grid) {
     return launch_pdl(kern, dim3(grid), dim3(256), 0, dev->stream, partial, splits, M, N, alpha, beta, C, ldc,
-                      epi.bias, epi.act, epi.dmask, epi.dact, so, ro);
+                      epi.bias, epi.act, epi.dmask, epi.dact, so);
   };
-  cudaError_t e;
-  if (vec) {
-    const unsigned g = wave_grid(dev, k_splitk_reduce4<false>, (size_t)(M * N / 4), 256);
-    e = ro.a ? launch(k_splitk_reduce4<true>, g) : launch(k_splitk_reduce4<false>, g);
-  } else {
-    const unsigned g = stream_grid(dev, (size_t)(M * N), 256);
-    e = ro.a ? launch(k_splitk_reduce<true>, g) : launch(k_splitk_reduce<false>, g);
-  }
+  const cudaError_t e = vec ? launch(k_splitk_reduce4, wave_grid(dev, k_splitk_reduce4, (size_t)(M * N / 4), 256))
+                            : launch(k_splitk_reduce, stream_grid(dev, (size_t)(M * N), 256));
   if (e != cudaSuccess) return set_error(VKC_ERR_CUDA, "splitk_reduce launch: %s", cudaGetErrorString(e));
   return check_launch("splitk_reduce");
 }
@@ -1009,13 +1027,13 @@ int max_clusters(Kern kern, uint32_t smem, int size) {
   return n;
 }
 
-template <int PARTS, int BN, int STAGES, int DRAIN>
+template <int PARTS, int BN, int STAGES, int DRAIN, bool SPLIT = false>
 int launch_tcp(vkc_device_t dev, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& malo,
                const CUtensorMap& mblo, int64_t M, int64_t N, int64_t K, float alpha, float beta, float* C,
                int64_t ldc, const GemmEpilogue& epi, int splits, const SplitOut* out,
                const RepairOperands& ro = RepairOperands{}, uint32_t* repair = nullptr) {
   using Cfg = PCfg<PARTS, BN, STAGES>;
-  auto kern = k_gemm_tcp<PARTS, BN, STAGES, DRAIN>;
+  auto kern = k_gemm_tcp<PARTS, BN, STAGES, DRAIN, SPLIT>;
   static bool attr_set = false;
   if (!attr_set) {
     VKC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem));
@@ -1061,17 +1079,18 @@ int launch_tcp(vkc_device_t dev, const CUtensorMap& ma, const CUtensorMap& mb, c
     const int ctas = (int)std::min<int64_t>(tiles, clusters) * splits;
     e = launch_pdl_cluster(kern, dim3((unsigned)ctas), dim3(kThreadsP), Cfg::kSmem, dev->stream, (unsigned)splits, ma,
                            mb, malo, mblo, (int)M, (int)N, (int)K, alpha, beta, C, ldc, epi.bias, epi.act,
-                           dev->err_word, partial, splits, kps, (int)m_blocks, n_blocks, 1, epi.dmask, epi.dact, nullptr);
+                           dev->err_word, partial, splits, kps, (int)m_blocks, n_blocks, 1, epi.dmask, epi.dact, nullptr,
+                           ro);
   } else {
     const int ctas = (int)std::min<int64_t>(units, max_ctas(dev, kern, Cfg::kSmem));
     e = launch_pdl(kern, dim3((unsigned)ctas), dim3(kThreadsP), Cfg::kSmem, dev->stream, ma, mb, malo, mblo, (int)M,
                    (int)N, (int)K, alpha, beta, C, ldc, epi.bias, epi.act, dev->err_word, partial, splits, kps,
-                   (int)m_blocks, n_blocks, 0, epi.dmask, epi.dact, repair);
+                   (int)m_blocks, n_blocks, 0, epi.dmask, epi.dact, repair, ro);
   }
   int r = e == cudaSuccess ? check_launch("gemm_tc")
                            : set_error(VKC_ERR_CUDA, "gemm_tc launch: %s", cudaGetErrorString(e));
   if (r == VKC_OK && splits > 1 && clusters == 0)
-    r = splitk_reduce(dev, partial, splits, M, N, alpha, beta, C, ldc, epi, out, ro);
+    r = splitk_reduce(dev, partial, splits, M, N, alpha, beta, C, ldc, epi, out);
   else if (r == VKC_OK && PARTS == 3)
     r = gemm_repair(dev, ro, M, N, alpha, beta, C, ldc, epi, repair);
   else if (r == VKC_OK && out)  // no reduction launch to write it: the pre-pass kernel on C
@@ -1250,8 +1269,9 @@ int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t 
   }
   {
     static std::atomic<uint64_t> loaded{0};
-    load_kernels(dev, loaded, k_split_pair<3>, k_gemm_tcp<3, 128, 2, 1>, k_gemm_tcp<3, 128, 2, 2>,
-                 k_splitk_reduce4<true>, k_splitk_reduce<true>, k_gemm_repair<false, false>, k_gemm_repair<false, true>,
+    load_kernels(dev, loaded, k_split_pair<3>, k_gemm_tcp<3, 128, 2, 1>, k_gemm_tcp<3, 128, 2, 1, true>,
+                 k_gemm_tcp<3, 128, 2, 2, true>,
+                 k_splitk_reduce4, k_splitk_reduce, k_gemm_repair<false, false>, k_gemm_repair<false, true>,
                  k_gemm_repair<true, false>, k_gemm_repair<true, true>);
   }
   auto* a = static_cast<__nv_bfloat16*>(scratch);
@@ -1267,7 +1287,7 @@ int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t 
     // ranges, U[0,1) data: error 8.0e-8 -> 5.5e-8, where FMAs in 16 ranges of
     // 16 gave 6.1e-8); else one, which drains half as often (2048^3 in 2
     // ranges: 128 -> 114 us) and which the grouped kernel reproduces
-    r = (splits > 1 && Kp / splits <= 256 ? launch_tcp<3, 128, 2, 2> : launch_tcp<3, 128, 2, 1>)(
+    r = (splits == 1 ? launch_tcp<3, 128, 2, 1> : Kp / splits <= 256 ? launch_tcp<3, 128, 2, 2, true> : launch_tcp<3, 128, 2, 1, true>)(
         dev, ma, mb, ma, mb, M, N, K, alpha, beta, C, ldc, epi, splits, nullptr,
         RepairOperands{A, B, lda, ldb, K, ta ? 1 : 0, tb ? 1 : 0}, repair);
   scratch_free(dev, scratch);
