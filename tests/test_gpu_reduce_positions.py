@@ -1,0 +1,31 @@
+"""Arg-reductions with the extreme at every place of a thread's group of 16, and
+axis reductions with every remainder of eight rows."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+# one block (256 threads, 16 elements each) and a little more; aligned and not
+@pytest.mark.parametrize("n", [1, 5, 255, 1030, 4096, 4099])
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("op", ["argmax", "argmin"])
+def test_extreme_at_every_place(gpu, n, offset, op):
+    import ctypes as C
+    import vulkpy_gb300 as vk
+    from vulkpy_gb300 import _lib
+    sign = np.float32(1 if op == "argmax" else -1)
+    out = vk.U32Array(gpu, shape=(1,))
+    for at in sorted({0, 1, 3, 4, n // 4, n // 2, 3 * n // 4, n - 4, n - 2, n - 1} & set(range(n))):
+        for twin in (n - 1, at):
+            x = np.zeros(n + 1, np.float32)
+            x[offset + at] = x[offset + max(at, twin)] = 2 * sign     # equal ones: the first
+            x[offset + n:] = 9 * sign                                # not part of the input
+            if offset:
+                x[0] = 9 * sign
+            a = vk.Array(gpu, data=x)
+            st = _lib.lib.vkc_arg_reduce_all(gpu.handle, _lib.ARGMAX if op == "argmax" else _lib.ARGMIN,
+                                             C.c_void_p(a._dptr() + 4 * offset), n, out._buf.ptr)
+            assert st == 0
+            out._written()
+            assert np.asarray(out)[0] == at, (at, twin)
