@@ -300,7 +300,12 @@ __global__ void k_combine_splits(const float2* partials, size_t prev, size_t axi
 
 // post > 1: each thread owns VW consecutive columns (VW = 4 -> float4) of
 // one (prev, slice) and walks its slice of the axis.
-template <int OP, bool COMP, int VW>
+// STREAM (VW == 1): loads that do not stay in the L2 cache, for an input that
+// does not fit it.  Rows of an odd width share sectors with their neighbours,
+// so for one that does fit they cost (3000 x 5001 sum: 40 us with them, 18
+// without; 8191 x 8193 maximum: 61 and 64).
+constexpr size_t kStreamElems = size_t(30) << 20;  // 120 MiB
+template <int OP, bool COMP, int VW, bool STREAM>
 __global__ void __launch_bounds__(kThreads)
 k_cols(const float* a, size_t prev, size_t axis, size_t post, int splits, float* out, float2* partials,
        int rebroadcast, float scale) {
@@ -336,13 +341,15 @@ k_cols(const float* a, size_t prev, size_t axis, size_t post, int splits, float*
       acc[0].push(v.x); acc[1].push(v.y); acc[2].push(v.z); acc[3].push(v.w);
     }
   } else {
-    // one column (post not a multiple of 4): 16 rows' loads ahead of their adds
-    for (; k + 15 < k1; k += 16) {
-      float v[16];
+    // one column (post not a multiple of 4): several rows' loads ahead of
+    // their adds, eight where an add is the compensated sum's chain
+    constexpr int U = COMP ? 8 : 16;
+    for (; k + (U - 1) < k1; k += U) {
+      float v[U];
 #pragma unroll
-      for (int u = 0; u < 16; ++u) v[u] = __ldcs(base + (k + u) * post);
+      for (int u = 0; u < U; ++u) v[u] = STREAM ? __ldcs(base + (k + u) * post) : base[(k + u) * post];
 #pragma unroll
-      for (int u = 0; u < 16; ++u) acc[0].push(v[u]);
+      for (int u = 0; u < U; ++u) acc[0].push(v[u]);
     }
 #pragma unroll 4
     for (; k < k1; ++k) acc[0].push(base[k * post]);
@@ -391,8 +398,8 @@ k_cols_block(const float* a, size_t prev, size_t axis, size_t post, float* out, 
   for (int v = 0; v < VW; ++v) acc[v].init();
   if (cin) {
     const float* base = a + i * axis * post + j;
-    size_t k = k0;
     if constexpr (VW == 4) {
+      size_t k = k0;
       for (; k + 7 < k1; k += 8) {
         float4 x[8];
 #pragma unroll
@@ -407,19 +414,29 @@ k_cols_block(const float* a, size_t prev, size_t axis, size_t post, float* out, 
         acc[0].push(x.x); acc[1].push(x.y); acc[2].push(x.z); acc[3].push(x.w);
       }
     } else {
-      for (; k + 7 < k1; k += 8) {
+      // through a stepped pointer: the offsets of eight rows would not fit 32 registers
+      const float* p = base + k0 * post;
+      int left = (int)(k1 - k0);
+      for (; left >= 8; left -= 8) {
         float x[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) x[u] = base[(k + u) * post];
+        for (int u = 0; u < 8; ++u, p += post) x[u] = *p;
 #pragma unroll
         for (int u = 0; u < 8; ++u) acc[0].push(x[u]);
       }
-      float x[7];  // the rest of the slice, its loads together too
+      if (left >= 4) {  // the rest of the slice: four to seven rows' loads together too
+        float x[7];
 #pragma unroll
-      for (int u = 0; u < 7; ++u) x[u] = k + u < k1 ? base[(k + u) * post] : 0.f;
+        for (int u = 0; u < 7; ++u) {
+          x[u] = *p;
+          if (u + 1 < left) p += post;
+        }
 #pragma unroll
-      for (int u = 0; u < 7; ++u)
-        if (k + u < k1) acc[0].push(x[u]);
+        for (int u = 0; u < 7; ++u)
+          if (u < left) acc[0].push(x[u]);
+      } else {
+        for (; left > 0; --left, p += post) acc[0].push(*p);
+      }
     }
   }
 #pragma unroll
@@ -433,7 +450,7 @@ k_cols_block(const float* a, size_t prev, size_t axis, size_t post, float* out, 
     const int col = lane * VW + w;
     Acc<OP, COMP> r;
     r.init();
-#pragma unroll
+// (unrolled whole, the merges of 32 warps took 50 registers, and one block fitted an SM)
     for (int ww = 0; ww < NW; ++ww) r.merge(sh_s[ww][col], sh_c[ww][col]);
     float val = r.value();
     if (OP == VKC_SUM || OP == VKC_PROD) val *= scale;
@@ -545,11 +562,14 @@ int reduce_axis_impl(vkc_device_t dev, const float* a, size_t prev, size_t axis,
   }
   dim3 grid((unsigned)((cols_threads + kThreads - 1) / kThreads), (unsigned)splits);
   if (vec)
-    k_cols<OP, COMP, 4><<<grid, kThreads, 0, dev->stream>>>(a, prev, axis, post, splits, out, partials,
-                                                            rebroadcast, scale);
+    k_cols<OP, COMP, 4, false><<<grid, kThreads, 0, dev->stream>>>(a, prev, axis, post, splits, out, partials,
+                                                                   rebroadcast, scale);
+  else if (prev * axis * post < kStreamElems)
+    k_cols<OP, COMP, 1, false><<<grid, kThreads, 0, dev->stream>>>(a, prev, axis, post, splits, out, partials,
+                                                                   rebroadcast, scale);
   else
-    k_cols<OP, COMP, 1><<<grid, kThreads, 0, dev->stream>>>(a, prev, axis, post, splits, out, partials,
-                                                            rebroadcast, scale);
+    k_cols<OP, COMP, 1, true><<<grid, kThreads, 0, dev->stream>>>(a, prev, axis, post, splits, out, partials,
+                                                                  rebroadcast, scale);
   int r = vkc::check_launch("reduce_cols");
   if (r == VKC_OK && splits > 1) {
     unsigned g2 = (unsigned)((prev * post + kThreads - 1) / kThreads);
