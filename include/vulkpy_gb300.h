@@ -332,7 +332,10 @@ int vkc_gemm(vkc_device_t dev, int precision, int trans_a, int trans_b,
  * table written by vulkpy_gb300/autotune.py is loaded at import; shapes
  * without an entry use 256-wide tiles and an occupancy heuristic for splits.
  * fp32: tile_n = 256 sets the split count of the FMA GEMM, 128 that of the
- * three-part tensor-core product too.  get: the plan a shape will use.  tune_set/tune_get are the same with
+ * three-part tensor-core product too.  (vkc_matmul takes the faster of the two
+ * by an estimate of the FMA GEMM's time, which its split count enters.)
+ * get: the plan that vkc_gemm will use for a shape, in fp32 the split count of
+ * the kernel that the shape runs on.  tune_set/tune_get are the same with
  * tile_n = 256 / without it.  No reference counterpart (matmul.comp has no
  * tiling). */
 int vkc_gemm_plan_set(int precision, int64_t m, int64_t n, int64_t k, int splits, int tile_n);

@@ -1,6 +1,9 @@
 """
 Autotuner for the GEMMs: CTA tile width and split-K count of the tensor-core
-GEMM (bf16 and split-bf16x3), split-K count of the fp32 SIMT GEMM.
+GEMM (bf16 and split-bf16x3), split-K count of the fp32 FMA GEMM.  (fp32
+products that vkc_gemm runs on the tensor cores, from m n k = 2^30 on, are not
+tuned: their split count has a rule of its own, and a bucket's entry is
+measured on a shape of it that runs FMAs.)
 
 For each size bucket (ceil(log2) of M, N and K) the tuner times every
 candidate (tile width 256 or 128, split count) on a representative problem of
@@ -19,7 +22,7 @@ import json
 import os
 import sys
 import time
-from typing import Dict, Iterable, List, Tuple
+from typing import Dict, Iterable, List, Optional, Tuple
 
 import numpy as np
 
@@ -80,6 +83,20 @@ def default_shapes() -> List[Tuple[int, int, int]]:
     return sorted(rep.values())
 
 
+FP32_TENSOR_WORK = 1 << 30  # m n k from which vkc_gemm's fp32 products leave the FMA GEMM
+
+
+def fma_shape(m: int, n: int, k: int) -> Optional[Tuple[int, int, int]]:
+    """A shape of the bucket of (m, n, k), that one if possible, whose fp32
+    vkc_gemm runs FMAs; None when the whole bucket runs on the tensor cores."""
+    low = [(1 << bucket(x)) // 2 + 1 for x in (m, n, k)]
+    for f in (1.0, 0.9, 0.8, 0.7, 0.6, 0.5):
+        s = tuple(max(lo, int(x * f)) for lo, x in zip(low, (m, n, k)))
+        if s[0] * s[1] * s[2] < FP32_TENSOR_WORK:
+            return s
+    return None
+
+
 def _time_gemm(gpu, a, b, c, m, n, k, reps=5, calls=16, prec=None) -> float:
     """Device time of one call in ms.  The calls are captured in a CUDA
     graph and replayed, so host-side launch cost (which a graph removes)
@@ -130,8 +147,13 @@ def tune(shapes: Iterable[Tuple[int, int, int]] = None, verbose: bool = True, on
         if only is not None and name != only:
             continue
         entries = []
-        tiles = TILES if prec != _lib.MM_FP32 else (256,)   # the SIMT GEMM has one tile shape
-        for (m, n, k) in shapes:
+        tiles = TILES if prec != _lib.MM_FP32 else (256,)   # the FMA GEMM has one tile shape
+        for shape in shapes:
+            if prec == _lib.MM_FP32:
+                shape = fma_shape(*shape)
+                if shape is None:
+                    continue
+            m, n, k = shape
             rng = np.random.default_rng(m * 31 + n * 7 + k)
             A = vk.Array(gpu, data=rng.standard_normal((m, k)).astype(np.float32))
             B = vk.Array(gpu, data=rng.standard_normal((n, k)).astype(np.float32))

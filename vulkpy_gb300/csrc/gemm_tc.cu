@@ -1155,6 +1155,7 @@ VKC_EXPORT int vkc_gemm_plan_get(vkc_device_t dev, int precision, int64_t m, int
   VKC_REQUIRE(dev && splits, "NULL argument");
   if (precision == VKC_MM_FP32) {
     *splits = vkc::simt_splits(dev, m, n, k);
+    if (vkc::layer_fp32_on_tensor_cores(m, n, k, *splits)) *splits = vkc::fp32_tc_splits(dev, m, n, k);
     if (tile_n) *tile_n = 128;
     return VKC_OK;
   }
