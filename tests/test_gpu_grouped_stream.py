@@ -74,3 +74,30 @@ def test_training_step_on_a_callers_stream(gpu, caller_stream, step):
     caller_stream(False)
     for a, b in zip(own, got):
         np.testing.assert_array_equal(a, b)
+
+
+def test_side_branch_where_the_gpu_is_waited_for(gpu, monkeypatch):
+    """A step of small models run call by call waits for the host, and stays on
+    one stream; the same values as on the branch, which a graph uses."""
+    import vulkpy_gb300 as vk
+    from vulkpy_gb300.nn.grouped import GroupedSequence
+    used = []
+    beside = GroupedSequence._beside
+    monkeypatch.setattr(GroupedSequence, "_beside", lambda self, side, run: used.append(side) or beside(self, side, run))
+    off = _grouped_step(gpu)
+    assert not any(used)
+    with monkeypatch.context() as m:
+        m.setattr(GroupedSequence, "_gpu_bound", lambda self, batch: True)
+        on = _grouped_step(gpu)
+    assert any(used)
+    for a, b in zip(off, on):
+        np.testing.assert_array_equal(a, b)
+    from vulkpy_gb300 import nn
+    nets, xs, ys = _models(gpu, lambda: nn.SGD(lr=1e-2))
+    group = GroupedSequence(nets)
+    ax, ay = ([vk.Array(gpu, data=v) for v in a] for a in (xs, ys))
+    group.train(ax, ay)
+    used.clear()
+    with vk.graph.Graph(gpu):
+        group.train(ax, ay)
+    assert used and all(used)

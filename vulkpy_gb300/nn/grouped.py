@@ -129,9 +129,6 @@ class GroupedSequence:
         px, py = _ptrs([p._dptr() for p in preds]), _ptrs([y._dptr() for y in ys])
         batch = (C.c_int64 * n)(*[p.shape[0] for p in preds])
         cols = (C.c_int64 * n)(*[p.shape[1] for p in preds])
-        check(lib.vkc_mse_grouped(gpu._dev.h, px, py, _ptrs([d._buf.ptr or 0 for d in dys]), batch, cols, None, n))
-        for d in dys:
-            d._written()
         # The loss values and the bias gradients and steps are needed by
         # nothing in the backward: on the device's own stream they run on the
         # side branch, beside the tiling passes and GEMMs, and join at the
@@ -139,19 +136,40 @@ class GroupedSequence:
         # until then: freed on the main stream before, it could be handed to
         # the next allocation.
         keep = [dys]
-        side = gpu._dev.own_stream()
+        side = gpu._dev.own_stream() and self._gpu_bound(max(x.shape[0] for x in xs))
+        check(lib.vkc_mse_grouped(gpu._dev.h, px, py, _ptrs([d._buf.ptr or 0 for d in dys]), batch, cols,
+                                  None if side else losses._buf.ptr or 0, n))
+        for d in dys:
+            d._written()
+        losses._written()
         if side:
             check(lib.vkc_side_defer(gpu._dev.h, 1))
         try:
-            self._beside(side, lambda: check(lib.vkc_mse_grouped(
-                gpu._dev.h, px, py, None, batch, cols, losses._buf.ptr or 0, n)))
-            losses._written()
+            if side:
+                self._beside(True, lambda: check(lib.vkc_mse_grouped(
+                    gpu._dev.h, px, py, None, batch, cols, losses._buf.ptr or 0, n)))
             self._backward(acts, dys, keep, side)
         finally:
             if side:
                 check(lib.vkc_side_defer(gpu._dev.h, 0))
             del keep
         return preds, losses
+
+    def _gpu_bound(self, batch: int) -> bool:
+        """Whether the step waits for the GPU, so that the side branch pays for
+        its events (10 us of host time: 1 split-bf16x3 model call by call 94
+        us without it, 104 with it; 4 models 181 and 194).  A graph does.  Call
+        by call the host takes about 60 us and 30 a model, and the tensor-core
+        GEMMs less; fp32 GEMMs are a chain of 0.115 us per element of K, 70 us
+        for the rest (2 models of up to 200: 170 us without, 154 with it)."""
+        if self.gpu._dev.capture is not None:
+            return True
+        if self.gpu.matmul_precision != "fp32":
+            return False
+        chain = len(self._plan[0]) * batch   # the weight gradients', then the forward's and the input gradients'
+        for l, dense in enumerate(zip(*([d for d, _ in p] for p in self._plan))):
+            chain += max(d.input_dim for d in dense) + (max(d.output_dim for d in dense) if l else 0)
+        return 0.115 * chain > 30 * len(self.models) - 10
 
     def _beside(self, side: bool, run):
         """``run()`` on the side branch (after everything issued so far)."""
