@@ -43,13 +43,18 @@ inline bool fp32_on_tensor_cores(int64_t M, int64_t N, int64_t K, int splits) {
 }
 
 // The same for the products of layers: vkc_gemm, the grouped GEMM and the
-// Dense calls, which agree with one another bit for bit.  A layer's call is
-// bound by the host up to about 2^30 (256 x 784 -> 1024 -> 1024 -> 10 run call
-// by call: 176 us a step with FMAs, 191 with the tensor path's extra launches;
-// 4096 x 2048 -> 2048 forward and backward: 2410 us with FMAs, 637 on the
-// tensor cores).  In a network a ReLU passes another rounding on as another
-// sign wherever a value is within it of zero, so below that line trained
-// models keep the values of the FMA path too.
+// Dense calls, which agree with one another bit for bit where the single call
+// does not split K (the grouped GEMM never does).  Run call by call a layer is
+// bound by the host up to about 2^30 (256 x 784 -> 1024 -> 1024 -> 10: 176 us a
+// step with FMAs, 191 with the tensor path's extra launches; 4096 x 2048 -> 2048
+// forward and backward: 2410 us with FMAs, 637 on the tensor cores).  In a
+// graph or a grouped launch, where that cost is gone, the tensor path is the
+// faster one from less work on (256 x 1024 x 784: 22.8 -> 14.3 us; a grouped
+// step of 64 models 2160 -> 974), but there too the line stays here: in a
+// network a ReLU passes another rounding on as another sign wherever a value
+// is within it of zero, so that below the line trained models would leave the
+// values they have with FMAs (gradients of that grouped step by 4.5e-4, though
+// nearer to float64: 7e-5 against 2.8e-4).
 inline bool layer_fp32_on_tensor_cores(int64_t M, int64_t N, int64_t K, int splits) {
   return fp32_on_tensor_cores(M, N, K, splits) && M * N * K >= (int64_t(1) << 30);
 }

@@ -251,9 +251,10 @@ __device__ __forceinline__ F2 log_unit(F2 w) {
   return f2_fma(e, f2(0x1.62e4p-1f), f2_fma(e, f2(0x1.7f7d1cp-20f), g));
 }
 
-// sqrt(-2 x), x in [-2^4, 0]: one Newton step from the reciprocal root (of
-// 1e-36 for x = 0, so that 0 gives 0 and not 0 times infinity; the smallest
-// other x is -2^-23).
+// sqrt(a), a = -2 x, x in [-2^4, 0]: g = a y with y the hardware's reciprocal
+// root (of 1e-36 for x = 0, so that 0 gives 0 and not 0 times infinity; the
+// smallest other x is -2^-23), then a step of Newton's method for g^2 = a with
+// y / 2 in the place of 1 / 2g.
 __device__ __forceinline__ F2 sqrt_minus2(F2 x) {
   const F2 a = f2_mul(x, f2(-2.0f));
   float a0, a1, y0, y1;

@@ -1135,7 +1135,10 @@ def matmul_grouped(a_list: Sequence["Array"], b_list: Sequence["Array"], precisi
     """``[a @ b for a, b in zip(a_list, b_list)]`` for 2-D operands of any
     sizes, computed by one grouped launch (per 128 products) instead of one
     launch per product.  ``precision`` as for ``matmul`` (default: the GPU's
-    ``matmul_precision``).  No counterpart in the reference."""
+    ``matmul_precision``); in "fp32" a product may differ from ``a @ b`` in
+    rounding, since it runs on the tensor cores only from 2^30 multiply-adds
+    on, like a layer's, and never in several K ranges.  No counterpart in the
+    reference."""
     if len(a_list) != len(b_list):
         raise ValueError("a_list and b_list differ in length")
     if not a_list:
