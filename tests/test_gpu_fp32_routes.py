@@ -149,6 +149,35 @@ def test_without_room_for_the_partial_sums(gpu, vk, no_plans):
     assert launches == 3 and rel_fro(np.asarray(c), exp) < BOUND
 
 
+def test_without_room_in_a_capture(gpu, vk, no_plans):
+    """The same while a graph is captured (copies and, in a second product,
+    partial sums that cannot be had)."""
+    from vulkpy_gb300 import _lib
+    A, B = _operands(np.random.default_rng(5), 300, 300, 400, 0, 0)
+    a, b = vk.Array(gpu, data=A), vk.Array(gpu, data=B)
+    exp = A.astype(np.float64) @ B
+    a @ b
+    for after, launches in ((1, 1), (2, 2), (-1, 3)):
+        g = vk.graph.Graph(gpu)
+        try:
+            assert _lib.lib.vkc_inject_alloc_failure(after) == 0
+            with g:
+                n, c = _launches(gpu, lambda: a @ b)
+        finally:
+            _lib.lib.vkc_inject_alloc_failure(-1)
+        assert n == launches
+        g.launch()
+        assert rel_fro(np.asarray(c), exp) < 1e-6
+    big = vk.Array(gpu, data=np.ones((6144, 6144), np.float32))    # 450 MB of copies: with room for them
+    big @ big
+    g = vk.graph.Graph(gpu)
+    with g:
+        n, c = _launches(gpu, lambda: big @ big)
+    assert n == 3
+    g.launch()
+    assert np.all(np.asarray(c) == 6144)
+
+
 def _grouped(vk, gpu, A, B):
     """A @ B as a grouped product of one problem: launches and result."""
     from vulkpy_gb300 import _lib

@@ -161,6 +161,12 @@ inline void load_kernels(vkc_device_t dev, std::atomic<uint64_t>& done, K*... ke
 int scratch_alloc(vkc_device_t dev, size_t bytes, void** p);
 void scratch_free(vkc_device_t dev, void* p);
 
+// scratch_alloc for scratch that the call can do without.  While the stream is
+// captured an allocation that does not fit fails only when the graph is
+// launched, so from 256 MiB on it is refused there unless the device has twice
+// as much free.
+int scratch_alloc_optional(vkc_device_t dev, size_t bytes, void** p);
+
 // ---- programmatic dependent launch (PDL)
 // A kernel launched with launch_pdl may be scheduled while the kernel before
 // it on the stream is still running: its blocks become resident as that

@@ -1048,7 +1048,8 @@ int launch_tcp(vkc_device_t dev, const CUtensorMap& ma, const CUtensorMap& mb, c
   splits = (nk + kps - 1) / kps;
   float* partial = nullptr;
   if (splits > 1) {
-    int r = scratch_alloc(dev, sizeof(float) * (size_t)splits * M * N, (void**)&partial);
+    const size_t bytes = sizeof(float) * (size_t)splits * M * N;
+    int r = (PARTS == 3 ? scratch_alloc_optional : scratch_alloc)(dev, bytes, (void**)&partial);
     if (r != VKC_OK) return r;
   }
   const int64_t units = tiles * splits;
@@ -1263,7 +1264,7 @@ int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t 
   const size_t elems = 3 * (size_t)(M + N) * Kp;
   const size_t list = (elems * sizeof(__nv_bfloat16) + 15) / 16 * 16;
   void* scratch = nullptr;
-  if (scratch_alloc(dev, list + (size_t)(1 + tiles) * 4, &scratch) != VKC_OK) {
+  if (scratch_alloc_optional(dev, list + (size_t)(1 + tiles) * 4, &scratch) != VKC_OK) {
     // no room for the operands' copies: the SIMT GEMM reads them in place
     clear_error();
     return simt();

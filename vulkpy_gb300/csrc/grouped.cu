@@ -1043,7 +1043,7 @@ int grouped_tc(vkc_device_t dev, const vkc_gemm_problem* probs, const vkc_gemm_u
     const size_t list = bytes;  // bytes is a multiple of 16 KB
     if (PARTS == 3) bytes += 4 * (1 + ctiles);
     void* scratch = nullptr;
-    int r = scratch_alloc(dev, bytes, &scratch);
+    int r = (PARTS == 3 ? scratch_alloc_optional : scratch_alloc)(dev, bytes, &scratch);
     if (r != VKC_OK && PARTS == 3) {
       // no room for the operands' copies: the SIMT kernel reads them in place
       clear_error();

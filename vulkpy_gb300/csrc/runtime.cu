@@ -68,6 +68,22 @@ int scratch_alloc(vkc_device_t dev, size_t bytes, void** p) {
   return VKC_OK;
 }
 
+int scratch_alloc_optional(vkc_device_t dev, size_t bytes, void** p) {
+  if (bytes >= (size_t(1) << 28)) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    size_t free = 0, total = 0;
+    const bool asked = cudaStreamIsCapturing(dev->stream, &cap) == cudaSuccess &&
+                       (cap == cudaStreamCaptureStatusNone || cudaMemGetInfo(&free, &total) == cudaSuccess);
+    if (!asked) {
+      cudaGetLastError();
+    } else if (cap != cudaStreamCaptureStatusNone && bytes > free / 2) {
+      *p = nullptr;
+      return set_error(VKC_ERR_OOM, "captured allocation of %zu bytes with %zu free", bytes, free);
+    }
+  }
+  return scratch_alloc(dev, bytes, p);
+}
+
 void scratch_free(vkc_device_t dev, void* p) {
   if (p) cudaFreeAsync(p, dev->stream);
 }
