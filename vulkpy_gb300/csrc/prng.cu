@@ -192,7 +192,7 @@ __device__ __forceinline__ float to_unit(uint32_t r) { return __uint_as_float((r
 // packed float32 arithmetic (fma.rn.f32x2).  The kernel is bound by its
 // instructions, the integer ones above all (the generator's own 20 per pair):
 // 2^27 normals took 225 us with logf / sqrtf / sincosf (102 instructions per
-// pair even with these functions in scalar form: 215 us), 177 us so; the
+// pair even with these functions in scalar form: 215 us), 175 us so (82); the
 // store alone takes 79.  Polynomials are minimax fits (Lawson's iteration)
 // made for this file.  Over all 2^23 arguments, in ulps of the exact value: log
 // within 0.9, sin within 1.42 and cos within 1.46 (sincosf: 1.45 and 1.47),
