@@ -1272,9 +1272,8 @@ int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t 
   {
     static std::atomic<uint64_t> loaded{0};
     load_kernels(dev, loaded, k_split_pair<3>, k_gemm_tcp<3, 128, 2, 1>, k_gemm_tcp<3, 128, 2, 1, true>,
-                 k_gemm_tcp<3, 128, 2, 2, true>,
-                 k_splitk_reduce4, k_splitk_reduce, k_gemm_repair<false, false>, k_gemm_repair<false, true>,
-                 k_gemm_repair<true, false>, k_gemm_repair<true, true>);
+                 k_gemm_tcp<3, 128, 2, 2, true>, k_splitk_reduce4, k_splitk_reduce, k_gemm_repair<false, false>,
+                 k_gemm_repair<false, true>, k_gemm_repair<true, false>, k_gemm_repair<true, true>);
   }
   auto* a = static_cast<__nv_bfloat16*>(scratch);
   auto* b = a + 3 * (size_t)M * Kp;
@@ -1289,7 +1288,9 @@ int gemm_fp32(vkc_device_t dev, bool ta, bool tb, int64_t M, int64_t N, int64_t 
     // ranges, U[0,1) data: error 8.0e-8 -> 5.5e-8, where FMAs in 16 ranges of
     // 16 gave 6.1e-8); else one, which drains half as often (2048^3 in 2
     // ranges: 128 -> 114 us) and which the grouped kernel reproduces
-    r = (splits == 1 ? launch_tcp<3, 128, 2, 1> : Kp / splits <= 256 ? launch_tcp<3, 128, 2, 2, true> : launch_tcp<3, 128, 2, 1, true>)(
+    r = (splits == 1           ? launch_tcp<3, 128, 2, 1>
+         : Kp / splits <= 256 ? launch_tcp<3, 128, 2, 2, true>
+                              : launch_tcp<3, 128, 2, 1, true>)(
         dev, ma, mb, ma, mb, M, N, K, alpha, beta, C, ldc, epi, splits, nullptr,
         RepairOperands{A, B, lda, ldb, K, ta ? 1 : 0, tb ? 1 : 0}, repair);
   scratch_free(dev, scratch);
